@@ -44,6 +44,17 @@ __host__ __device__ __forceinline__ V mul_i(V a) {
     return r;
 }
 
+// ---- programmatic dependent launch -------------------------------------------
+// First statement of every kernel that launch_pdl starts: such a kernel may
+// become resident before the kernel in front of it on the stream has ended,
+// so nothing may be read or written before that one is complete and its
+// memory visible (the wait; at once for an ordinary launch).  The kernel
+// behind may take its place in turn once every CTA of this one is resident.
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---- reductions ------------------------------------------------------------
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll

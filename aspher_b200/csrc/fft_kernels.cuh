@@ -303,6 +303,7 @@ template <typename T, int LR, bool PAD, int V, class Load, class Store>
 __global__ void __launch_bounds__(row_threads<T>(LR, V), (row_fwd_minb<T, LR, PAD, V>()))
 row_fwd_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
                const cplx<T>* __restrict__ tw_2lr, const int* __restrict__ gate) {
+    pdl_wait();
     if (gate && gate[blockIdx.y * kGateStride]) return;
     constexpr int RPT = row_rpt<T>(LR, V);
     constexpr int TT = LR / RPT;
@@ -487,6 +488,7 @@ template <typename T, int LR, bool PAD, int V, class Load, class Store>
 __global__ void __launch_bounds__(row_threads<T>(LR, V), row_minb<T>(LR, V))
 row_inv_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
                const cplx<T>* __restrict__ tw_2lr, const int* __restrict__ gate) {
+    pdl_wait();
     if (gate && gate[blockIdx.y * kGateStride]) return;
     constexpr int RPT = row_rpt<T>(LR, V);
     constexpr int TT = LR / RPT;
@@ -642,6 +644,7 @@ template <typename T, int LC, int NCM1, bool PAD, int V, class Mult>
 __global__ void __launch_bounds__(col_threads<T>(LC, NCM1, V), col_minb<T>(LC, NCM1, V))
 col_kernel(cplx<T>* __restrict__ spec, int nrows, Mult mul,
            const cplx<T>* __restrict__ tw_lc, const int* __restrict__ gate) {
+    pdl_wait();
     if (gate && gate[blockIdx.y * kGateStride]) return;
     constexpr int RPT = col_rpt<T>(LC, V);
     constexpr int CT = col_ct_v<T>(LC, NCM1, V);
@@ -729,6 +732,7 @@ __global__ void __launch_bounds__(col_threads<T>(LH, NCM1, V), col_minb<T>(LH, N
 col_split_kernel(cplx<T>* __restrict__ spec, cplx<T>* __restrict__ acc, int nrows, Mult mul,
                  const cplx<T>* __restrict__ tw_lh, const cplx<T>* __restrict__ tw_m,
                  const int* __restrict__ gate) {
+    pdl_wait();
     if (gate && gate[blockIdx.y * kGateStride]) return;
     constexpr int RPT = col_rpt<T>(LH, V);
     constexpr int CT = col_ct_v<T>(LH, NCM1, V);

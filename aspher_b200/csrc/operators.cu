@@ -350,8 +350,8 @@ void launch_col_split(cplx<T>* spec, cplx<T>* acc, int nrows, Mult m, cudaStream
     fft_attrs((const void*)k0, sm);
     fft_attrs((const void*)k1, sm);
     const dim3 grid(NCM1 / ct + 1, B);
-    k0<<<grid, thr, sm, s>>>(spec, acc, nrows, m, tw<T>(LH), tw<T>(2 * LH), gate);
-    k1<<<grid, thr, sm, s>>>(spec, acc, nrows, m, tw<T>(LH), tw<T>(2 * LH), gate);
+    launch_pdl(k0, grid, thr, sm, s, spec, acc, nrows, m, tw<T>(LH), tw<T>(2 * LH), gate);
+    launch_pdl(k1, grid, thr, sm, s, spec, acc, nrows, m, tw<T>(LH), tw<T>(2 * LH), gate);
 }
 
 #define ASB_V_SWITCH(VV, L, ...)                                                   \

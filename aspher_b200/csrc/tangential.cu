@@ -198,6 +198,7 @@ template <typename T, int LC, int CT>
 __global__ void __launch_bounds__(2 * CT * (LC / col_rpt<T>(LC, 0)))
 col_pair_kernel(cplx<T>* __restrict__ spec, long bsp, int nrows, TanMix<T> mix,
                 const cplx<T>* __restrict__ tw_lc) {
+    pdl_wait();
     constexpr int RPT = col_rpt<T>(LC, 0);
     constexpr int TT = LC / RPT;
     constexpr int S = 2 * CT;
@@ -435,7 +436,7 @@ void TanOperator::apply(const T* q, T* u, cudaStream_t s) {
         fft_attrs((const void*)k, sm);
         const TanMix<T> mix{static_cast<const T*>(kt[dbl][0]), static_cast<const T*>(kt[dbl][1]),
                             static_cast<const T*>(kt[dbl][2]), NS + 1, CT, LC};
-        k<<<NS / CT + 1, thr, sm, s>>>(sp, bsp, NS, mix, tw<T>(LC));
+        launch_pdl(k, dim3(NS / CT + 1), thr, sm, s, sp, bsp, NS, mix, tw<T>(LC));
     }
     launch_row_inv<T, LR, true, RV>(LoadTiled<T>{sp, NS, CT, bsp}, StoreRealRows<T>{u, NS, N}, NS,
                                    s, nullptr, 2);

@@ -41,8 +41,11 @@ class ContactSolver:
     def matvec(self, p):
         return self.mv(np.asarray(p, dtype=np.float64).reshape(-1))
 
+    def love_table(self):
+        return np.asarray(self.op.table).reshape(self.Ns, self.Ns)
+
     def solve(self, gap, p_nominal, tol=1e-8, max_iter=5000, use_pr=True,
-              precond="none", p_init=None):
+              precond="none", p_init=None, stall_limit=200):
         N = self.Ns * self.Ns
         g0 = np.asarray(gap, dtype=np.float64).reshape(-1)
         if g0.size != N:
@@ -56,7 +59,7 @@ class ContactSolver:
             pc = lambda g, c: fp.apply(g, c, np.float64)
         elif precond not in ("none", ""):
             raise ValueError("precond must be 'none', 'fourier' or 'fourier-fft'")
-        opt = SolveOptions(tol=tol, max_iter=max_iter, use_pr=use_pr)
+        opt = SolveOptions(tol=tol, max_iter=max_iter, use_pr=use_pr, stall_limit=stall_limit)
         p0 = None if p_init is None else np.asarray(p_init, np.float64).reshape(-1)
         r = solve_contact_impl(lambda x: self.mv(x, np.float64), g0, p_nominal,
                                opt, pc, p0, dtype=np.float64)

@@ -637,12 +637,14 @@ row_inv_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
 }
 
 // ---- column forward * multiplier * inverse --------------------------------------
-// Mult: cplx<T> operator()(cplx<T> X, int kx, int ky).  One unit = one tile
-// of CT columns; instance blockIdx.y owns NCM1/CT + 1 contiguous tiles.
+// Mult: cplx<T> operator()(cplx<T> X, int kx, int ky).  nrows: rows of the
+// layout; ndata: the rows that hold data (fewer only in the zero-padded
+// transform of an embedded operator: the rest read as zero and are not
+// written).  One unit = one tile of CT columns; instance blockIdx.y owns NCM1/CT + 1 contiguous tiles.
 // Dynamic shared memory: col_smem_total<T, LC, NCM1, PAD, V>().
 template <typename T, int LC, int NCM1, bool PAD, int V, class Mult>
 __global__ void __launch_bounds__(col_threads<T>(LC, NCM1, V), col_minb<T>(LC, NCM1, V))
-col_kernel(cplx<T>* __restrict__ spec, int nrows, Mult mul,
+col_kernel(cplx<T>* __restrict__ spec, int nrows, int ndata, Mult mul,
            const cplx<T>* __restrict__ tw_lc, const int* __restrict__ gate) {
     pdl_wait();
     if (gate && gate[blockIdx.y * kGateStride]) return;
@@ -680,7 +682,7 @@ col_kernel(cplx<T>* __restrict__ spec, int nrows, Mult mul,
         block_fft<T, LC, RPT, +1, CT, false, ALT, P1>(v, t, sm, c, tw_lc);
 #pragma unroll
         for (int m = 0; m < RPT; ++m) {
-            if (PAD && m >= RPT / 2) continue;
+            if (PAD && (m >= RPT / 2 || t + m * TT >= ndata)) continue;
             base[(size_t)(t + m * TT) * CT + c] = v[m];
         }
     };
@@ -710,7 +712,7 @@ col_kernel(cplx<T>* __restrict__ spec, int nrows, Mult mul,
         cplx<T> v[RPT];
 #pragma unroll
         for (int m = 0; m < RPT; ++m) {
-            if (PAD && m >= RPT / 2) v[m] = mk<T>(0, 0);
+            if (PAD && (m >= RPT / 2 || t + m * TT >= ndata)) v[m] = mk<T>(0, 0);
             else v[m] = base[(size_t)(t + m * TT) * CT + c];
         }
         body(tile, v);
@@ -729,7 +731,8 @@ col_kernel(cplx<T>* __restrict__ spec, int nrows, Mult mul,
 // back on one stream.  One column tile per CTA; shared memory col_smem<T>(LH, CT).
 template <typename T, int LH, int NCM1, int V, int PARITY, class Mult>
 __global__ void __launch_bounds__(col_threads<T>(LH, NCM1, V), col_minb<T>(LH, NCM1, V))
-col_split_kernel(cplx<T>* __restrict__ spec, cplx<T>* __restrict__ acc, int nrows, Mult mul,
+col_split_kernel(cplx<T>* __restrict__ spec, cplx<T>* __restrict__ acc, int nrows, int ndata,
+                 Mult mul,
                  const cplx<T>* __restrict__ tw_lh, const cplx<T>* __restrict__ tw_m,
                  const int* __restrict__ gate) {
     pdl_wait();
@@ -748,7 +751,7 @@ col_split_kernel(cplx<T>* __restrict__ spec, cplx<T>* __restrict__ acc, int nrow
 #pragma unroll
     for (int m = 0; m < RPT; ++m) {
         const int n = t + m * TT;
-        v[m] = base[(size_t)n * CT + c];
+        v[m] = n < ndata ? base[(size_t)n * CT + c] : mk<T>(0, 0);
         if constexpr (PARITY) v[m] = cmul(v[m], __ldg(&tw_m[n]));
     }
     block_fft<T, LH, RPT, -1, CT>(v, t, sm, c, tw_lh);
@@ -759,6 +762,7 @@ col_split_kernel(cplx<T>* __restrict__ spec, cplx<T>* __restrict__ acc, int nrow
 #pragma unroll
     for (int m = 0; m < RPT; ++m) {
         const size_t i = (size_t)(t + m * TT) * CT + c;
+        if (t + m * TT >= ndata) continue;
         if constexpr (PARITY) {
             base[i] = cadd(cmulc(v[m], __ldg(&tw_m[t + m * TT])), abase[i]);
         } else {

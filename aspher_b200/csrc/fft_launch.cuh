@@ -64,7 +64,7 @@ void launch_row_inv(Load ld, Store st, int nrows, cudaStream_t s, const int* gat
     launch_pdl(k, dim3(gx, B), thr, sm, s, ld, st, nrows, tw<T>(LR), tw<T>(2 * LR), gate);
 }
 template <typename T, int LC, int NCM1, bool PAD, int V, class Mult>
-void launch_col(cplx<T>* spec, int nrows, Mult m, cudaStream_t s, const int* gate, int B = 1) {
+void launch_col(cplx<T>* spec, int nrows, int ndata, Mult m, cudaStream_t s, const int* gate, int B = 1) {
     constexpr int ct = col_ct_v<T>(LC, NCM1, V), thr = col_threads<T>(LC, NCM1, V);
     constexpr int sm = col_smem_total<T, LC, NCM1, PAD, V>();
     auto k = col_kernel<T, LC, NCM1, PAD, V, Mult>;
@@ -72,7 +72,7 @@ void launch_col(cplx<T>* spec, int nrows, Mult m, cudaStream_t s, const int* gat
     const int gx = col_staged<T, LC, NCM1, PAD, V>()
                        ? persistent_blocks((const void*)k, thr, sm, NCM1 / ct + 1)
                        : NCM1 / ct + 1;
-    launch_pdl(k, dim3(gx, B), thr, sm, s, spec, nrows, m, tw<T>(LC), gate);
+    launch_pdl(k, dim3(gx, B), thr, sm, s, spec, nrows, ndata, m, tw<T>(LC), gate);
 }
 
 

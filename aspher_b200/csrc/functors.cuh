@@ -52,6 +52,43 @@ struct StoreRealRows {
     __device__ void finish(double*) const {}
 };
 
+// An embedded operator's caller field (Nl rows of Nl values): z[n] of the
+// compute grid's row, 0 outside the caller's block.  Scalar accesses: an odd
+// Nl leaves the rows at every alignment.
+template <typename T>
+struct LoadBlockRows {
+    const T* x;
+    int Nl;
+    long bs;
+    static constexpr bool kTiled = false;
+    static constexpr bool kRaw = false;
+    __device__ __forceinline__ cplx<T> operator()(int row, int n) const {
+        cplx<T> z = mk<T>(T(0), T(0));
+        if (row < Nl) {
+            const T* r = x + blockIdx.y * bs + (size_t)row * Nl;
+            if (2 * n < Nl) z.x = r[2 * n];
+            if (2 * n + 1 < Nl) z.y = r[2 * n + 1];
+        }
+        return z;
+    }
+};
+
+template <typename T>
+struct StoreBlockRows {
+    T* y;
+    int Nl;
+    long bs;
+    static constexpr bool kFinish = false;
+    static constexpr bool kTiled = false;
+    __device__ __forceinline__ void operator()(int row, int n, cplx<T> z) const {
+        if (row >= Nl) return;
+        T* r = y + blockIdx.y * bs + (size_t)row * Nl;
+        if (2 * n < Nl) r[2 * n] = z.x;
+        if (2 * n + 1 < Nl) r[2 * n + 1] = z.y;
+    }
+    __device__ void finish(double*) const {}
+};
+
 // FP64 rows in, FP32 pairs out: x - x0 (x0 optional), rounded once.  The
 // defect-corrected FP64 apply (Operator::matvec_defect) transforms this
 // difference in FP32.

@@ -142,8 +142,8 @@ void na_apply(NaDevice& d, double scale, const T* x, T* y, cudaStream_t s) {
     }
     {
         constexpr int thr = col_threads<T>(LC, LR, V);
-        K::col<<<LR / ct + 1, thr, K::sm_col, s>>>(spec, NS, PeriodicMult<T>{scale, NS}, tw + LC,
-                                                   nullptr);
+        K::col<<<LR / ct + 1, thr, K::sm_col, s>>>(spec, NS, NS, PeriodicMult<T>{scale, NS},
+                                                   tw + LC, nullptr);
     }
     {
         constexpr int rb = row_rb_v<T>(LR, V), thr = row_threads<T>(LR, V);

@@ -1,0 +1,26 @@
+// The periodic pipeline and the full-grid |k| preconditioner in FP32 (see
+// op_impl.cuh).
+#include "op_impl.cuh"
+
+namespace asb {
+
+template <>
+void periodic_matvec<float>(const Operator& op, const float* x, float* y, cplx<float>* spec, cudaStream_t s,
+                        const int* gate, int B, const PkState* sc) {
+    ASB_SIZE_SWITCH(op.Ns, (PeriodicImpl<float, NS>::matvec(op, x, y, spec, s, gate, B, sc)));
+}
+
+template <>
+void periodic_precond<float>(Operator& op, const float* g, const uint8_t* mask, PkState* st, float* z,
+                         double* part, cudaStream_t s, const int* gate, int B, void* spec) {
+    ASB_SIZE_SWITCH(op.Ns, (FourierImpl<float, NS>::run(op, g, mask, st, z, part, s, gate, B, spec)));
+}
+
+void periodic_defect(const Operator& op, LoadDiffRows ld, StoreAddRows st, float2* spec,
+                     cudaStream_t s, const int* gate, int B) {
+    ASB_SIZE_SWITCH(op.Ns, (PeriodicImpl<float, NS>::apply(
+                               op.rowv[0], op.colv[0], ld, PeriodicImpl<float, NS>::mult(op), st,
+                               spec, s, gate, B)));
+}
+
+}  // namespace asb

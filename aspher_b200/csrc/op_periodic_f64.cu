@@ -1,0 +1,19 @@
+// The periodic pipeline and the full-grid |k| preconditioner in FP64 (see
+// op_impl.cuh).
+#include "op_impl.cuh"
+
+namespace asb {
+
+template <>
+void periodic_matvec<double>(const Operator& op, const double* x, double* y, cplx<double>* spec, cudaStream_t s,
+                        const int* gate, int B, const PkState* sc) {
+    ASB_SIZE_SWITCH(op.Ns, (PeriodicImpl<double, NS>::matvec(op, x, y, spec, s, gate, B, sc)));
+}
+
+template <>
+void periodic_precond<double>(Operator& op, const double* g, const uint8_t* mask, PkState* st, double* z,
+                         double* part, cudaStream_t s, const int* gate, int B, void* spec) {
+    ASB_SIZE_SWITCH(op.Ns, (FourierImpl<double, NS>::run(op, g, mask, st, z, part, s, gate, B, spec)));
+}
+
+}  // namespace asb

@@ -100,11 +100,7 @@ struct Operator {
     int Nl = 0;
     int backend = OP_FFT;
     bool embedded() const { return Nl != Ns || backend != kind; }
-    // embedded: Ns*Ns scratch fields of the caller-facing apply (lazy)
-    void* emb_x = nullptr;
-    void* emb_y = nullptr;
-    // caller-facing apply: x, y hold Nl*Nl values (embedded: copied into the
-    // compute grid's block and back; otherwise matvec)
+    // caller-facing apply: x, y hold Nl*Nl values
     void apply_caller(bool dbl, const void* x, void* y, cudaStream_t s);
     // embedded grids (even Nl) with the full-grid |k| preconditioner: the
     // spectrum of its real-space kernel on the Nl torus, canonical and tiled
@@ -153,6 +149,7 @@ struct Operator {
     Operator& operator=(const Operator&) = delete;
 
     // u = S x on `stream`; x, y device arrays of Ns*Ns values of the dtype.
+    // Embedded: x is zero past row Nl, and y is written up to there only.
     // gate: optional device int; when nonzero at kernel start, kernels return.
     // Batched (B > 1): x, y hold B fields back to back, spec_b a spectrum
     // scratch of B * spectrum_bytes(dbl), and gate[b * kGateStride] gates

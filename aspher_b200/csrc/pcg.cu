@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_eval(const PkPar
     const T gs = (T)P.gshift;
     const PScale<T> ps(st);
     double acc[5] = {0.0, 0.0, (double)INFINITY, 0.0, 0.0};  // sum_C v, n_C, min v, pv, psum
-    GRID_LOOP4(P.N) {
+    GRID_LOOP4(P.Nv) {
         T uu[4], gg0[4], pp[4], vv[4];
         uint8_t mm[4];
         ldp4(u, i4, uu);
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_evalpk(const PkP
     const T aT = (T)st->alpha;
     const PScale<T> ps(st);
     double acc[1] = {0.0};
-    GRID_LOOP4(P.N) {
+    GRID_LOOP4(P.Nv) {
         T pp[4], gv[4];
         ldp4(p, i4, pp);
         ldp4(g, i4, gv);
@@ -287,7 +287,7 @@ __global__ void k_center(const PkParams* __restrict__ Pp, const PkState* st, T* 
     st += blockIdx.y;
     g += (long)blockIdx.y * Pp->N;
     const T aT = (T)st->alpha;
-    GRID_LOOP4(Pp->N) {
+    GRID_LOOP4(Pp->Nv) {
         T gv[4];
         ldp4(g, i4, gv);
 #pragma unroll
@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_dots(const PkPar
     if (st->halt) return;
     const T zm = (T)st->zmean, aT = (T)st->alpha;
     double acc[3] = {0, 0, 0};  // G, G_pr, gg
-    GRID_LOOP4(P.N) {
+    GRID_LOOP4(P.Nv) {
         T zz[4], gv[4], gp[4];
         uint8_t mm[4];
         ldm4(mask, i4, mm);
@@ -752,7 +752,7 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_tupd(const PkPar
     const T zm = (T)st->zmean, beta = (T)st->beta, aT = (T)st->alpha;
     const int cb = st->copy_best;
     const PScale<T> ps(st);
-    GRID_LOOP4(P.N) {
+    GRID_LOOP4(P.Nv) {
         T zz[4], gv[4], tt[4];
         uint8_t mm[4];
         ldm4(mask, i4, mm);
@@ -793,7 +793,7 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_rden(const PkPar
     if (st->halt) return;
     const T aT = (T)st->alpha;
     double acc[4] = {0, 0, 0, 0};  // sum_C r, sum_C g t, sum_C r t, sum_C t
-    GRID_LOOP4(P.N) {
+    GRID_LOOP4(P.Nv) {
         T rr[4], gv[4], tt[4];
         uint8_t mm[4];
         ldm4(mask, i4, mm);
@@ -833,7 +833,7 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_pupd(const PkPar
     // last-block counter; only the last block's tail rewrites it
     const PScale<T> ps(st);
     double acc[2] = {0, 0};  // changed (max), total
-    GRID_LOOP4(P.N) {
+    GRID_LOOP4(P.Nv) {
         T pp[4], tt[4], gv[4];
         ldp4(p, i4, pp);
         ldp4(t, i4, tt);
@@ -894,7 +894,7 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_materialize(
     const PScale<T> ps(st);
     const bool identity = ps.f == T(1) && ps.a == T(0);
     if (!identity) {
-        GRID_LOOP4(P.N) {
+        GRID_LOOP4(P.Nv) {
             T pp[4];
             ldp4(p, i4, pp);
 #pragma unroll
@@ -936,7 +936,7 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_reduce(const PkP
     const T gs = (T)P.gshift;
     double acc[3] = {0, 0, 0};
     if (mode == 0) { acc[0] = (double)INFINITY; acc[1] = -(double)INFINITY; }
-    GRID_LOOP4(P.N) {
+    GRID_LOOP4(P.Nv) {
         T A[4], B[4], C[4], D[4];
         ldp4(a, i4, A);
         if (b) ldp4(b, i4, B);
@@ -986,7 +986,7 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_gd(const PkParam
                                                     const T* z, const T* p, double* part) {
     const PkParams& P = *Pp;
     double acc[1] = {0};
-    GRID_LOOP4(P.N) {
+    GRID_LOOP4(P.Nv) {
         T G[4], Z[4], Pp[4];
         ldp4(g, i4, G);
         ldp4(z, i4, Z);
@@ -1126,6 +1126,7 @@ struct SolverCtx : SolverCtxBase {
     Operator& op;
     int cap = 1;
     long N = 0;
+    long Nv = 0;  // the prefix of a field that the vector passes visit (PkParams::Nv)
     T *p = nullptr, *t = nullptr, *u = nullptr, *g = nullptr, *gprev = nullptr, *z = nullptr,
       *r = nullptr, *best = nullptr;
     T* g0c = nullptr;  // the solves' gaps, copied in so the loop graph is reusable
@@ -1167,16 +1168,22 @@ struct SolverCtx : SolverCtxBase {
         ASB_CUDA(cudaEventCreateWithFlags(&ev_in, cudaEventDisableTiming));
         ASB_CUDA(cudaEventCreateWithFlags(&ev_out, cudaEventDisableTiming));
         N = (long)o.Ns * o.Ns;
+        Nv = o.embedded() ? (long)o.Nl * o.Ns : N;  // Ns is a multiple of 16
         const size_t b = (size_t)cap * N * sizeof(T);
         T** vecs[] = {&p, &t, &u, &g, &gprev, &z, &r, &best, &g0c};
         for (T** v : vecs) ASB_CUDA(cudaMalloc((void**)v, b));
         ASB_CUDA(cudaMalloc((void**)&mask, (size_t)cap * N));
+        if (Nv != N) {  // the rows past Nv are never written: 0, and no contact
+            for (T** v : vecs) ASB_CUDA(cudaMemset(*v, 0, b));
+            ASB_CUDA(cudaMemset(mask, 0, (size_t)cap * N));
+            ASB_CUDA(cudaDeviceSynchronize());  // before anything on ws writes them
+        }
         ASB_CUDA(cudaMalloc((void**)&part, (size_t)cap * kPartStride * sizeof(double)));
         ASB_CUDA(cudaMalloc((void**)&st, (size_t)cap * sizeof(PkState)));
         ASB_CUDA(cudaMalloc((void**)&Pd, (size_t)cap * sizeof(PkParams)));
         ASB_CUDA(cudaMemset(st, 0, (size_t)cap * sizeof(PkState)));
         ASB_CUDA(cudaMemset(z, 0, b));
-        grid = red_grid(N);
+        grid = red_grid(Nv);
         // spectra allocated before any capture; none for a precision whose
         // applies do not exist at this size (FP64 above 8192: this context
         // then only holds the FP64 fields of a mixed solve)
@@ -1256,6 +1263,10 @@ struct SolverCtx : SolverCtxBase {
             std::lock_guard<std::recursive_mutex> setup(setup_mutex());
             ASB_CUDA(cudaMalloc((void**)&p0, (size_t)cap * N * sizeof(double)));
             ASB_CUDA(cudaMalloc((void**)&u0, (size_t)cap * N * sizeof(double)));
+            if (Nv != N) {
+                ASB_CUDA(cudaMemset(u0, 0, (size_t)cap * N * sizeof(double)));
+                ASB_CUDA(cudaDeviceSynchronize());
+            }
             (void)op.spectrum(false, nullptr);  // the FP32 scratch of unbatched applies
         }
         defect = on;
@@ -1501,7 +1512,7 @@ struct Solver {
 
     // project_load_simplex on instance b's z (contact_solver.cpp:31-60)
     void project_simplex(int b, double P_total) {
-        const long N = c.N;
+        const long N = c.Nv;  // z is 0 past it
         T* z = c.at(c.z, b);
         double ssum = reduce(b, 1, z, nullptr, nullptr, nullptr, 0.0);
         long nact = N;
@@ -1537,7 +1548,7 @@ struct Solver {
             I.s_id = (pu > 0.0 && pp > 0.0) ? pp / pu : 1.0;
         }
         for (int trial = 0; trial < 12; ++trial) {
-            k_axpy_trial<T><<<c.grid, kRedThreads, 0, s>>>(c.N, z, p, g, (T)I.s_id);
+            k_axpy_trial<T><<<c.grid, kRedThreads, 0, s>>>(c.Nv, z, p, g, (T)I.s_id);
             count_launches(1);
             project_simplex(b, I.P_total);
             c.op.matvec(sizeof(T) == 8, z, r, s, nullptr);  // unbatched scratch
@@ -1604,6 +1615,7 @@ struct Solver {
         for (int b = 0; b < B; ++b) {
             P[b] = PkParams{};
             P[b].N = N;
+            P[b].Nv = c.Nv;
             P[b].Ns = Ns;
             P[b].Nl = c.op.Nl;
             if (g0s[b] != c.at(c.g0c, b))
@@ -2081,6 +2093,7 @@ void mixed_prepare(Operator& op, const aspher_solve_opts& o, int B, const double
     Solver<double> probe(cd, s, B);
     for (int b = 0; b < B; ++b) {
         probe.P[b].N = N;
+        probe.P[b].Nv = cd.Nv;
         probe.P[b].Ns = op.Ns;
         probe.P[b].Nl = op.Nl;
     }
@@ -2317,6 +2330,7 @@ void precond_apply_impl(Operator& op, int precond, int radius, const T* g_in,
     ASB_CUDA(cudaMemsetAsync(st, 0, sizeof(PkState), s));  // alpha = 0: g used as given
     PkParams P{};
     P.N = N;
+    P.Nv = N;
     P.Ns = op.Ns;
     P.Nl = op.Nl;
     P.precond = precond;
@@ -2591,6 +2605,7 @@ void adjoint_core(Operator& op, const double* p, const double* w, double tol, in
     ASB_CUDA(cudaMemsetAsync(st, 0, sizeof(PkState), s));
     PkParams P{};
     P.N = N;
+    P.Nv = N;
     P.Ns = op.Ns;
     P.Nl = op.Nl;
     P.tol = tol;

@@ -30,7 +30,10 @@ enum Status : int {
 
 // Solve constants, passed by value to every kernel.
 struct PkParams {
-    long N;
+    long N;   // cells of the compute grid: an instance's fields are N apart
+    // the cells the vector passes visit, a prefix of the field: N, or
+    // (embedded operators) the Nl rows that hold the caller's cells
+    long Nv;
     int Ns;
     // the caller's grid side: Ns, or (embedded operators) the side of the
     // top-left block of the Ns x Ns field that holds the caller's cells

@@ -194,9 +194,10 @@ struct TanMix {
 // as 2 CT transforms: field c / CT, column c % CT); per column the pruned
 // forward transform (upper half zero), the 2x2 mix with the other field's
 // column through shared memory, the inverse transform keeping rows < Ns.
+// ndata as in col_kernel.
 template <typename T, int LC, int CT>
 __global__ void __launch_bounds__(2 * CT * (LC / col_rpt<T>(LC, 0)))
-col_pair_kernel(cplx<T>* __restrict__ spec, long bsp, int nrows, TanMix<T> mix,
+col_pair_kernel(cplx<T>* __restrict__ spec, long bsp, int nrows, int ndata, TanMix<T> mix,
                 const cplx<T>* __restrict__ tw_lc) {
     pdl_wait();
     constexpr int RPT = col_rpt<T>(LC, 0);
@@ -219,7 +220,8 @@ col_pair_kernel(cplx<T>* __restrict__ spec, long bsp, int nrows, TanMix<T> mix,
     cplx<T> v[RPT];
 #pragma unroll
     for (int m = 0; m < RPT; ++m)
-        v[m] = m >= RPT / 2 ? mk<T>(0, 0) : base[(size_t)(t + m * TT) * CT + cc];
+        v[m] = m >= RPT / 2 || t + m * TT >= ndata ? mk<T>(0, 0)
+                                                   : base[(size_t)(t + m * TT) * CT + cc];
     block_fft<T, LC, RPT, -1, S, true, ALT>(v, t, sm, c, tw_lc);
     // every thread publishes its column's spectrum, then reads the other
     // field's column at the same kx (the forward transform's last stage ran
@@ -240,7 +242,8 @@ col_pair_kernel(cplx<T>* __restrict__ spec, long bsp, int nrows, TanMix<T> mix,
     if constexpr (ALT == 0) __syncthreads();
     block_fft<T, LC, RPT, +1, S, false, ALT, ALT ? (PX ^ 1) : 0>(v, t, sm, c, tw_lc);
 #pragma unroll
-    for (int m = 0; m < RPT / 2; ++m) base[(size_t)(t + m * TT) * CT + cc] = v[m];
+    for (int m = 0; m < RPT / 2; ++m)
+        if (t + m * TT < ndata) base[(size_t)(t + m * TT) * CT + cc] = v[m];
 }
 
 }  // namespace
@@ -255,9 +258,6 @@ struct TanOperator {
     int Ns = 0, Nl = 0;
     double L = 1.0, E = 1.0, nu = 0.3;
     bool embedded() const { return Nl != Ns; }
-    // embedded: two-field compute-grid scratch of the caller-facing apply
-    void* emb_q = nullptr;
-    void* emb_u = nullptr;
     // caller-facing apply: q, u hold 2 Nl^2 values
     void apply_caller(bool dbl, const void* q, void* u, cudaStream_t s);
     int device = 0;
@@ -274,8 +274,12 @@ struct TanOperator {
     void release();
     void matvec(bool dbl, const void* q, void* u, cudaStream_t s);
 
+    template <typename T, int NS, class Load, class Store>
+    void apply(Load ld, Store st, int nd, cudaStream_t s);
     template <typename T, int NS>
-    void apply(const T* q, T* u, cudaStream_t s);
+    void apply_full(const T* q, T* u, cudaStream_t s);
+    template <typename T, int NS>
+    void apply_block(const T* q, T* u, cudaStream_t s);
     template <int NS>
     void build();
 };
@@ -402,9 +406,6 @@ void TanOperator::release() {
     cudaFree(tab_xx);
     cudaFree(tab_xy);
     tab_xx = tab_xy = nullptr;
-    cudaFree(emb_q);
-    cudaFree(emb_u);
-    emb_q = emb_u = nullptr;
     for (int d = 0; d < 2; ++d) {
         for (int j = 0; j < 3; ++j) {
             cudaFree(kt[d][j]);
@@ -416,18 +417,17 @@ void TanOperator::release() {
     if (cur != device) cudaSetDevice(cur);
 }
 
-template <typename T, int NS>
-void TanOperator::apply(const T* q, T* u, cudaStream_t s) {
+// the apply of two NS x NS fields whose first nd rows hold data
+template <typename T, int NS, class Load, class Store>
+void TanOperator::apply(Load ld, Store st, int nd, cudaStream_t s) {
     constexpr int LR = NS, LC = 2 * NS;
     constexpr int CT = tan_ct<T>(LC, NS);
     const int dbl = sizeof(T) == 8;
-    const long N = (long)NS * NS;
     const long bsp = (long)(LR / CT + 1) * NS * CT;
     cplx<T>* sp = static_cast<cplx<T>*>(spec[dbl]);
     // both fields' rows (instances 0 = q_x, 1 = q_y)
     constexpr int RV = tan_row_variant<T>(NS);
-    launch_row_fwd<T, LR, true, RV>(LoadRealRows<T>{q, NS, N}, StoreTiled<T>{sp, NS, CT, bsp}, NS,
-                                   s, nullptr, 2);
+    launch_row_fwd<T, LR, true, RV>(ld, StoreTiled<T>{sp, NS, CT, bsp}, nd, s, nullptr, 2);
     {
         constexpr int thr = 2 * CT * (LC / col_rpt<T>(LC, 0));
         constexpr int sm = col_pair_pp<T>(LC, CT) ? 2 * align16(col_smem<T>(LC, 2 * CT))
@@ -436,49 +436,42 @@ void TanOperator::apply(const T* q, T* u, cudaStream_t s) {
         fft_attrs((const void*)k, sm);
         const TanMix<T> mix{static_cast<const T*>(kt[dbl][0]), static_cast<const T*>(kt[dbl][1]),
                             static_cast<const T*>(kt[dbl][2]), NS + 1, CT, LC};
-        launch_pdl(k, dim3(NS / CT + 1), thr, sm, s, sp, bsp, NS, mix, tw<T>(LC));
+        launch_pdl(k, dim3(NS / CT + 1), thr, sm, s, sp, bsp, NS, nd, mix, tw<T>(LC));
     }
-    launch_row_inv<T, LR, true, RV>(LoadTiled<T>{sp, NS, CT, bsp}, StoreRealRows<T>{u, NS, N}, NS,
-                                   s, nullptr, 2);
+    launch_row_inv<T, LR, true, RV>(LoadTiled<T>{sp, NS, CT, bsp}, st, nd, s, nullptr, 2);
     count_launches(3);
     ASB_CUDA(cudaGetLastError());
 }
 
+template <typename T, int NS>
+void TanOperator::apply_full(const T* q, T* u, cudaStream_t s) {
+    const long N = (long)NS * NS;
+    apply<T, NS>(LoadRealRows<T>{q, NS, N}, StoreRealRows<T>{u, NS, N}, NS, s);
+}
+
+// embedded: the row passes read and write the caller's rows themselves
+template <typename T, int NS>
+void TanOperator::apply_block(const T* q, T* u, cudaStream_t s) {
+    const long nl = (long)Nl * Nl;
+    apply<T, NS>(LoadBlockRows<T>{q, Nl, nl}, StoreBlockRows<T>{u, Nl, nl}, Nl, s);
+}
+
 void TanOperator::matvec(bool dbl, const void* q, void* u, cudaStream_t s) {
     if (dbl) {
-        ASB_TAN_SIZE_SWITCH(Ns, (apply<double, NS>((const double*)q, (double*)u, s)));
+        ASB_TAN_SIZE_SWITCH(Ns, (apply_full<double, NS>((const double*)q, (double*)u, s)));
     } else {
-        ASB_TAN_SIZE_SWITCH(Ns, (apply<float, NS>((const float*)q, (float*)u, s)));
+        ASB_TAN_SIZE_SWITCH(Ns, (apply_full<float, NS>((const float*)q, (float*)u, s)));
     }
 }
 
 void TanOperator::apply_caller(bool dbl, const void* q, void* u, cudaStream_t s) {
     if (!embedded()) {
         matvec(dbl, q, u, s);
-        return;
-    }
-    const long n = (long)Ns * Ns, nl = (long)Nl * Nl;
-    if (!emb_q) {
-        std::lock_guard<std::recursive_mutex> setup(setup_mutex());
-        ASB_CUDA(cudaMalloc(&emb_q, 2 * n * sizeof(double)));
-        ASB_CUDA(cudaMalloc(&emb_u, 2 * n * sizeof(double)));
-    }
-    if (dbl) {
-        k_embed<double, double><<<embed_grid(2 * n), 256, 0, s>>>(Nl, Ns, 2, (const double*)q,
-                                                                  (double*)emb_q, 0.0);
-        matvec(true, emb_q, emb_u, s);
-        k_extract<double, double><<<embed_grid(2 * nl), 256, 0, s>>>(Nl, Ns, 2,
-                                                                     (const double*)emb_u,
-                                                                     (double*)u);
+    } else if (dbl) {
+        ASB_TAN_SIZE_SWITCH(Ns, (apply_block<double, NS>((const double*)q, (double*)u, s)));
     } else {
-        k_embed<float, float><<<embed_grid(2 * n), 256, 0, s>>>(Nl, Ns, 2, (const float*)q,
-                                                                (float*)emb_q, 0.0f);
-        matvec(false, emb_q, emb_u, s);
-        k_extract<float, float><<<embed_grid(2 * nl), 256, 0, s>>>(Nl, Ns, 2,
-                                                                   (const float*)emb_u, (float*)u);
+        ASB_TAN_SIZE_SWITCH(Ns, (apply_block<float, NS>((const float*)q, (float*)u, s)));
     }
-    count_launches(2);
-    ASB_CUDA(cudaGetLastError());
 }
 
 }  // namespace asb

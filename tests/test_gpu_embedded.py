@@ -243,3 +243,22 @@ def test_embedded_solve_with_fourier_preconditioner(backend):
     assert _rel(r.pressure, o.pressure) <= 10 * tol
     assert abs(r.contact_area - o.contact_area) <= 1e-4
     assert abs(r.iterations - o.iterations) <= 6
+
+
+@pytest.mark.parametrize("backend", ["fft", "periodic"])
+@pytest.mark.parametrize("Ns", [17, 33, 100, 255, 520])
+def test_embedded_apply_leaves_nothing_behind(backend, Ns):
+    """The passes of an embedded operator run on the caller's rows alone, so
+    the spectrum rows past them keep what the last call left: an apply after
+    another one, after an FP32 one and after a solve on the same operator
+    equals the first apply of a fresh operator bit for bit."""
+    import aspher_b200 as asb
+    n = Ns * Ns
+    for dtype in (torch.float64, torch.float32):
+        x = torch.randn(n, dtype=dtype, device="cuda")
+        want = asb.Operator(backend, Ns).matvec_(x, torch.empty_like(x))
+        op = asb.Operator(backend, Ns)
+        op.matvec_(1e3 * torch.randn(n, dtype=dtype, device="cuda"), torch.empty_like(x))
+        assert torch.equal(op.matvec_(x, torch.empty_like(x)), want)
+        asb.solve_device_mixed(op, torch.as_tensor(_gap(Ns), device="cuda"), 0.01, tol=1e-6)
+        assert torch.equal(op.matvec_(x, torch.empty_like(x)), want)

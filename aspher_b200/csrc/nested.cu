@@ -13,6 +13,7 @@
 #include "common.cuh"
 #include "ops.hpp"
 #include "pcg.hpp"
+#include "reduce.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -53,32 +54,38 @@ __global__ void k_prolong(int Nc, const double* __restrict__ pc, double* __restr
     }
 }
 
-__global__ void k_minmax_f64(long n, const double* __restrict__ x, double* out3) {
-    // single block: min, max, count of non-finite values
-    double mn = INFINITY, mx = -INFINITY, nf = 0.0;
-    for (long i = threadIdx.x; i < n; i += blockDim.x) {
+// out[0..2] = min, max, count of non-finite values of x; out holds
+// kMinMaxDoubles values (the blocks' counter and partials behind the result).
+// One block took 0.77 ms on 2048 x 2048 values; 296 read them at 5 us.
+constexpr int kMinMaxBlocks = 296;
+constexpr int kMinMaxDoubles = 4 + 3 * kMinMaxBlocks;
+__global__ void __launch_bounds__(kRedThreads) k_minmax_f64(long n, const double* __restrict__ x,
+                                                            double* out) {
+    double acc[3] = {(double)INFINITY, -(double)INFINITY, 0.0};
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
+         i += (long)gridDim.x * blockDim.x) {
         const double v = x[i];
-        mn = fmin(mn, v);
-        mx = fmax(mx, v);
-        if (!isfinite(v)) nf += 1.0;
+        acc[0] = fmin(acc[0], v);
+        acc[1] = fmax(acc[1], v);
+        if (!isfinite(v)) acc[2] += 1.0;
     }
-    __shared__ double s[3][32];
-    mn = warp_min(mn);
-    mx = warp_max(mx);
-    nf = warp_sum(nf);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) { s[0][wid] = mn; s[1][wid] = mx; s[2][wid] = nf; }
-    __syncthreads();
-    if (wid == 0) {
-        const int nw = blockDim.x / 32;
-        mn = lane < nw ? s[0][lane] : INFINITY;
-        mx = lane < nw ? s[1][lane] : -INFINITY;
-        nf = lane < nw ? s[2][lane] : 0.0;
-        mn = warp_min(mn);
-        mx = warp_max(mx);
-        nf = warp_sum(nf);
-        if (lane == 0) { out3[0] = mn; out3[1] = mx; out3[2] = nf; }
+    const int kinds[3] = {1, 2, 0};
+    if (grid_reduce_last<3>(acc, kinds, out + 4, reinterpret_cast<unsigned*>(out + 3)) &&
+        threadIdx.x == 0) {
+        out[0] = acc[0];
+        out[1] = acc[1];
+        out[2] = acc[2];
     }
+}
+// its launch: mm[0..2] on the host, after a synchronisation of the stream
+void minmax_f64(long n, const double* x, double* dev, double (&mm)[3], cudaStream_t s) {
+    ASB_CUDA(cudaMemsetAsync(dev, 0, 4 * sizeof(double), s));
+    const long nb = std::min<long>(kMinMaxBlocks, (n + kRedThreads - 1) / kRedThreads);
+    k_minmax_f64<<<(unsigned)nb, kRedThreads, 0, s>>>(n, x, dev);
+    count_launches(1);
+    ASB_CUDA(cudaGetLastError());
+    ASB_CUDA(cudaMemcpyAsync(mm, dev, sizeof(mm), cudaMemcpyDeviceToHost, s));
+    ASB_CUDA(cudaStreamSynchronize(s));
 }
 
 // ---- active set (restricted levels) ------------------------------------------
@@ -283,21 +290,19 @@ void active_level(Operator& op, const aspher_solve_opts& o, bool level_float, co
             if (v) cudaFreeAsync(v, s);
     };
     try {
-        ASB_CUDA(cudaMallocAsync((void**)&cm, n2, s));
-        ASB_CUDA(cudaMallocAsync((void**)&tmp, n2, s));
-        ASB_CUDA(cudaMallocAsync((void**)&viol, n2, s));
-        ASB_CUDA(cudaMallocAsync((void**)&ga, n2 * sizeof(double), s));
-        ASB_CUDA(cudaMallocAsync((void**)&pw, n2 * sizeof(double), s));
-        ASB_CUDA(cudaMallocAsync((void**)&part, 3 * (size_t)gb * sizeof(double), s));
-        ASB_CUDA(cudaMallocAsync((void**)&mm_d, 3 * sizeof(double), s));
-        ASB_CUDA(cudaMallocAsync(&u, n2 * (level_float ? sizeof(float) : sizeof(double)), s));
-        if (level_float) ASB_CUDA(cudaMallocAsync((void**)&p32, n2 * sizeof(float), s));
+        ASB_CUDA(scratch_alloc((void**)&cm, n2, s));
+        ASB_CUDA(scratch_alloc((void**)&tmp, n2, s));
+        ASB_CUDA(scratch_alloc((void**)&viol, n2, s));
+        ASB_CUDA(scratch_alloc((void**)&ga, n2 * sizeof(double), s));
+        ASB_CUDA(scratch_alloc((void**)&pw, n2 * sizeof(double), s));
+        ASB_CUDA(scratch_alloc((void**)&part, 3 * (size_t)gb * sizeof(double), s));
+        ASB_CUDA(scratch_alloc((void**)&mm_d, kMinMaxDoubles * sizeof(double), s));
+        ASB_CUDA(scratch_alloc((void**)&u, n2 * (level_float ? sizeof(float) : sizeof(double)), s));
+        if (level_float) ASB_CUDA(scratch_alloc((void**)&p32, n2 * sizeof(float), s));
 
         // the level gap's range sets delta and the violation threshold
-        k_minmax_f64<<<1, 1024, 0, s>>>(n2, glvl, mm_d);
         double mm[3];
-        ASB_CUDA(cudaMemcpyAsync(mm, mm_d, sizeof(mm), cudaMemcpyDeviceToHost, s));
-        ASB_CUDA(cudaStreamSynchronize(s));
+        minmax_f64(n2, glvl, mm_d, mm, s);
         const double g_scale = mm[1] > mm[0] ? mm[1] - mm[0] : 1.0;
         const double delta = np.active_delta * g_scale;
         const double vthresh = -lvl_tol * g_scale;
@@ -525,12 +530,9 @@ void solve_nested(int kind, int Ns, double L, double E, const double* g0, double
     const long N = (long)Ns * Ns;
     // gap statistics (FP64) -> datum and g_ref (nested_solve.cpp:634-636)
     double* mm_d = nullptr;
-    ASB_CUDA(cudaMallocAsync((void**)&mm_d, 3 * sizeof(double), s));
-    k_minmax_f64<<<1, 1024, 0, s>>>(N, g0, mm_d);
-    count_launches(1);
+    ASB_CUDA(scratch_alloc((void**)&mm_d, kMinMaxDoubles * sizeof(double), s));
     double mm[3];
-    ASB_CUDA(cudaMemcpyAsync(mm, mm_d, sizeof(mm), cudaMemcpyDeviceToHost, s));
-    ASB_CUDA(cudaStreamSynchronize(s));
+    minmax_f64(N, g0, mm_d, mm, s);
     cudaFreeAsync(mm_d, s);
     if (mm[2] > 0.0) throw Error(ASPHER_EINVAL, "solve_contact_nested: gap contains non-finite values");
     const double datum = mm[0] + 0.5 * (mm[1] - mm[0]);
@@ -541,7 +543,7 @@ void solve_nested(int kind, int Ns, double L, double E, const double* g0, double
     std::vector<double*> gaps(ncoarse, nullptr);
     for (int i = ncoarse - 1; i >= 0; --i) {
         const int n = levels[i];
-        ASB_CUDA(cudaMallocAsync((void**)&gaps[i], (size_t)n * n * sizeof(double), s));
+        ASB_CUDA(scratch_alloc((void**)&gaps[i], (size_t)n * n * sizeof(double), s));
         const double* src = (i == ncoarse - 1) ? g0 : gaps[i + 1];
         k_restrict<<<std::min(1184L, ((long)n * n + 255) / 256), 256, 0, s>>>(2 * n, src, gaps[i]);
         count_launches(1);
@@ -628,11 +630,11 @@ void solve_nested(int kind, int Ns, double L, double E, const double* g0, double
             o.precond = pc;
             o.precond_radius = r_lvl;
 
-            ASB_CUDA(cudaMallocAsync((void**)&p_lvl, (size_t)Nl * sizeof(double), s));
+            ASB_CUDA(scratch_alloc((void**)&p_lvl, (size_t)Nl * sizeof(double), s));
             double* dout = finest ? disp : nullptr;
             double* gout = finest ? gap : nullptr;
             if (keep_gap) {
-                ASB_CUDA(cudaMallocAsync((void**)&gap_keep, (size_t)Nl * sizeof(double), s));
+                ASB_CUDA(scratch_alloc((void**)&gap_keep, (size_t)Nl * sizeof(double), s));
                 gout = gap_keep;
             }
             double* hout = o.record_history ? hist_host : nullptr;
@@ -700,7 +702,7 @@ void solve_nested(int kind, int Ns, double L, double E, const double* g0, double
             }
             if (!finest) {
                 t_coarse += r.time_total;
-                ASB_CUDA(cudaMallocAsync((void**)&p_init, (size_t)4 * Nl * sizeof(double), s));
+                ASB_CUDA(scratch_alloc((void**)&p_init, (size_t)4 * Nl * sizeof(double), s));
                 k_prolong<<<std::min(1184L, (Nl + 255) / 256), 256, 0, s>>>(n, p_lvl, p_init);
                 count_launches(1);
                 ASB_CUDA(cudaGetLastError());

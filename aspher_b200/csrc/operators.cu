@@ -86,6 +86,47 @@ std::atomic<long long> g_launches{0};
 void count_launches(long n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
+namespace {
+std::mutex g_pool_mu;
+cudaMemPool_t g_pool[64] = {};  // per device
+std::atomic<int> g_live_ops{0};
+}  // namespace
+
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    cudaMemPool_t pool = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(g_pool_mu);
+        if (!g_pool[dev]) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            cudaMemPool_t made = nullptr;
+            e = cudaMemPoolCreate(&made, &props);
+            if (e != cudaSuccess) return e;
+            unsigned long long keep = kScratchKeep;
+            e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
+            if (e != cudaSuccess) {
+                cudaMemPoolDestroy(made);
+                return e;
+            }
+            g_pool[dev] = made;
+        }
+        pool = g_pool[dev];
+    }
+    return cudaMallocFromPoolAsync(p, bytes, pool, s);
+}
+
+void scratch_trim() {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    for (cudaMemPool_t pool : g_pool)
+        if (pool) cudaMemPoolTrimTo(pool, 0);
+}
+
 void smem_optin(const void* func, int bytes) {
     if (bytes <= 48 * 1024) return;
     ASB_CUDA(cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
@@ -589,10 +630,12 @@ Operator::Operator(int kind_, int Ns_, double L_, double E_, int flags)
         set_variants(dbl != 0, rv, cv);
     }
     ASB_CUDA(cudaDeviceSynchronize());
+    g_live_ops.fetch_add(1);
 }
 
 Operator::~Operator() {
     std::lock_guard<std::recursive_mutex> setup(setup_mutex());
+    if (g_live_ops.fetch_sub(1) == 1) scratch_trim();
     ctx_f.reset();
     ctx_d.reset();
     cudaFree(khp_canon);

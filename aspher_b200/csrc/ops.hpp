@@ -78,6 +78,17 @@ void tuned_variants(int kind, int dbl, int Ns, int& rv, int& cv);
 // cudaDeviceSynchronize / blocking copies).  Recursive: set-up paths nest.
 std::recursive_mutex& setup_mutex();
 
+// Stream-ordered scratch of the host drivers (freed with cudaFreeAsync), from
+// a pool of the library's own on the current device.  The default pool gives
+// every freed byte back to the driver at the next synchronisation, and these
+// drivers synchronise: a nested call to 2048 x 2048 in FP64, 37 ms of kernels,
+// took 44-160 ms and once 1.2 s, mapping its 150 MB anew.  This pool keeps up
+// to kScratchKeep bytes between calls; scratch_trim() gives them back (the
+// last operator's end does).  Safe from any thread and stream.
+constexpr size_t kScratchKeep = size_t(1) << 30;
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
+void scratch_trim();
+
 // Opt into >48 KB dynamic shared memory once per kernel per device.
 void smem_optin(const void* func, int bytes);
 

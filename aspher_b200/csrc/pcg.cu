@@ -2032,7 +2032,7 @@ struct EmbedIO {
     template <typename T>
     T* alloc() {
         void* p = nullptr;
-        ASB_CUDA(cudaMallocAsync(&p, (size_t)n() * sizeof(T), s));
+        ASB_CUDA(scratch_alloc((void**)&p, (size_t)n() * sizeof(T), s));
         bufs.push_back(p);
         return static_cast<T*>(p);
     }
@@ -2312,9 +2312,9 @@ void precond_apply_impl(Operator& op, int precond, int radius, const T* g_in,
     T* z = z_out;
     void* tmp[3] = {nullptr, nullptr, nullptr};
     if (op.embedded()) {
-        ASB_CUDA(cudaMallocAsync(&tmp[0], (size_t)N * sizeof(T), s));
-        ASB_CUDA(cudaMallocAsync(&tmp[1], (size_t)N, s));
-        ASB_CUDA(cudaMallocAsync(&tmp[2], (size_t)N * sizeof(T), s));
+        ASB_CUDA(scratch_alloc((void**)&tmp[0], (size_t)N * sizeof(T), s));
+        ASB_CUDA(scratch_alloc((void**)&tmp[1], (size_t)N, s));
+        ASB_CUDA(scratch_alloc((void**)&tmp[2], (size_t)N * sizeof(T), s));
         k_embed<T, T><<<embed_grid(N), 256, 0, s>>>(op.Nl, op.Ns, 1, g_in, (T*)tmp[0], T(0));
         k_embed<uint8_t, uint8_t><<<embed_grid(N), 256, 0, s>>>(op.Nl, op.Ns, 1, mask_in,
                                                                 (uint8_t*)tmp[1], 0);
@@ -2325,8 +2325,8 @@ void precond_apply_impl(Operator& op, int precond, int radius, const T* g_in,
     }
     PkState* st = nullptr;
     double* part = nullptr;
-    ASB_CUDA(cudaMallocAsync((void**)&st, sizeof(PkState), s));
-    ASB_CUDA(cudaMallocAsync((void**)&part, kPartStride * sizeof(double), s));
+    ASB_CUDA(scratch_alloc((void**)&st, sizeof(PkState), s));
+    ASB_CUDA(scratch_alloc((void**)&part, kPartStride * sizeof(double), s));
     ASB_CUDA(cudaMemsetAsync(st, 0, sizeof(PkState), s));  // alpha = 0: g used as given
     PkParams P{};
     P.N = N;
@@ -2335,7 +2335,7 @@ void precond_apply_impl(Operator& op, int precond, int radius, const T* g_in,
     P.Nl = op.Nl;
     P.precond = precond;
     PkParams* Pd = nullptr;
-    ASB_CUDA(cudaMallocAsync((void**)&Pd, sizeof(PkParams), s));
+    ASB_CUDA(scratch_alloc((void**)&Pd, sizeof(PkParams), s));
     ASB_CUDA(cudaMemcpyAsync(Pd, &P, sizeof(PkParams), cudaMemcpyHostToDevice, s));
     const int grid = red_grid(N);
     k_gmean<T><<<grid, kRedThreads, 0, s>>>(N, st, g, mask, part);
@@ -2597,11 +2597,11 @@ void adjoint_core(Operator& op, const double* p, const double* w, double tol, in
     PkState* st = nullptr;
     PkParams* Pd = nullptr;
     T** vecs[] = {&wT, &r, &z, &d, &q, &lam};
-    for (T** v : vecs) ASB_CUDA(cudaMallocAsync((void**)v, vb, s));
-    ASB_CUDA(cudaMallocAsync((void**)&mask, (size_t)N, s));
-    ASB_CUDA(cudaMallocAsync((void**)&part, kPartStride * sizeof(double), s));
-    ASB_CUDA(cudaMallocAsync((void**)&st, sizeof(PkState), s));
-    ASB_CUDA(cudaMallocAsync((void**)&Pd, sizeof(PkParams), s));
+    for (T** v : vecs) ASB_CUDA(scratch_alloc((void**)v, vb, s));
+    ASB_CUDA(scratch_alloc((void**)&mask, (size_t)N, s));
+    ASB_CUDA(scratch_alloc((void**)&part, kPartStride * sizeof(double), s));
+    ASB_CUDA(scratch_alloc((void**)&st, sizeof(PkState), s));
+    ASB_CUDA(scratch_alloc((void**)&Pd, sizeof(PkParams), s));
     ASB_CUDA(cudaMemsetAsync(st, 0, sizeof(PkState), s));
     PkParams P{};
     P.N = N;

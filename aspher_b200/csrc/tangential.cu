@@ -1342,7 +1342,7 @@ void solve_tangential(TanOperator& op, const double* s, bool force_control, doub
     std::vector<double*> bufs;
     auto alloc = [&](long count) {
         double* p = nullptr;
-        ASB_CUDA(cudaMallocAsync((void**)&p, (size_t)count * sizeof(double), st));
+        ASB_CUDA(scratch_alloc((void**)&p, (size_t)count * sizeof(double), st));
         bufs.push_back(p);
         return p;
     };

@@ -16,9 +16,10 @@ void free_apply_block<float>(const Operator& op, const float* x, float* y, cplx<
 }
 
 template <>
-void embedded_precond<float>(Operator& op, const float* g, const uint8_t* mask, PkState* st, float* z,
+void embedded_precond<float>(Operator& op, const float* ga, const float* gb, const uint8_t* mask, PkState* st,
+                        float* z,
                          double* part, cudaStream_t s, const int* gate, int B, void* spec) {
-    ASB_SIZE_SWITCH(op.Ns, (EmbeddedFourierImpl<float, NS>::run(op, g, mask, st, z, part, s, gate, B,
+    ASB_SIZE_SWITCH(op.Ns, (EmbeddedFourierImpl<float, NS>::run(op, ga, gb, mask, st, z, part, s, gate, B,
                                                             spec)));
 }
 

@@ -16,9 +16,10 @@ void free_apply_block<double>(const Operator& op, const double* x, double* y, cp
 }
 
 template <>
-void embedded_precond<double>(Operator& op, const double* g, const uint8_t* mask, PkState* st, double* z,
+void embedded_precond<double>(Operator& op, const double* ga, const double* gb, const uint8_t* mask, PkState* st,
+                        double* z,
                          double* part, cudaStream_t s, const int* gate, int B, void* spec) {
-    ASB_SIZE_SWITCH(op.Ns, (EmbeddedFourierImpl<double, NS>::run(op, g, mask, st, z, part, s, gate, B,
+    ASB_SIZE_SWITCH(op.Ns, (EmbeddedFourierImpl<double, NS>::run(op, ga, gb, mask, st, z, part, s, gate, B,
                                                             spec)));
 }
 

@@ -228,7 +228,8 @@ template <typename T>
 struct LoadMaskCentered {  // contact ? g - T(gsum/ng) : 0, pairwise; g = v - T(alpha)
     static constexpr bool kTiled = false;
     static constexpr bool kRaw = false;
-    const T* g;
+    const T* ga;  // the gap is in ga or gb (PkState::par)
+    const T* gb;
     const uint8_t* mask;
     const PkState* st;
     int pitch;
@@ -241,7 +242,7 @@ struct LoadMaskCentered {  // contact ? g - T(gsum/ng) : 0, pairwise; g = v - T(
         // alpha is 0 for the standalone preconditioner)
         const T aT = (T)sb->alpha;
         const size_t i = blockIdx.y * bs + (size_t)row * pitch + 2 * n;
-        const cplx<T> v = *reinterpret_cast<const cplx<T>*>(g + i);
+        const cplx<T> v = *reinterpret_cast<const cplx<T>*>((sb->par ? gb : ga) + i);
         const uchar2 m = *reinterpret_cast<const uchar2*>(mask + i);
         return mk<T>(m.x ? (T)((T)(v.x - aT) - gm) : T(0), m.y ? (T)((T)(v.y - aT) - gm) : T(0));
     }
@@ -292,14 +293,15 @@ struct StoreGather {  // z = contact ? G : 0; contact sum of G -> zmean
 template <typename T, int NS>
 struct FourierImpl {
     using PI = PeriodicImpl<T, NS>;
-    static void run(Operator& op, const T* g, const uint8_t* mask, PkState* st, T* z,
+    static void run(Operator& op, const T* ga, const T* gb, const uint8_t* mask, PkState* st,
+                        T* z,
                     double* part, cudaStream_t s, const int* gate, int B, void* spec_b) {
         cplx<T>* spec = static_cast<cplx<T>*>(spec_b ? spec_b : op.spectrum(sizeof(T) == 8, s));
         int rv = 0, cv = 0;
         tuned_variants(OP_PERIODIC, sizeof(T) == 8, NS, rv, cv);
         const float norm = 1.0f / ((float)NS * (float)NS);
         const long bx = (long)NS * NS;
-        PI::apply(rv, cv, LoadMaskCentered<T>{g, mask, st, NS, bx}, FourierMult<T>{NS, norm},
+        PI::apply(rv, cv, LoadMaskCentered<T>{ga, gb, mask, st, NS, bx}, FourierMult<T>{NS, norm},
                   StoreGather<T>{z, mask, NS, st, part, bx, 0.0}, spec, s, gate, B);
     }
 };
@@ -310,14 +312,15 @@ struct FourierImpl {
 // sum (the same load and store as the periodic form)
 template <typename T, int NS>
 struct EmbeddedFourierImpl {
-    static void run(Operator& op, const T* g, const uint8_t* mask, PkState* st, T* z,
+    static void run(Operator& op, const T* ga, const T* gb, const uint8_t* mask, PkState* st,
+                        T* z,
                     double* part, cudaStream_t s, const int* gate, int B, void* spec_b) {
         if (!op.khp_canon)
             throw Error(-1, "fourier-fft preconditioner spectrum not built (set-up order)");
         cplx<T>* spec = static_cast<cplx<T>*>(spec_b ? spec_b : op.spectrum(sizeof(T) == 8, s));
         const long bx = (long)NS * NS;
         const T* kh = sizeof(T) == 8 ? (const T*)op.khp_d : (const T*)op.khp_f;
-        FreeImpl<T, NS>::apply(op, LoadMaskCentered<T>{g, mask, st, NS, bx},
+        FreeImpl<T, NS>::apply(op, LoadMaskCentered<T>{ga, gb, mask, st, NS, bx},
                                StoreGather<T>{z, mask, NS, st, part, bx, 0.0}, spec, s, gate, B,
                                kh);
     }
@@ -351,7 +354,8 @@ void free_apply_block(const Operator& op, const T* x, T* y, cplx<T>* spec, cudaS
 void free_defect(const Operator& op, LoadDiffRows ld, StoreAddRows st, float2* spec,
                  cudaStream_t s, const int* gate, int B);
 template <typename T>
-void embedded_precond(Operator& op, const T* g, const uint8_t* mask, PkState* st, T* z,
+void embedded_precond(Operator& op, const T* ga, const T* gb, const uint8_t* mask, PkState* st,
+                        T* z,
                       double* part, cudaStream_t s, const int* gate, int B, void* spec);
 template <typename T>
 void periodic_matvec(const Operator& op, const T* x, T* y, cplx<T>* spec, cudaStream_t s,
@@ -359,7 +363,8 @@ void periodic_matvec(const Operator& op, const T* x, T* y, cplx<T>* spec, cudaSt
 void periodic_defect(const Operator& op, LoadDiffRows ld, StoreAddRows st, float2* spec,
                      cudaStream_t s, const int* gate, int B);
 template <typename T>
-void periodic_precond(Operator& op, const T* g, const uint8_t* mask, PkState* st, T* z,
+void periodic_precond(Operator& op, const T* ga, const T* gb, const uint8_t* mask, PkState* st,
+                        T* z,
                       double* part, cudaStream_t s, const int* gate, int B, void* spec);
 
 }  // namespace asb

@@ -11,9 +11,10 @@ void periodic_matvec<float>(const Operator& op, const float* x, float* y, cplx<f
 }
 
 template <>
-void periodic_precond<float>(Operator& op, const float* g, const uint8_t* mask, PkState* st, float* z,
+void periodic_precond<float>(Operator& op, const float* ga, const float* gb, const uint8_t* mask, PkState* st,
+                        float* z,
                          double* part, cudaStream_t s, const int* gate, int B, void* spec) {
-    ASB_SIZE_SWITCH(op.Ns, (FourierImpl<float, NS>::run(op, g, mask, st, z, part, s, gate, B, spec)));
+    ASB_SIZE_SWITCH(op.Ns, (FourierImpl<float, NS>::run(op, ga, gb, mask, st, z, part, s, gate, B, spec)));
 }
 
 void periodic_defect(const Operator& op, LoadDiffRows ld, StoreAddRows st, float2* spec,

@@ -11,9 +11,10 @@ void periodic_matvec<double>(const Operator& op, const double* x, double* y, cpl
 }
 
 template <>
-void periodic_precond<double>(Operator& op, const double* g, const uint8_t* mask, PkState* st, double* z,
+void periodic_precond<double>(Operator& op, const double* ga, const double* gb, const uint8_t* mask, PkState* st,
+                        double* z,
                          double* part, cudaStream_t s, const int* gate, int B, void* spec) {
-    ASB_SIZE_SWITCH(op.Ns, (FourierImpl<double, NS>::run(op, g, mask, st, z, part, s, gate, B, spec)));
+    ASB_SIZE_SWITCH(op.Ns, (FourierImpl<double, NS>::run(op, ga, gb, mask, st, z, part, s, gate, B, spec)));
 }
 
 }  // namespace asb

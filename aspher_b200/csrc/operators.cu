@@ -892,14 +892,15 @@ void Operator::ensure_precond_spectrum() {
 }
 
 template <typename T>
-void fourier_precond_pk(Operator& op, const T* g, const uint8_t* mask, PkState* st, T* z,
+void fourier_precond_pk(Operator& op, const T* ga, const T* gb, const uint8_t* mask, PkState* st,
+                        T* z,
                         double* part, cudaStream_t s, const int* gate, int B, void* spec) {
-    if (op.embedded()) embedded_precond<T>(op, g, mask, st, z, part, s, gate, B, spec);
-    else periodic_precond<T>(op, g, mask, st, z, part, s, gate, B, spec);
+    if (op.embedded()) embedded_precond<T>(op, ga, gb, mask, st, z, part, s, gate, B, spec);
+    else periodic_precond<T>(op, ga, gb, mask, st, z, part, s, gate, B, spec);
 }
-template void fourier_precond_pk<float>(Operator&, const float*, const uint8_t*, PkState*, float*,
+template void fourier_precond_pk<float>(Operator&, const float*, const float*, const uint8_t*, PkState*, float*,
                                         double*, cudaStream_t, const int*, int, void*);
-template void fourier_precond_pk<double>(Operator&, const double*, const uint8_t*, PkState*,
+template void fourier_precond_pk<double>(Operator&, const double*, const double*, const uint8_t*, PkState*,
                                          double*, double*, cudaStream_t, const int*, int, void*);
 
 }  // namespace asb

@@ -7,12 +7,18 @@
 //
 // One CG iteration is the kernel sequence
 //   [apply p->u] eval [evalpk] stencil+dots tupd [apply t->r] rden pupd
-// where each pass is one HBM sweep and each reduction's scalar logic runs in
-// the last block of its pass (see pk_state.hpp).  The loop is a CUDA graph
+// where each pass is one sweep and each reduction's scalar logic runs in the
+// last block of its pass (see pk_state.hpp).  Outside the contact set p, t
+// and the direction's dots are exactly zero, and a solve spends its
+// iterations at contact fractions of 1-30 %, so the passes read the mask (a
+// byte per cell) first and touch the fields of a group of four cells only
+// where the group has contact: at Ns = 2048 FP32 a pass that read 54-88 MB
+// reads the 4 MB of the mask and the contact's share of that.  The loop is a CUDA graph
 // with a while node; once a pass sets `halt`, the rest of the iteration is a
 // no-op.  Every kernel serves B instances at once (gridDim.y = B, instance
 // blockIdx.y reading its own parameters, state, partials and fields).
 #include "../../include/aspher_b200.h"
+#include "fft_launch.cuh"
 #include "ops.hpp"
 #include "pk_state.hpp"
 #include "pcg.hpp"
@@ -78,6 +84,37 @@ __device__ __forceinline__ void stm4(uint8_t* m, long i4, const uint8_t (&a)[4])
     reinterpret_cast<uchar4*>(m)[i4] = make_uchar4(a[0], a[1], a[2], a[3]);
 }
 
+__device__ __forceinline__ uint32_t ldm4w(const uint8_t* m, long i4) {
+    return reinterpret_cast<const uint32_t*>(m)[i4];
+}
+// Visits the groups i4 of four cells whose mask word is nonzero: f(i4, word).
+// The words of kAhead strides are loaded together, so a stretch without
+// contact costs one memory latency per kAhead strides and not one per stride.
+constexpr int kAhead = 4;
+template <class F>
+__device__ __forceinline__ void contact_groups(const uint8_t* mask, long n4, F&& f) {
+    const long step = (long)gridDim.x * blockDim.x;
+    for (long i0 = blockIdx.x * (long)blockDim.x + threadIdx.x; i0 < n4; i0 += kAhead * step) {
+        uint32_t w[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) w[k] = i0 + k * step < n4 ? ldm4w(mask, i0 + k * step) : 0u;
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k)
+            if (w[k]) f(i0 + k * step, w[k]);
+    }
+}
+__device__ __forceinline__ bool mbyte(uint32_t w, int j) { return (w >> (8 * j)) & 0xffu; }
+
+// the gap of the last evaluation and the one before it (PkState::par)
+template <typename T>
+__device__ __forceinline__ const T* gap_now(const PkState* st, const T* ga, const T* gb) {
+    return st->par ? gb : ga;
+}
+template <typename T>
+__device__ __forceinline__ const T* gap_before(const PkState* st, const T* ga, const T* gb) {
+    return st->par ? ga : gb;
+}
+
 #define GRID_LOOP4(N) \
     for (long i4 = blockIdx.x * (long)blockDim.x + threadIdx.x; i4 < (N) / 4; i4 += (long)gridDim.x * blockDim.x)
 
@@ -129,9 +166,10 @@ struct PScale {
     __device__ __forceinline__ T operator()(T x) const { return x * f + a; }
 };
 
-// One pass for evaluate() (contact_solver.cpp:263-303): v -> g buffer, the
-// contact mask, and the sums whose last-block logic is the certificate, the
-// convergence test and the best/stall bookkeeping (contact_solver.cpp:379-412).
+// One pass for evaluate() (contact_solver.cpp:263-303): v -> the gap buffer
+// that does not hold the last evaluation's (PkState::par), the contact mask,
+// and the sums whose last-block logic is the certificate, the convergence
+// test and the best/stall bookkeeping (contact_solver.cpp:379-412).
 // The second-pass sums of the reference are linear in the centring, so they
 // come from first-pass sums:
 //   gcs = sum_C Real(v - a)            -> sum_C v - n_C a
@@ -139,11 +177,16 @@ struct PScale {
 // with a = Real(alpha), m = Real(gmin) (equal up to the rounding of each
 // Real difference; in FP64 to ~1e-16 relative).  pk = sum p |g| is not
 // linear; k_evalpk computes it when a history is recorded and at the end.
+// The mask holds the cells whose stored p is not zero (k_pupd keeps it), so
+// p itself is read at those groups only; the contact is p > 0 after the
+// pending rescale, and a cell where the two differ is corrected here.  After
+// the host has written p (PkState::mask_stale) p is read everywhere.
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_eval(const PkParams* __restrict__ Pp, PkState* st,
-                                                      const T* u, const T* g0, const T* p, T* g,
-                                                      uint8_t* mask, double* part,
+                                                      const T* u, const T* g0, const T* p, T* ga,
+                                                      T* gb, uint8_t* mask, double* part,
                                                       int final_mode) {
+    pdl_wait();
     // instance blockIdx.y of a batched solve (0 when unbatched)
     Pp += blockIdx.y;
     st += blockIdx.y;
@@ -152,34 +195,41 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_eval(const PkPar
     u += bo_;
     g0 += bo_;
     p += bo_;
-    g += bo_;
     mask += bo_;
     const PkParams& P = *Pp;
     if (!final_mode && st->halt) return;
+    T* g = (st->par ? ga : gb) + bo_;
+    const bool stale = st->mask_stale != 0;
     const T gs = (T)P.gshift;
     const PScale<T> ps(st);
     double acc[5] = {0.0, 0.0, (double)INFINITY, 0.0, 0.0};  // sum_C v, n_C, min v, pv, psum
     GRID_LOOP4(P.Nv) {
-        T uu[4], gg0[4], pp[4], vv[4];
-        uint8_t mm[4];
+        T uu[4], gg0[4], pp[4] = {T(0), T(0), T(0), T(0)}, vv[4];
+        const uint32_t mw = stale ? 1u : ldm4w(mask, i4);
         ldp4(u, i4, uu);
         ldp4(g0, i4, gg0);
-        ldp4(p, i4, pp);
+        if (mw) {
+            ldp4(p, i4, pp);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) pp[j] = ps(pp[j]);
+            for (int j = 0; j < 4; ++j) pp[j] = ps(pp[j]);
+        }
+        uint32_t mn = 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const T v = uu[j] + (gg0[j] - gs);
             vv[j] = v;
             const double vd = (double)v, pd = (double)pp[j];
             acc[2] = fmin(acc[2], vd);
-            if (pp[j] > T(0)) { acc[0] += vd; acc[1] += 1.0; }
+            if (pp[j] > T(0)) {
+                acc[0] += vd;
+                acc[1] += 1.0;
+                mn |= 1u << (8 * j);
+            }
             acc[3] += pd * vd;
             acc[4] += pd;
-            mm[j] = pp[j] > T(0) ? 1 : 0;
         }
         st4(g, i4, vv);
-        stm4(mask, i4, mm);
+        if (stale || mn != mw) reinterpret_cast<uint32_t*>(mask)[i4] = mn;
     }
     const int kinds[5] = {0, 0, 1, 0, 0};
     if (grid_reduce_last<5>(acc, kinds, part, &st->counter[0]) && threadIdx.x == 0) {
@@ -197,6 +247,9 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_eval(const PkPar
         st->nc = nc;
         st->gsum = acc[0];
         st->vmin = acc[2];
+        st->par ^= 1;
+        st->mask_stale = 0;
+        st->alpha_prev = st->alpha;
         st->alpha = alpha;
         st->gmin = gmin;
         double ar = alpha, gr = gmin;
@@ -250,16 +303,18 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_eval(const PkPar
 // (pk_due) or in final mode.
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_evalpk(const PkParams* __restrict__ Pp, PkState* st,
-                                                        const T* p, const T* g, double* part,
-                                                        double* hist, int final_mode) {
+                                                        const T* p, const T* ga, const T* gb,
+                                                        double* part, double* hist,
+                                                        int final_mode) {
+    pdl_wait();
     Pp += blockIdx.y;
     st += blockIdx.y;
     part += (size_t)blockIdx.y * kPartStride;
     const long bo_ = (long)blockIdx.y * Pp->N;
     p += bo_;
-    g += bo_;
     const PkParams& P = *Pp;
     if (!final_mode && !st->pk_due) return;
+    const T* g = gap_now(st, ga, gb) + bo_;
     const T aT = (T)st->alpha;
     const PScale<T> ps(st);
     double acc[1] = {0.0};
@@ -282,10 +337,10 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_evalpk(const PkP
 
 // g <- centred gap (materialised for the host-side branches and the output)
 template <typename T>
-__global__ void k_center(const PkParams* __restrict__ Pp, const PkState* st, T* g) {
+__global__ void k_center(const PkParams* __restrict__ Pp, const PkState* st, T* ga, T* gb) {
     Pp += blockIdx.y;
     st += blockIdx.y;
-    g += (long)blockIdx.y * Pp->N;
+    T* g = (st->par ? gb : ga) + (long)blockIdx.y * Pp->N;
     const T aT = (T)st->alpha;
     GRID_LOOP4(Pp->Nv) {
         T gv[4];
@@ -309,13 +364,9 @@ __device__ __forceinline__ void beta_update(const PkParams& P, PkState* st, doub
 
 // ---- stencil preconditioner (stencil_precond.cpp:63-109) ---------------------
 // z = T(sum_t w_t gc(i + d_t)) on contact, gc = contact ? g - gmean : 0 with
-// periodic wrap; the contact mean of z is removed downstream.  A CTA of 256
-// threads owns a 64 x 32 tile of outputs whose (64 + 2R) x (32 + 2R) halo
-// of centred values sits in shared memory (FP64, as the reference
-// accumulates); thread (x, q) computes the 8 outputs (x, 8q .. 8q + 7) with
-// the disc's taps unrolled at compile time (R is a template parameter) and
-// summed in the reference's tap order (dy-major, dx-minor).
-constexpr int kStX = 64, kStY = 32, kStRows = 8, kMaxR = 4;
+// periodic wrap, accumulated in FP64 in the reference's tap order (dy-major,
+// dx-minor); the contact mean of z is removed downstream.
+constexpr int kMaxR = 4;
 
 // the disc's weights by signed offset, w[dy + kMaxR][dx + kMaxR] (even in
 // each offset on an even kernel grid; on an odd one the reference's
@@ -324,290 +375,207 @@ struct StencilW {
     double w[2 * kMaxR + 1][2 * kMaxR + 1];
 };
 
-// LAZY: g holds v uncentred (the solve loop; centred by Real(alpha) on the
-// fly), else g is used as given (standalone preconditioner, adjoint).
+// half width of the disc's row dy
+__host__ __device__ constexpr int disc_half(int R, int dy) {
+    int h = 0;
+    while ((h + 1) * (h + 1) + dy * dy <= R * R) ++h;
+    return h;
+}
+
+// A CTA scans the mask of a tile of `words` words per thread (four cells
+// each), lists the words with contact in shared memory in tile order, and its
+// threads then take one listed word each and gather its taps straight from
+// global memory (the neighbours are L1 lines that the CTA reads anyway).  At
+// the contact fractions of a solve a spot of contact is some ten cells wide
+// and most warps over consecutive cells would hold one or two: the list fills
+// the warps with contact alone.  What bounds the pass is the taps' FP64 work
+// and loads per cell in contact and, on small grids, the latency of mask,
+// list, taps and reduction.
+// FULL: full grids (the side Ns a power of two >= 16, wrapped by a bit mask,
+// 16-byte loads); else embedded grids, which wrap at the caller's side Nl at
+// any alignment.
+// LAZY: the gap buffers hold v uncentred (the solve loop; centred by
+// Real(alpha) on the fly) and z is needed on contact only; else ga is used as
+// given and z is 0 off contact (standalone preconditioner, adjoint).
 // DOTS: also the CG dots of the loop -- with zf = Real(z - zm) the
-// contact-mean-free direction,
-//   G = sum_C zf g,  G_pr = sum_C zf Real(g - gprev),  gg = sum_C g^2,
+// contact-mean-free direction and gp the centred gap of the evaluation before,
+//   G = sum_C zf g,  G_pr = sum_C zf Real(g - gp),  gg = sum_C g^2,
 // from sums linear in zm (zm is this pass's own reduction):
-//   G = sum_C z g - zm sum_C g,  G_pr = sum_C z (g - gprev) - zm sum_C (g - gprev).
-template <typename T, int R, bool LAZY, bool DOTS>
-__global__ void __launch_bounds__(256) k_stencil_t(const PkParams* __restrict__ Pp, PkState* st,
-                                                   StencilW W, const T* g, const T* gprev,
-                                                   const uint8_t* mask, T* z, double* part,
-                                                   int gated) {
+//   G = sum_C z g - zm sum_C g,  G_pr = sum_C z (g - gp) - zm sum_C (g - gp).
+constexpr int kStMaxWords = 16;  // words per thread of the largest tile (16, 4 or 1)
+template <typename T, int R, bool LAZY, bool DOTS, bool FULL>
+__global__ void __launch_bounds__(256, 2) k_stencil(const PkParams* __restrict__ Pp, PkState* st,
+                                                    const __grid_constant__ StencilW W,
+                                                    const T* ga, const T* gb,
+                                                    const uint8_t* mask, T* z, double* part,
+                                                    int gated, int words) {
+    __shared__ uint16_t list[256 * kStMaxWords];
+    __shared__ int wtot[8];
+    pdl_wait();
     // instance blockIdx.y of a batched solve (0 when unbatched)
     Pp += blockIdx.y;
     st += blockIdx.y;
     part += (size_t)blockIdx.y * kPartStride;
     const long bo_ = (long)blockIdx.y * Pp->N;
-    g += bo_;
     mask += bo_;
     z += bo_;
-    if (DOTS) gprev += bo_;
     const PkParams& P = *Pp;
     if (gated && st->halt) return;
-    constexpr int TW = kStX + 2 * R, TH = kStY + 2 * R;
-    __shared__ double tile[TH * TW];
-    // Nw: the periodic grid of the wrap (the caller's side; Ns, the row
-    // pitch, unless the operator is embedded)
+    const T* g = (LAZY ? gap_now(st, ga, gb) : ga) + bo_;
+    const T* gq = DOTS ? gap_before(st, ga, gb) + bo_ : nullptr;
     const int Ns = P.Ns, Nw = P.Nl;
-    // halo coordinates run from -R to the last tile's end (up to 63 + R past
-    // Nw); 2R + 1 <= Nw
-    auto wrap = [Nw](int v) { return v < 0 ? v + Nw : v % Nw; };
     const double gmean = st->nc ? st->gcs / st->nc : 0.0;
-    const T aT = LAZY ? (T)st->alpha : T(0);
-    const int ntx = (Nw + kStX - 1) / kStX, nty = (Nw + kStY - 1) / kStY;
-    const int tx = threadIdx.x % kStX, tq = threadIdx.x / kStX;
+    const T aT = LAZY ? (T)st->alpha : T(0), aq = DOTS ? (T)st->alpha_prev : T(0);
+    auto centred = [&](uint32_t m, T v) -> double {
+        return m ? (double)(LAZY ? (T)(v - aT) : v) - gmean : 0.0;
+    };
     // sum z (unrounded), sum zT g, sum g, sum zT (g - gp), sum (g - gp), sum g^2
     double acc[DOTS ? 6 : 1];
 #pragma unroll
     for (int i = 0; i < (DOTS ? 6 : 1); ++i) acc[i] = 0.0;
-    // each thread issues all of its loads before it uses any (none depends
-    // on another), so a tile costs about one memory latency, not one per
-    // element
-    constexpr int NL = (TW * TH + 255) / 256;  // halo elements per thread
-    for (int tid = blockIdx.x; tid < ntx * nty; tid += gridDim.x) {
-        const int tx0 = (tid % ntx) * kStX, ty0 = (tid / ntx) * kStY;
-        T hv[NL];
-        uint8_t hm[NL];
-#pragma unroll
-        for (int u = 0; u < NL; ++u) {
-            const int idx = threadIdx.x + u * 256;
-            if (idx < TW * TH) {
-                const int ly = idx / TW, lx = idx - ly * TW;
-                const int gy = wrap(ty0 + ly - R), gx = wrap(tx0 + lx - R);
-                const size_t j = (size_t)gy * Ns + gx;
-                hm[u] = mask[j];
-                hv[u] = g[j];
-            }
-        }
-        const int x = tx0 + tx;
-        const bool xin = x < Nw;
-        uint8_t om[kStRows];
-        T og[kStRows], op[kStRows];
-#pragma unroll
-        for (int k = 0; k < kStRows; ++k) {
-            const int y = ty0 + tq * kStRows + k;
-            const bool in = xin && y < Nw;
-            const size_t i = (size_t)(in ? y : 0) * Ns + (in ? x : 0);
-            om[k] = in ? mask[i] : 0;
-            og[k] = g[i];
-            if constexpr (DOTS) op[k] = gprev[i];
-        }
-#pragma unroll
-        for (int u = 0; u < NL; ++u) {
-            const int idx = threadIdx.x + u * 256;
-            if (idx < TW * TH)
-                tile[idx] = hm[u] ? (double)(LAZY ? (T)(hv[u] - aT) : hv[u]) - gmean : 0.0;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kStRows; ++k) {
-            const int ly = tq * kStRows + k, y = ty0 + ly;
-            if (!xin || y >= Nw) continue;
-            const size_t i = (size_t)y * Ns + x;
-            if (!om[k]) {
-                z[i] = T(0);
-                continue;
-            }
-            double a = 0.0;
-#pragma unroll
-            for (int dy = -R; dy <= R; ++dy)
-#pragma unroll
-                for (int dx = -R; dx <= R; ++dx)
-                    if (dx * dx + dy * dy <= R * R)
-                        a += W.w[dy + kMaxR][dx + kMaxR] *
-                             tile[(ly + R + dy) * TW + (tx + R + dx)];
-            const T zT = (T)a;
-            z[i] = zT;
-            acc[0] += a;
-            if constexpr (DOTS) {
-                const T gi = LAZY ? (T)(og[k] - aT) : og[k];
-                const double gd = (double)gi, dg = (double)(T)(gi - op[k]);
-                acc[1] += (double)zT * gd;
-                acc[2] += gd;
-                acc[3] += (double)zT * dg;
-                acc[4] += dg;
-                acc[5] += gd * gd;
-            }
-        }
-        __syncthreads();
-    }
-    int kinds[DOTS ? 6 : 1];
-#pragma unroll
-    for (int i = 0; i < (DOTS ? 6 : 1); ++i) kinds[i] = 0;
-    if (grid_reduce_last<DOTS ? 6 : 1>(acc, kinds, part, &st->counter[2]) && threadIdx.x == 0) {
-        const double zmean = st->nc ? (double)(T)(acc[0] / st->nc) : 0.0;
-        st->zmean = zmean;
-        st->pc++;
+    // one output cell: its tap sum a, raw gap v and raw gap before q
+    auto out = [&](double a, T v, T q) -> T {
+        const T zT = (T)a;
+        acc[0] += a;
         if constexpr (DOTS) {
-            beta_update(P, st, acc[1] - zmean * acc[2], acc[3] - zmean * acc[4], acc[5]);
-            st->beta = (double)((T)st->delta * (T)st->bv);
+            const T gi = LAZY ? (T)(v - aT) : v;
+            const double gd = (double)gi, dg = (double)(T)(gi - (T)(q - aq));
+            acc[1] += (double)zT * gd;
+            acc[2] += gd;
+            acc[3] += (double)zT * dg;
+            acc[4] += dg;
+            acc[5] += gd * gd;
         }
-    }
-}
-
-// Register-blocked form for Ns >= 128 (the tile form above serves smaller
-// grids): a warp owns a 128-wide segment of a 32-row strip, lane l the four
-// consecutive columns x0 = seg*128 + 4l .. x0+3.  It streams the strip's
-// rows top to bottom through a window of 2R+1 rows of centred values in
-// registers (one float4 / double2x2 load of g and one uchar4 of the mask per
-// new row); horizontal neighbours come from the adjacent lanes by shuffles
-// and, at the segment edges, from the strip's halo columns staged in shared
-// memory once per strip.  No block-wide barrier inside the strip.
-constexpr int kSwSeg = 128, kSwRows = 32, kSwWarps = 4;
-
-template <typename T, int R, bool LAZY, bool DOTS>
-__global__ void __launch_bounds__(32 * kSwWarps) k_stencil_w(const PkParams* __restrict__ Pp,
-                                                             PkState* st, StencilW W, const T* g,
-                                                             const T* gprev, const uint8_t* mask,
-                                                             T* z, double* part, int gated,
-                                                             int rows) {
-    Pp += blockIdx.y;
-    st += blockIdx.y;
-    part += (size_t)blockIdx.y * kPartStride;
-    const long bo_ = (long)blockIdx.y * Pp->N;
-    g += bo_;
-    mask += bo_;
-    z += bo_;
-    if (DOTS) gprev += bo_;
-    const PkParams& P = *Pp;
-    if (gated && st->halt) return;
-    constexpr int WR = 2 * R + 1;            // window rows
-    constexpr int HR = kSwRows + 2 * R;      // halo rows of the longest strip
-    __shared__ double halo[kSwWarps][HR][2 * R];
-    const int Ns = P.Ns, msk = Ns - 1;
-    const double gmean = st->nc ? st->gcs / st->nc : 0.0;
-    const T aT = LAZY ? (T)st->alpha : T(0);
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int nseg = Ns / kSwSeg, nstrips = nseg * (Ns / rows);
-    auto centred = [&](uint8_t m, T v) -> double {
-        return m ? (double)(LAZY ? (T)(v - aT) : v) - gmean : 0.0;
+        return zT;
     };
-    auto load4 = [&](const T* base, size_t i, T (&o)[4]) {
-        if constexpr (sizeof(T) == 4) {
-            const float4 q = *reinterpret_cast<const float4*>(base + i);
-            o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w;
-        } else {
-            const double2 q0 = *reinterpret_cast<const double2*>(base + i);
-            const double2 q1 = *reinterpret_cast<const double2*>(base + i + 2);
-            o[0] = q0.x; o[1] = q0.y; o[2] = q1.x; o[3] = q1.y;
-        }
-    };
-    double acc[DOTS ? 6 : 1];
-#pragma unroll
-    for (int i = 0; i < (DOTS ? 6 : 1); ++i) acc[i] = 0.0;
-    for (int sw = blockIdx.x * kSwWarps + wib; sw < nstrips; sw += gridDim.x * kSwWarps) {
-        const int seg = sw % nseg, y0 = (sw / nseg) * rows;
-        const int xs = seg * kSwSeg, x0 = xs + 4 * lane;
-        // the strip's halo columns (R left of the segment, R right), centred
-        for (int e = lane; e < (rows + 2 * R) * 2 * R; e += 32) {
-            const int hr = e / (2 * R), c = e - hr * (2 * R);
-            const int x = (c < R ? xs - R + c : xs + kSwSeg + (c - R)) & msk;
-            const size_t j = (size_t)((y0 - R + hr) & msk) * Ns + x;
-            halo[wib][hr][c] = centred(mask[j], g[j]);
-        }
-        __syncwarp();
-        double win[WR][4];
-        uint32_t wmk[WR];  // the window rows' masks, 4 bytes
-        // raw loads of one row (issued a step ahead of their use, so a row's
-        // load latency hides behind the previous row's arithmetic)
-        auto fetch = [&](int y, T (&v)[4], uint32_t& m4) {
-            const size_t i = (size_t)(y & msk) * Ns + x0;
-            m4 = *reinterpret_cast<const uint32_t*>(mask + i);
-            load4(g, i, v);
+    const long n4 = (FULL ? P.N : P.Nv) / 4;
+    const int lg = 31 - __clz(Ns), lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int tile = 256 * words;
+    for (long base = (long)blockIdx.x * tile; base < n4; base += (long)gridDim.x * tile) {
+        // the tile's words with contact, in order: thread t holds words
+        // base + t * words ...
+        int cnt = 0;
+        uint32_t has = 0;
+        const long w0 = base + (long)threadIdx.x * words;
+        auto scan = [&](int k, uint32_t m) {
+            if (m) {
+                has |= 1u << k;
+                ++cnt;
+            } else if constexpr (!LAZY) {
+                const T zero[4] = {T(0), T(0), T(0), T(0)};
+                st4(z, w0 + k, zero);
+            }
         };
-        auto put = [&](const T (&v)[4], uint32_t m4, double (&w)[4], uint32_t& mk) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = centred((m4 >> (8 * j)) & 0xff, v[j]);
-            mk = m4;
-        };
-#pragma unroll
-        for (int r = 1; r < WR; ++r) {
-            T v[4];
-            uint32_t m4;
-            fetch(y0 - R + r - 1, v, m4);
-            put(v, m4, win[r], wmk[r]);
+        if (words >= 4) {  // n4 is a multiple of 4 (Ns of 16)
+            for (int k = 0; k < words && w0 + k < n4; k += 4) {
+                const uint4 q = *reinterpret_cast<const uint4*>(mask + 4 * (w0 + k));
+                scan(k, q.x);
+                scan(k + 1, q.y);
+                scan(k + 2, q.z);
+                scan(k + 3, q.w);
+            }
+        } else if (w0 < n4) {
+            scan(0, ldm4w(mask, w0));
         }
-        T nv[4], np[4];
-        uint32_t nm;
-        fetch(y0 + R, nv, nm);
-        if constexpr (DOTS) load4(gprev, (size_t)y0 * Ns + x0, np);
-        for (int k = 0; k < rows; ++k) {
+        int at = cnt;  // inclusive prefix over the warp
 #pragma unroll
-            for (int r = 0; r + 1 < WR; ++r) {
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= o) at += up;
+        }
+        if (lane == 31) wtot[wid] = at;
+        __syncthreads();
+        int total = 0, off = 0;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) win[r][j] = win[r + 1][j];
-                wmk[r] = wmk[r + 1];
-            }
-            put(nv, nm, win[WR - 1], wmk[WR - 1]);
-            T gp[4];
+        for (int k = 0; k < 8; ++k) {
+            if (k < wid) off += wtot[k];
+            total += wtot[k];
+        }
+        off += at - cnt;
+        for (; has; has &= has - 1)
+            list[off++] = (uint16_t)(threadIdx.x * words + __ffs(has) - 1);
+        __syncthreads();
+        for (int e = threadIdx.x; e < total; e += 256) {
+            const long i4 = base + list[e];
+            const uint32_t mc = ldm4w(mask, i4);
+            const int y = (int)(i4 >> (lg - 2)), x0 = (int)(4 * i4) & (Ns - 1);
+            T zo[4] = {T(0), T(0), T(0), T(0)};
+            if constexpr (FULL) {
+                const int msk = Ns - 1;
+                double a[4] = {0.0, 0.0, 0.0, 0.0};
+                T own[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) gp[j] = np[j];
-            if (k + 1 < rows) {
-                fetch(y0 + k + 1 + R, nv, nm);
-                if constexpr (DOTS) load4(gprev, (size_t)(y0 + k + 1) * Ns + x0, np);
-            }
-            // value at column offset d (in [-R, 3 + R]) of window row r
-            auto at = [&](int r, int d) -> double {
-                if (d >= 0 && d < 4) return win[r][d];
-                double own, v;
-                if (d < 0) {
-                    own = win[r][4 + d];  // lane-1 holds it at index 4 + d
-                    v = __shfl_up_sync(0xffffffffu, own, 1);
-                    if (lane == 0) v = halo[wib][k + r][R + d];
-                } else {
-                    own = win[r][d - 4];  // lane+1 holds it at index d - 4
-                    v = __shfl_down_sync(0xffffffffu, own, 1);
-                    if (lane == 31) v = halo[wib][k + r][R + (d - 4)];
+                for (int dy = -R; dy <= R; ++dy) {
+                    constexpr int WMAX = 4 + 2 * R;
+                    const int hw = disc_half(R, dy);
+                    const long row = (long)((y + dy) & msk) << (lg - 2);
+                    double v[WMAX];  // columns x0 - R .. x0 + 3 + R
+                    T c4[4];
+                    const uint32_t m1 = ldm4w(mask, row + (x0 >> 2));
+                    ldp4(g, row + (x0 >> 2), c4);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) v[R + j] = centred(mbyte(m1, j), c4[j]);
+                    if (dy == 0) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) own[j] = c4[j];
+                    }
+                    if (hw > 0) {
+                        const long il = row + (((x0 - 4) & msk) >> 2);
+                        const long ir = row + (((x0 + 4) & msk) >> 2);
+                        const uint32_t ml = ldm4w(mask, il), mr = ldm4w(mask, ir);
+                        T l4[4], r4[4];
+                        ldp4(g, il, l4);
+                        ldp4(g, ir, r4);
+#pragma unroll
+                        for (int j = 0; j < R; ++j) {
+                            if (j < hw) {
+                                v[R - 1 - j] = centred(mbyte(ml, 3 - j), l4[3 - j]);
+                                v[R + 4 + j] = centred(mbyte(mr, j), r4[j]);
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int dx = -R; dx <= R; ++dx) {
+                        if (dx * dx + dy * dy > R * R) continue;
+                        const double w = W.w[dy + kMaxR][dx + kMaxR];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) a[j] += w * v[R + j + dx];
+                    }
                 }
-                return v;
-            };
-            const int y = y0 + k;
-            const size_t i = (size_t)y * Ns + x0;
-            double a[4] = {0.0, 0.0, 0.0, 0.0};
+                T q[4] = {T(0), T(0), T(0), T(0)};
+                if constexpr (DOTS) ldp4(gq, i4, q);
 #pragma unroll
-            for (int dy = -R; dy <= R; ++dy) {
-#pragma unroll
-                for (int dx = -R; dx <= R; ++dx) {
-                    if (dx * dx + dy * dy > R * R) continue;
-                    const double w = W.w[dy + kMaxR][dx + kMaxR];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) a[j] += w * at(R + dy, j + dx);
-                }
-            }
-            const uint32_t mc = wmk[R];
-            T zo[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const bool on = (mc >> (8 * j)) & 0xff;
-                zo[j] = on ? (T)a[j] : T(0);
-                if (on) acc[0] += a[j];
-            }
-            if constexpr (sizeof(T) == 4) {
-                *reinterpret_cast<float4*>(z + i) = make_float4(zo[0], zo[1], zo[2], zo[3]);
+                for (int j = 0; j < 4; ++j)
+                    if (mbyte(mc, j)) zo[j] = out(a[j], own[j], q[j]);
             } else {
-                *reinterpret_cast<double2*>(z + i) = make_double2(zo[0], zo[1]);
-                *reinterpret_cast<double2*>(z + i + 2) = make_double2(zo[2], zo[3]);
-            }
-            if constexpr (DOTS) {
-                T gv[4];
-                load4(g, i, gv);  // loaded R rows ago: a cache hit
-#pragma unroll
+                // Nw: the periodic grid of the wrap; 2R + 1 <= Nw
+                auto wrap = [Nw](int v) { return v < 0 ? v + Nw : (v >= Nw ? v - Nw : v); };
+#pragma unroll 1
                 for (int j = 0; j < 4; ++j) {
-                    if (!((mc >> (8 * j)) & 0xff)) continue;
-                    const T gi = LAZY ? (T)(gv[j] - aT) : gv[j];
-                    const double gd = (double)gi, dg = (double)(T)(gi - gp[j]);
-                    acc[1] += (double)zo[j] * gd;
-                    acc[2] += gd;
-                    acc[3] += (double)zo[j] * dg;
-                    acc[4] += dg;
-                    acc[5] += gd * gd;
+                    if (!mbyte(mc, j)) continue;
+                    const int x = x0 + j;
+                    double a = 0.0;
+#pragma unroll
+                    for (int dy = -R; dy <= R; ++dy) {
+                        const size_t row = (size_t)wrap(y + dy) * Ns;
+#pragma unroll
+                        for (int dx = -R; dx <= R; ++dx) {
+                            if (dx * dx + dy * dy > R * R) continue;
+                            const size_t i = row + wrap(x + dx);
+                            a += W.w[dy + kMaxR][dx + kMaxR] * centred(mask[i], g[i]);
+                        }
+                    }
+                    const size_t i = (size_t)y * Ns + x;
+                    const T zT = out(a, g[i], DOTS ? gq[i] : T(0));
+                    zo[0] = j == 0 ? zT : zo[0];
+                    zo[1] = j == 1 ? zT : zo[1];
+                    zo[2] = j == 2 ? zT : zo[2];
+                    zo[3] = j == 3 ? zT : zo[3];
                 }
             }
+            st4(z, i4, zo);
         }
-        __syncwarp();  // the halo buffer is refilled by the next strip
+        __syncthreads();  // the next tile's list
     }
     int kinds[DOTS ? 6 : 1];
 #pragma unroll
@@ -621,18 +589,6 @@ __global__ void __launch_bounds__(32 * kSwWarps) k_stencil_w(const PkParams* __r
             st->beta = (double)((T)st->delta * (T)st->bv);
         }
     }
-}
-
-inline int num_sms() {
-    int dev = 0, n = 0;
-    ASB_CUDA(cudaGetDevice(&dev));
-    ASB_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
-    return n > 0 ? n : 1;
-}
-
-inline int stencil_grid(int Ns) {
-    const int n = ((Ns + kStX - 1) / kStX) * ((Ns + kStY - 1) / kStY);
-    return n < kMaxRowBlocks ? n : kMaxRowBlocks;
 }
 
 StencilW stencil_weights(const StencilTaps& taps) {
@@ -642,39 +598,38 @@ StencilW stencil_weights(const StencilTaps& taps) {
     return W;
 }
 
-// launch of the stencil pass for the runtime radius R in [1, kMaxR]: the
-// register-window kernel for Ns >= 128, the tile kernel below that and for
-// embedded grids (Nl < Ns: the wrap is at the caller's side Nl)
+inline int num_sms() {
+    int dev = 0, n = 0;
+    ASB_CUDA(cudaGetDevice(&dev));
+    ASB_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+    return n > 0 ? n : 1;
+}
+
+// launch of the stencil pass for the runtime radius R in [1, kMaxR] on B
+// instances (the full form on grids that are not embedded)
 template <typename T, bool LAZY, bool DOTS>
-void launch_stencil(int R, int Ns, int Nl, dim3 grid, cudaStream_t s, const PkParams* Pp,
-                    PkState* st, const StencilW& W, const T* g, const T* gprev,
-                    const uint8_t* mask, T* z, double* part, int gated) {
-    if (Ns >= kSwSeg && Nl == Ns) {
-        // strips of 32, 16 or 8 rows: the longest that still gives every SM
-        // 12 or more warps (a shorter strip re-reads more halo rows; at
-        // Ns=2048 16-row strips measured 1 % faster per solve than 8 or 32)
-        int rows = kSwRows;
-        const long want = 12L * num_sms();
-        while (rows > 8 && (long)(Ns / kSwSeg) * (Ns / rows) * grid.y < want) rows /= 2;
-        const int strips = (Ns / kSwSeg) * (Ns / rows);
-        int nb = (strips + kSwWarps - 1) / kSwWarps;
-        if (nb > kMaxRowBlocks) nb = kMaxRowBlocks;
-        const dim3 gw(nb, grid.y);
-        switch (R) {
-            case 1: k_stencil_w<T, 1, LAZY, DOTS><<<gw, 32 * kSwWarps, 0, s>>>(Pp, st, W, g, gprev, mask, z, part, gated, rows); break;
-            case 2: k_stencil_w<T, 2, LAZY, DOTS><<<gw, 32 * kSwWarps, 0, s>>>(Pp, st, W, g, gprev, mask, z, part, gated, rows); break;
-            case 3: k_stencil_w<T, 3, LAZY, DOTS><<<gw, 32 * kSwWarps, 0, s>>>(Pp, st, W, g, gprev, mask, z, part, gated, rows); break;
-            case 4: k_stencil_w<T, 4, LAZY, DOTS><<<gw, 32 * kSwWarps, 0, s>>>(Pp, st, W, g, gprev, mask, z, part, gated, rows); break;
-            default: throw Error(ASPHER_EINVAL, "stencil radius must be in [1, 4]");
-        }
-        count_launches(1);
-        return;
-    }
+void launch_stencil(int R, int Ns, int Nl, int B, cudaStream_t s, const PkParams* Pp, PkState* st,
+                    const StencilW& W, const T* ga, const T* gb, const uint8_t* mask, T* z,
+                    double* part, int gated) {
+    const bool full = Nl == Ns;
+    // the largest tile that still leaves a CTA for every other SM (of the
+    // rows that hold data)
+    const long n4 = (long)Nl * Ns / 4;
+    int words = kStMaxWords;
+    while (words > 1 && n4 * B < 256L * words * (num_sms() / 2)) words /= 4;
+    long nb = (n4 + 256L * words - 1) / (256L * words);
+    if (nb > kMaxBlocks / 2) nb = kMaxBlocks / 2;
+    auto go = [&](auto r) {
+        constexpr int RR = decltype(r)::value;
+        launch_pdl(full ? k_stencil<T, RR, LAZY, DOTS, true> : k_stencil<T, RR, LAZY, DOTS, false>,
+                   dim3((unsigned)nb, B), 256, 0, s, Pp, st, W, ga, gb, mask, z, part, gated,
+                   words);
+    };
     switch (R) {
-        case 1: k_stencil_t<T, 1, LAZY, DOTS><<<grid, 256, 0, s>>>(Pp, st, W, g, gprev, mask, z, part, gated); break;
-        case 2: k_stencil_t<T, 2, LAZY, DOTS><<<grid, 256, 0, s>>>(Pp, st, W, g, gprev, mask, z, part, gated); break;
-        case 3: k_stencil_t<T, 3, LAZY, DOTS><<<grid, 256, 0, s>>>(Pp, st, W, g, gprev, mask, z, part, gated); break;
-        case 4: k_stencil_t<T, 4, LAZY, DOTS><<<grid, 256, 0, s>>>(Pp, st, W, g, gprev, mask, z, part, gated); break;
+        case 1: go(std::integral_constant<int, 1>{}); break;
+        case 2: go(std::integral_constant<int, 2>{}); break;
+        case 3: go(std::integral_constant<int, 3>{}); break;
+        case 4: go(std::integral_constant<int, 4>{}); break;
         default: throw Error(ASPHER_EINVAL, "stencil radius must be in [1, 4]");
     }
     count_launches(1);
@@ -690,39 +645,39 @@ __device__ __forceinline__ T zfinal(const PkParams& P, T z, T g, T zm) {
 // preconditioner; g centred on the fly)
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_dots(const PkParams* __restrict__ Pp, PkState* st, const T* z,
-                                                      const T* g, const T* gprev,
+                                                      const T* ga, const T* gb,
                                                       const uint8_t* mask, double* part) {
+    pdl_wait();
     // instance blockIdx.y of a batched solve (0 when unbatched)
     Pp += blockIdx.y;
     st += blockIdx.y;
     part += (size_t)blockIdx.y * kPartStride;
     const long bo_ = (long)blockIdx.y * Pp->N;
     z += bo_;
-    g += bo_;
-    gprev += bo_;
     mask += bo_;
     const PkParams& P = *Pp;
     if (st->halt) return;
-    const T zm = (T)st->zmean, aT = (T)st->alpha;
+    const T* g = gap_now(st, ga, gb) + bo_;
+    const T* gq = gap_before(st, ga, gb) + bo_;
+    const T zm = (T)st->zmean, aT = (T)st->alpha, aq = (T)st->alpha_prev;
+    const bool pre = P.precond != 0;
     double acc[3] = {0, 0, 0};  // G, G_pr, gg
-    GRID_LOOP4(P.Nv) {
+    contact_groups(mask, P.Nv / 4, [&](long i4, uint32_t mw) {
         T zz[4], gv[4], gp[4];
-        uint8_t mm[4];
-        ldm4(mask, i4, mm);
         ldp4(g, i4, gv);
-        ldp4(gprev, i4, gp);
-        if (P.precond) ldp4(z, i4, zz);
+        ldp4(gq, i4, gp);
+        if (pre) ldp4(z, i4, zz);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            if (!mm[j]) continue;
+            if (!mbyte(mw, j)) continue;
             const T gi = gc(gv[j], aT);
             const T zf = zfinal(P, zz[j], gi, zm);
             const double gd = (double)gi;
             acc[0] += (double)zf * gd;
-            acc[1] += (double)zf * (double)(T)(gi - gp[j]);
+            acc[1] += (double)zf * (double)(T)(gi - gc(gp[j], aq));
             acc[2] += gd * gd;
         }
-    }
+    });
     const int kinds[3] = {0, 0, 0};
     if (grid_reduce_last<3>(acc, kinds, part, &st->counter[3]) && threadIdx.x == 0) {
         beta_update(P, st, acc[0], acc[1], acc[2]);
@@ -730,47 +685,49 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_dots(const PkPar
     }
 }
 
-// Direction update t = chi_C(z_f + beta t), g_prev = g (and best = p when
-// copy_best) before the t apply; k_rden consumes r after it.
+// Direction update t = chi_C(z_f + beta t) (and best = p when copy_best)
+// before the t apply; k_rden consumes r after it.  t is 0 off contact (k_pupd
+// clears the cells that leave it), so only groups with contact are touched.
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_tupd(const PkParams* __restrict__ Pp, PkState* st, const T* z,
-                                                      const T* g, T* gprev, T* t,
+                                                      const T* ga, const T* gb, T* t,
                                                       const uint8_t* mask, const T* p, T* best) {
+    pdl_wait();
     // instance blockIdx.y of a batched solve (0 when unbatched)
     Pp += blockIdx.y;
     st += blockIdx.y;
     const long bo_ = (long)blockIdx.y * Pp->N;
     z += bo_;
-    g += bo_;
-    gprev += bo_;
     t += bo_;
     mask += bo_;
     p += bo_;
     best += bo_;
     const PkParams& P = *Pp;
     if (st->halt) return;
+    const T* g = gap_now(st, ga, gb) + bo_;
     const T zm = (T)st->zmean, beta = (T)st->beta, aT = (T)st->alpha;
-    const int cb = st->copy_best;
-    const PScale<T> ps(st);
-    GRID_LOOP4(P.Nv) {
+    const bool pre = P.precond != 0;
+    contact_groups(mask, P.Nv / 4, [&](long i4, uint32_t mw) {
         T zz[4], gv[4], tt[4];
-        uint8_t mm[4];
-        ldm4(mask, i4, mm);
-        ldp4(g, i4, gv);
         ldp4(t, i4, tt);
-        if (P.precond) ldp4(z, i4, zz);
+        if (pre) ldp4(z, i4, zz);
+        else ldp4(g, i4, gv);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            gv[j] = gc(gv[j], aT);
-            tt[j] = mm[j] ? (T)(zfinal(P, zz[j], gv[j], zm) + beta * tt[j]) : T(0);
+            const T zf = pre ? (T)(zz[j] - zm) : gc(gv[j], aT);
+            tt[j] = mbyte(mw, j) ? (T)(zf + beta * tt[j]) : T(0);
         }
         st4(t, i4, tt);
-        st4(gprev, i4, gv);
-        if (cb) {
-            T pp[4];
-            ldp4(p, i4, pp);
+    });
+    if (st->copy_best) {
+        const PScale<T> ps(st);
+        GRID_LOOP4(P.Nv) {
+            T pp[4] = {T(0), T(0), T(0), T(0)};
+            if (ldm4w(mask, i4)) {
+                ldp4(p, i4, pp);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) pp[j] = ps(pp[j]);
+                for (int j = 0; j < 4; ++j) pp[j] = ps(pp[j]);
+            }
             st4(best, i4, pp);
         }
     }
@@ -778,46 +735,55 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_tupd(const PkPar
 
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_rden(const PkParams* __restrict__ Pp, PkState* st, const T* r,
-                                                      const T* g, const T* t,
+                                                      const T* ga, const T* gb, const T* t,
                                                       const uint8_t* mask, double* part) {
+    pdl_wait();
     // instance blockIdx.y of a batched solve (0 when unbatched)
     Pp += blockIdx.y;
     st += blockIdx.y;
     part += (size_t)blockIdx.y * kPartStride;
     const long bo_ = (long)blockIdx.y * Pp->N;
     r += bo_;
-    g += bo_;
     t += bo_;
     mask += bo_;
     const PkParams& P = *Pp;
     if (st->halt) return;
+    const T* g = gap_now(st, ga, gb) + bo_;
     const T aT = (T)st->alpha;
     double acc[4] = {0, 0, 0, 0};  // sum_C r, sum_C g t, sum_C r t, sum_C t
-    GRID_LOOP4(P.Nv) {
+    contact_groups(mask, P.Nv / 4, [&](long i4, uint32_t mw) {
         T rr[4], gv[4], tt[4];
-        uint8_t mm[4];
-        ldm4(mask, i4, mm);
         ldp4(r, i4, rr);
         ldp4(g, i4, gv);
         ldp4(t, i4, tt);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            if (!mm[j]) continue;
+            if (!mbyte(mw, j)) continue;
             const double td = (double)tt[j];
             acc[0] += (double)rr[j];
             acc[1] += (double)gc(gv[j], aT) * td;
             acc[2] += (double)rr[j] * td;
             acc[3] += td;
         }
-    }
+    });
     const int kinds[4] = {0, 0, 0, 0};
     if (grid_reduce_last<4>(acc, kinds, part, &st->counter[4]) && threadIdx.x == 0)
         rden_tail<T>(st, acc);
 }
 
+// Projected update of the pressure (contact_solver.cpp:464-501).  Off contact
+// p is 0 and changes only where the gap is negative, so a group without
+// either reads its mask word and its gap.  Keeps the mask (cells whose p is
+// not 0) and clears t where a cell leaves contact.  The last kernel of an
+// iteration: in a loop graph it ends the loop (cond, of n instances) when
+// either end instance has halted; the host continues with the smallest range
+// that covers the instances still running.
 template <typename T>
-__global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_pupd(const PkParams* __restrict__ Pp, PkState* st, T* p, const T* t,
-                                                      const T* g, double* part) {
+__global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_pupd(const PkParams* __restrict__ Pp, PkState* st, T* p, T* t,
+                                                      const T* ga, const T* gb, uint8_t* mask,
+                                                      double* part, int loop,
+                                                      cudaGraphConditionalHandle cond, int n) {
+    pdl_wait();
     // instance blockIdx.y of a batched solve (0 when unbatched)
     Pp += blockIdx.y;
     st += blockIdx.y;
@@ -825,34 +791,58 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_pupd(const PkPar
     const long bo_ = (long)blockIdx.y * Pp->N;
     p += bo_;
     t += bo_;
-    g += bo_;
+    mask += bo_;
     const PkParams& P = *Pp;
-    if (st->halt) return;
+    const bool end = loop && ((int)blockIdx.y == 0 || (int)blockIdx.y == n - 1);
+    if (st->halt) {
+        if (end && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(cond, 0u);
+        return;
+    }
+    const T* g = gap_now(st, ga, gb) + bo_;
     const T tau = (T)st->tau, tov = (T)st->tau_ov, aT = (T)st->alpha;
     // every block reads the pending rescale here, before it arrives at the
     // last-block counter; only the last block's tail rewrites it
     const PScale<T> ps(st);
     double acc[2] = {0, 0};  // changed (max), total
     GRID_LOOP4(P.Nv) {
-        T pp[4], tt[4], gv[4];
-        ldp4(p, i4, pp);
-        ldp4(t, i4, tt);
+        T pp[4] = {T(0), T(0), T(0), T(0)}, tt[4] = {T(0), T(0), T(0), T(0)}, gv[4];
+        const uint32_t mw = ldm4w(mask, i4);
         ldp4(g, i4, gv);
+        bool neg = false;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            gv[j] = gc(gv[j], aT);
+            neg = neg || gv[j] < T(0);
+        }
+        if (!mw && !neg) continue;
+        if (mw) {
+            ldp4(p, i4, pp);
+            ldp4(t, i4, tt);
+        }
+        uint32_t mn = 0;
+        bool left = false;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             T pi = ps(pp[j]);
-            const T gi = gc(gv[j], aT);
             const bool was = pi > T(0);
             if (was) {
                 const T q = pi - tau * tt[j];
                 pi = q < T(0) ? T(0) : q;
             }
-            if (pi == T(0) && gi < T(0)) pi -= tov * gi;
+            if (pi == T(0) && gv[j] < T(0)) pi -= tov * gv[j];
             if ((pi > T(0)) != was) acc[0] = 1.0;
             pp[j] = pi;
             acc[1] += (double)pi;
+            if (pi != T(0)) {
+                mn |= 1u << (8 * j);
+            } else if (tt[j] != T(0)) {
+                tt[j] = T(0);
+                left = true;
+            }
         }
         st4(p, i4, pp);
+        if (left) st4(t, i4, tt);
+        if (mn != mw) reinterpret_cast<uint32_t*>(mask)[i4] = mn;
     }
     const int kinds[2] = {2, 0};
     if (grid_reduce_last<2>(acc, kinds, part, &st->counter[6]) && threadIdx.x == 0) {
@@ -873,9 +863,11 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_pupd(const PkPar
             st->scale = 1.0;
             st->scale_add = (double)(T)P.p_bar;
             st->fill = 1;
+            st->mask_stale = 1;
         }
         st->it++;
         if (st->it >= P.max_iter) set_halt(st, H_FINAL);  // status stays max_iterations
+        if (end && st->halt) cudaGraphSetConditional(cond, 0u);
     }
 }
 
@@ -1091,17 +1083,6 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_gmean(long N, Pk
     }
 }
 
-// ---- device-side loop control -------------------------------------------------------
-// Last kernel of the graph body of instances [0, n) (a range of the batch):
-// keep looping while both end instances are running.  When an end instance
-// halts the host continues with the loop graph of the smaller range that
-// covers the instances still running, so halted instances at the ends stop
-// costing gated blocks.
-__global__ void k_loop_cond(cudaGraphConditionalHandle h, const PkState* st, int n) {
-    if (threadIdx.x == 0)
-        cudaGraphSetConditional(h, (st[0].halt == H_RUN && st[n - 1].halt == H_RUN) ? 1u : 0u);
-}
-
 // ---- host driver -----------------------------------------------------------------
 namespace {
 
@@ -1127,7 +1108,7 @@ struct SolverCtx : SolverCtxBase {
     int cap = 1;
     long N = 0;
     long Nv = 0;  // the prefix of a field that the vector passes visit (PkParams::Nv)
-    T *p = nullptr, *t = nullptr, *u = nullptr, *g = nullptr, *gprev = nullptr, *z = nullptr,
+    T *p = nullptr, *t = nullptr, *u = nullptr, *g = nullptr, *g2 = nullptr, *z = nullptr,
       *r = nullptr, *best = nullptr;
     T* g0c = nullptr;  // the solves' gaps, copied in so the loop graph is reusable
     uint8_t* mask = nullptr;
@@ -1170,7 +1151,7 @@ struct SolverCtx : SolverCtxBase {
         N = (long)o.Ns * o.Ns;
         Nv = o.embedded() ? (long)o.Nl * o.Ns : N;  // Ns is a multiple of 16
         const size_t b = (size_t)cap * N * sizeof(T);
-        T** vecs[] = {&p, &t, &u, &g, &gprev, &z, &r, &best, &g0c};
+        T** vecs[] = {&p, &t, &u, &g, &g2, &z, &r, &best, &g0c};
         for (T** v : vecs) ASB_CUDA(cudaMalloc((void**)v, b));
         ASB_CUDA(cudaMalloc((void**)&mask, (size_t)cap * N));
         if (Nv != N) {  // the rows past Nv are never written: 0, and no contact
@@ -1198,7 +1179,7 @@ struct SolverCtx : SolverCtxBase {
     ~SolverCtx() override {
         std::lock_guard<std::recursive_mutex> setup(setup_mutex());
         drop_graph();
-        void* all[] = {p, t, u, g, gprev, z, r, best, g0c, mask, part, hist, st, Pd, spec, p0, u0};
+        void* all[] = {p, t, u, g, g2, z, r, best, g0c, mask, part, hist, st, Pd, spec, p0, u0};
         for (void* v : all)
             if (v) cudaFree(v);
         if (ev_in) cudaEventDestroy(ev_in);
@@ -1230,17 +1211,17 @@ struct SolverCtx : SolverCtxBase {
     // captures the iteration of instances [b0, b0 + n) with gridDim.y = n.
     struct InstanceView {
         SolverCtx& c;
-        T *p, *t, *u, *g, *gprev, *z, *r, *best, *g0c;
+        T *p, *t, *u, *g, *g2, *z, *r, *best, *g0c;
         uint8_t* mask;
         double *part, *p0, *u0;
         PkState* st;
         PkParams* Pd;
         InstanceView(SolverCtx& cx, int b0)
-            : c(cx), p(cx.p), t(cx.t), u(cx.u), g(cx.g), gprev(cx.gprev), z(cx.z), r(cx.r),
+            : c(cx), p(cx.p), t(cx.t), u(cx.u), g(cx.g), g2(cx.g2), z(cx.z), r(cx.r),
               best(cx.best), g0c(cx.g0c), mask(cx.mask), part(cx.part), p0(cx.p0), u0(cx.u0),
               st(cx.st), Pd(cx.Pd) {
             const size_t o = (size_t)b0 * cx.N;
-            T** vs[] = {&cx.p, &cx.t, &cx.u, &cx.g, &cx.gprev, &cx.z, &cx.r, &cx.best, &cx.g0c};
+            T** vs[] = {&cx.p, &cx.t, &cx.u, &cx.g, &cx.g2, &cx.z, &cx.r, &cx.best, &cx.g0c};
             for (T** v : vs) *v += o;
             cx.mask += o;
             cx.part += (size_t)b0 * kPartStride;
@@ -1250,7 +1231,7 @@ struct SolverCtx : SolverCtxBase {
             cx.Pd += b0;
         }
         ~InstanceView() {
-            c.p = p; c.t = t; c.u = u; c.g = g; c.gprev = gprev; c.z = z; c.r = r;
+            c.p = p; c.t = t; c.u = u; c.g = g; c.g2 = g2; c.z = z; c.r = r;
             c.best = best; c.g0c = g0c; c.mask = mask; c.part = part; c.p0 = p0; c.u0 = u0;
             c.st = st; c.Pd = Pd;
         }
@@ -1325,41 +1306,44 @@ struct SolverCtx : SolverCtxBase {
         }
         apply(t, r, &st->halt, s, B);
     }
-    void enqueue_iteration(cudaStream_t s, int B) {
+    // loop: the last kernel ends the loop graph of these B instances (cond)
+    void enqueue_iteration(cudaStream_t s, int B, int loop = 0,
+                           cudaGraphConditionalHandle cond = 0) {
         const dim3 gr(grid, B);
         int n = 0;
         apply_u(s, B);
-        k_eval<T><<<gr, kRedThreads, 0, s>>>(Pd, st, u, g0c, p, g, mask, part, 0);
+        launch_pdl(k_eval<T>, gr, kRedThreads, 0, s, Pd, st, u, g0c, p, g, g2, mask, part, 0);
         ++n;
         if (with_hist) {
-            k_evalpk<T><<<gr, kRedThreads, 0, s>>>(Pd, st, p, g, part, hist, 0);
+            launch_pdl(k_evalpk<T>, gr, kRedThreads, 0, s, Pd, st, p, g, g2, part, hist, 0);
             ++n;
         }
         if (precond == 1) {
-            launch_stencil<T, true, true>(radius, op.Ns, op.Nl, dim3(stencil_grid(op.Nl), B), s, Pd, st, W, g,
-                                          gprev, mask, z, part, 1);
+            launch_stencil<T, true, true>(radius, op.Ns, op.Nl, B, s, Pd, st, W, g, g2, mask, z,
+                                          part, 1);
             ++n;
         } else {
             if (precond == 2)
-                fourier_precond_pk<T>(op, g, mask, st, z, part, s, &st->halt, B,
+                fourier_precond_pk<T>(op, g, g2, mask, st, z, part, s, &st->halt, B,
                                       B > 1 ? spec : nullptr);
-            k_dots<T><<<gr, kRedThreads, 0, s>>>(Pd, st, z, g, gprev, mask, part);
+            launch_pdl(k_dots<T>, gr, kRedThreads, 0, s, Pd, st, z, g, g2, mask, part);
             ++n;
         }
-        k_tupd<T><<<gr, kRedThreads, 0, s>>>(Pd, st, z, g, gprev, t, mask, p, best);
+        launch_pdl(k_tupd<T>, gr, kRedThreads, 0, s, Pd, st, z, g, g2, t, mask, p, best);
         apply_r(s, B);
-        k_rden<T><<<gr, kRedThreads, 0, s>>>(Pd, st, r, g, t, mask, part);
+        launch_pdl(k_rden<T>, gr, kRedThreads, 0, s, Pd, st, r, g, g2, t, mask, part);
         n += 2;
-        k_pupd<T><<<gr, kRedThreads, 0, s>>>(Pd, st, p, t, g, part);
+        launch_pdl(k_pupd<T>, gr, kRedThreads, 0, s, Pd, st, p, t, g, g2, mask, part, loop, cond,
+                   B);
         count_launches(n + 1);
         ASB_CUDA(cudaGetLastError());
     }
     // g <- centred gap for instance b (or all B when b < 0)
     void center(cudaStream_t s, int B, int b = -1) {
         if (b < 0)
-            k_center<T><<<dim3(grid, B), kRedThreads, 0, s>>>(Pd, st, g);
+            k_center<T><<<dim3(grid, B), kRedThreads, 0, s>>>(Pd, st, g, g2);
         else
-            k_center<T><<<grid, kRedThreads, 0, s>>>(Pd + b, st + b, at(g, b));
+            k_center<T><<<grid, kRedThreads, 0, s>>>(Pd + b, st + b, at(g, b), at(g2, b));
         count_launches(1);
         ASB_CUDA(cudaGetLastError());
     }
@@ -1385,8 +1369,7 @@ struct SolverCtx : SolverCtxBase {
                                                cudaStreamCaptureModeRelaxed));
         try {
             InstanceView view(*this, lo);
-            enqueue_iteration(s, n);
-            k_loop_cond<<<1, 32, 0, s>>>(h, st, n);
+            enqueue_iteration(s, n, 1, h);
         } catch (...) {
             // leave no capture open on the stream, then report the failure
             cudaGraph_t partial = nullptr;
@@ -1510,6 +1493,9 @@ struct Solver {
         return r[0];
     }
 
+    // the buffer of instance b's last evaluated gap (h[b] read back)
+    T* gap_field(int b) { return c.at(h[b].par ? c.g2 : c.g, b); }
+
     // project_load_simplex on instance b's z (contact_solver.cpp:31-60)
     void project_simplex(int b, double P_total) {
         const long N = c.Nv;  // z is 0 past it
@@ -1537,8 +1523,8 @@ struct Solver {
     bool identification_step(int b) {
         InstHost& I = ih[b];
         PkState& H = h[b];
-        T *p = c.at(c.p, b), *u = c.at(c.u, b), *g = c.at(c.g, b), *z = c.at(c.z, b),
-          *r = c.at(c.r, b), *t = c.at(c.t, b), *gp = c.at(c.gprev, b);
+        T *p = c.at(c.p, b), *u = c.at(c.u, b), *g = gap_field(b), *z = c.at(c.z, b),
+          *r = c.at(c.r, b), *t = c.at(c.t, b);
         const T* g0 = c.at(c.g0c, b);
         double o[3];
         reduce(b, 2, p, u, g0, nullptr, 0.0, o);
@@ -1566,7 +1552,10 @@ struct Solver {
                 ASB_CUDA(cudaMemcpyAsync(p, z, bytes, cudaMemcpyDeviceToDevice, s));
                 ASB_CUDA(cudaMemcpyAsync(u, r, bytes, cudaMemcpyDeviceToDevice, s));
                 ASB_CUDA(cudaMemsetAsync(t, 0, bytes, s));
-                ASB_CUDA(cudaMemsetAsync(gp, 0, bytes, s));
+                // g_prev = 0: the next evaluation writes the other buffer
+                ASB_CUDA(cudaMemsetAsync(g, 0, bytes, s));
+                H.alpha = 0.0;
+                H.mask_stale = 1;
                 H.u_fresh = 1;
                 H.delta = 0.0;
                 H.G_old = 1.0;
@@ -1691,12 +1680,13 @@ struct Solver {
         }
         const size_t vb = (size_t)B * N * sizeof(T);
         ASB_CUDA(cudaMemsetAsync(c.t, 0, vb, s));
-        ASB_CUDA(cudaMemsetAsync(c.gprev, 0, vb, s));
+        ASB_CUDA(cudaMemsetAsync(c.g, 0, vb, s));  // g_prev of the first iteration
         ASB_CUDA(cudaMemsetAsync(c.z, 0, vb, s));
         for (int b = 0; b < B; ++b) {
             PkState& H = h[b];
             std::memset(&H, 0, sizeof(H));
             H.scale = 1.0;  // no load rescale pending
+            H.mask_stale = 1;
             H.G_old = 1.0;
             H.delta = 0.0;
             H.best_merit = std::numeric_limits<double>::infinity();
@@ -1776,6 +1766,7 @@ struct Solver {
                     // moved on
                     fill_p(c.at(c.p, b), (T)I.p_bar);
                     H.fill = 0;
+                    H.mask_stale = 1;
                     H.u_fresh = 0;
                     if (H.halt == H_FILL) {
                         H.halt = H_RUN;
@@ -1837,6 +1828,7 @@ struct Solver {
                     ASB_CUDA(cudaMemcpyAsync(c.at(c.p, b), c.at(c.best, b), (size_t)N * sizeof(T),
                                              cudaMemcpyDeviceToDevice, s));
                     H.u_fresh = 0;
+                    H.mask_stale = 1;
                     I.returned_best = true;
                 }
             }
@@ -1849,10 +1841,11 @@ struct Solver {
         }
         write_states();
         c.apply(c.p, c.u, &c.st->skip_mv1, s, B);
-        k_eval<T><<<dim3(c.grid, B), kRedThreads, 0, s>>>(c.Pd, c.st, c.u, c.g0c, c.p, c.g, c.mask,
-                                                        c.part, 1);
-        k_evalpk<T><<<dim3(c.grid, B), kRedThreads, 0, s>>>(c.Pd, c.st, c.p, c.g, c.part, nullptr,
-                                                          1);
+        const dim3 gr(c.grid, B);
+        launch_pdl(k_eval<T>, gr, kRedThreads, 0, s, c.Pd, c.st, c.u, c.g0c, c.p, c.g, c.g2, c.mask,
+                   c.part, 1);
+        launch_pdl(k_evalpk<T>, gr, kRedThreads, 0, s, c.Pd, c.st, c.p, c.g, c.g2, c.part, nullptr,
+                   1);
         count_launches(2);
         ASB_CUDA(cudaGetLastError());
         read_states();
@@ -1870,7 +1863,7 @@ struct Solver {
             if (disp) { k_to_f64<T><<<c.grid, kRedThreads, 0, s>>>(N, disp, c.u); count_launches(1); }
             if (gap) {
                 c.center(s, 1);
-                k_to_f64<T><<<c.grid, kRedThreads, 0, s>>>(N, gap, c.g);
+                k_to_f64<T><<<c.grid, kRedThreads, 0, s>>>(N, gap, gap_field(0));
                 count_launches(1);
             }
         }
@@ -2311,6 +2304,20 @@ void precond_apply_impl(Operator& op, int precond, int radius, const T* g_in,
     const uint8_t* mask = mask_in;
     T* z = z_out;
     void* tmp[3] = {nullptr, nullptr, nullptr};
+    // a full grid's stencil pass moves 16 bytes at a time: fields at other
+    // addresses through aligned copies
+    const bool moved = !op.embedded() &&
+                       (((uintptr_t)g_in | (uintptr_t)mask_in | (uintptr_t)z_out) % 16) != 0;
+    if (moved) {
+        ASB_CUDA(scratch_alloc((void**)&tmp[0], (size_t)N * sizeof(T), s));
+        ASB_CUDA(scratch_alloc((void**)&tmp[1], (size_t)N, s));
+        ASB_CUDA(scratch_alloc((void**)&tmp[2], (size_t)N * sizeof(T), s));
+        ASB_CUDA(cudaMemcpyAsync(tmp[0], g_in, (size_t)N * sizeof(T), cudaMemcpyDeviceToDevice, s));
+        ASB_CUDA(cudaMemcpyAsync(tmp[1], mask_in, (size_t)N, cudaMemcpyDeviceToDevice, s));
+        g = (const T*)tmp[0];
+        mask = (const uint8_t*)tmp[1];
+        z = (T*)tmp[2];
+    }
     if (op.embedded()) {
         ASB_CUDA(scratch_alloc((void**)&tmp[0], (size_t)N * sizeof(T), s));
         ASB_CUDA(scratch_alloc((void**)&tmp[1], (size_t)N, s));
@@ -2341,18 +2348,21 @@ void precond_apply_impl(Operator& op, int precond, int radius, const T* g_in,
     k_gmean<T><<<grid, kRedThreads, 0, s>>>(N, st, g, mask, part);
     if (precond == 1) {
         StencilTaps taps = make_stencil_taps(op.Nl, radius);
-        launch_stencil<T, false, false>(radius, op.Ns, op.Nl, dim3(stencil_grid(op.Nl)), s, Pd,
-                                        st, stencil_weights(taps), g, nullptr, mask, z, part, 0);
+        launch_stencil<T, false, false>(radius, op.Ns, op.Nl, 1, s, Pd, st, stencil_weights(taps),
+                                        g, nullptr, mask, z, part, 0);
     } else {
-        fourier_precond_pk<T>(op, g, mask, st, z, part, s, nullptr);
+        fourier_precond_pk<T>(op, g, g, mask, st, z, part, s, nullptr);
     }
     k_sub_zmean<T><<<grid, kRedThreads, 0, s>>>(N, z, mask, st);
     count_launches(2);
     if (op.embedded()) {
         k_extract<T, T><<<embed_grid((long)op.Nl * op.Nl), 256, 0, s>>>(op.Nl, op.Ns, 1, z, z_out);
         count_launches(1);
-        for (void* v : tmp) cudaFreeAsync(v, s);
     }
+    if (moved)
+        ASB_CUDA(cudaMemcpyAsync(z_out, z, (size_t)N * sizeof(T), cudaMemcpyDeviceToDevice, s));
+    for (void* v : tmp)
+        if (v) cudaFreeAsync(v, s);
     ASB_CUDA(cudaGetLastError());
     ASB_CUDA(cudaStreamSynchronize(s));
     cudaFreeAsync(st, s);
@@ -2440,6 +2450,7 @@ template <typename T>
 __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_adj_rz(const PkParams* __restrict__ Pp, PkState* st,
                                                         const T* z, const T* r,
                                                         const uint8_t* mask, double* part) {
+    pdl_wait();
     const PkParams& P = *Pp;
     if (st->halt) return;
     const T zm = (T)st->zmean;
@@ -2469,6 +2480,7 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_adj_rz(const PkP
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_adj_d(const PkParams* __restrict__ Pp, const PkState* st,
                                                        const T* z, const uint8_t* mask, T* d) {
+    pdl_wait();
     const PkParams& P = *Pp;
     if (st->halt) return;
     const T zm = (T)st->zmean, beta = (T)st->beta;
@@ -2489,6 +2501,7 @@ template <typename T>
 __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_adj_dq(const PkParams* __restrict__ Pp, PkState* st,
                                                         const T* d, const T* q,
                                                         const uint8_t* mask, double* part) {
+    pdl_wait();
     const PkParams& P = *Pp;
     if (st->halt) return;
     double acc[2] = {0.0, 0.0};
@@ -2520,6 +2533,7 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_adj_upd(const Pk
                                                          const T* d, const T* q,
                                                          const uint8_t* mask, T* lam, T* r,
                                                          double* part) {
+    pdl_wait();
     const PkParams& P = *Pp;
     if (st->halt) return;
     const T a = (T)st->tau, qm = (T)st->rmean;
@@ -2627,15 +2641,15 @@ void adjoint_core(Operator& op, const double* p, const double* w, double tol, in
         for (int k = 0; k < 16; ++k) {  // kernels return at entry once halted
             const T* zz = r;
             if (precond == ASPHER_PRECOND_STENCIL) {
-                launch_stencil<T, false, false>(radius, op.Ns, op.Nl, dim3(stencil_grid(op.Nl)),
-                                                s, Pd, st, W, r, nullptr, mask, z, part, 1);
+                launch_stencil<T, false, false>(radius, op.Ns, op.Nl, 1, s, Pd, st, W, r, nullptr,
+                                                mask, z, part, 1);
                 zz = z;
             }
-            k_adj_rz<T><<<grid, kRedThreads, 0, s>>>(Pd, st, zz, r, mask, part);
-            k_adj_d<T><<<grid, kRedThreads, 0, s>>>(Pd, st, zz, mask, d);
+            launch_pdl(k_adj_rz<T>, dim3(grid), kRedThreads, 0, s, Pd, st, zz, r, mask, part);
+            launch_pdl(k_adj_d<T>, dim3(grid), kRedThreads, 0, s, Pd, st, zz, mask, d);
             op.matvec(sizeof(T) == 8, d, q, s, &st->halt);
-            k_adj_dq<T><<<grid, kRedThreads, 0, s>>>(Pd, st, d, q, mask, part);
-            k_adj_upd<T><<<grid, kRedThreads, 0, s>>>(Pd, st, d, q, mask, lam, r, part);
+            launch_pdl(k_adj_dq<T>, dim3(grid), kRedThreads, 0, s, Pd, st, d, q, mask, part);
+            launch_pdl(k_adj_upd<T>, dim3(grid), kRedThreads, 0, s, Pd, st, d, q, mask, lam, r, part);
             count_launches(4);
         }
         ASB_CUDA(cudaGetLastError());

@@ -26,7 +26,8 @@ StencilTaps make_stencil_taps(int Ns, int R);
 // spec: B spectra, or nullptr for the operator's own when B = 1).
 // Defined in operators.cu.
 template <typename T>
-void fourier_precond_pk(Operator& op, const T* g, const uint8_t* mask, PkState* st, T* z,
+void fourier_precond_pk(Operator& op, const T* ga, const T* gb, const uint8_t* mask, PkState* st,
+                        T* z,
                         double* part, cudaStream_t s, const int* gate, int B = 1,
                         void* spec = nullptr);
 

@@ -56,6 +56,15 @@ struct PkParams {
 struct PkState {
     // evaluate() -- contact_solver.cpp:260-303
     double alpha, gmin;  // alpha: one-pass mean (g is centred by Real(alpha)); refined below
+    // the uncentred gap v alternates between two buffers: `par` is the one of
+    // the last evaluation (centred by alpha), the other holds the evaluation
+    // before it (centred by alpha_prev), whose centred value is the
+    // reference's g_prev
+    double alpha_prev;
+    int par;
+    // the host (or the p = p_bar fill) has written p since the mask was
+    // formed: the next evaluation reads p at every cell
+    int mask_stale;
     double alpha_ref, gmin_ref;
     double gsum, vmin;
     double pk, G, fw, pen, psum, pv, load, gcs;

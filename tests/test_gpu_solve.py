@@ -244,3 +244,31 @@ def test_eager_loop_matches_graph_loop(dtype):
         assert torch.equal(ma.pressure_device, mb.pressure_device)
     with pytest.raises(ValueError):
         solve_device(op, g0, pbar, loop_mode="stream")
+
+
+@pytest.mark.parametrize("backend,Ns", [("fft", 16), ("fft", 64), ("periodic", 128), ("fft", 48),
+                                        ("periodic", 75), ("fft", 512)])
+@pytest.mark.parametrize("precond", ["none", "fourier"])
+def test_sparse_passes_keep_the_minimiser(backend, Ns, precond):
+    """The vector passes touch a field only where the contact mask (or a
+    negative gap) says so, and t and p are kept at 0 elsewhere: from a full,
+    a sparse and a wrong warm start (contact where there is none in the end),
+    on one solver after other solves, the pressure is the cold solve's to the
+    certificate's accuracy, with the same contact."""
+    from aspher_b200 import ContactSolver
+    from aspher_b200.surfaces import self_affine_gap
+    tol, load = 1e-9, 0.004
+    g = self_affine_gap(Ns, hurst=0.8, rms=0.002, k_lo=1.5, k_hi=Ns / 4, seed=3)
+    s = ContactSolver(Ns, backend=backend)
+    cold = s.solve(g, load, tol=tol, precond=precond)
+    assert cold.status == "converged"
+    rng = np.random.default_rng(5)
+    wrong = np.where(np.asarray(cold.pressure) > 0, 0.0, rng.random((Ns, Ns)))
+    spot = np.zeros((Ns, Ns))
+    spot[Ns // 2, Ns // 2 - 1:Ns // 2 + 1] = 1.0
+    for p0 in (wrong, spot, np.asarray(cold.pressure), np.ones((Ns, Ns))):
+        r = s.solve(g, load, tol=tol, precond=precond, p_init=p0)
+        assert r.status == "converged", (r.status, r.status_reason)
+        err = np.linalg.norm(r.pressure - cold.pressure) / np.linalg.norm(cold.pressure)
+        assert err <= 20 * np.sqrt(tol), err  # two certified points: |dp|_S^2 <= 2 tol P g_ref
+        assert abs(r.contact_area - cold.contact_area) <= 1e-3

@@ -11,11 +11,12 @@
 // runs RPT/R butterflies per stage (j = t + q L/RPT), whose inputs are exactly
 // its own strided registers, so only the stage outputs go through shared
 // memory; the last stage's outputs land back in the strided pattern and stay
-// in registers.  Stages are radix 16 (the remainder last), so a 4096-point
-// transform makes two shared-memory round trips.
+// in registers.  Stages are radix 16, or 32 where a thread holds 32 points (the
+// remainder last), so a 4096-point transform makes two shared-memory round
+// trips, and an 8192-point one two at radix 32 instead of three.
 //
-// Shared memory is addressed as (i + i/16) * S + off: the 1-in-16 padding
-// breaks the power-of-two strides of the stage writes, S > 1 interleaves S
+// Shared memory is addressed as (i + i/16) * S + off (i/32 at radix 32): the
+// padding breaks the power-of-two strides of the stage writes, S > 1 interleaves S
 // independent transforms element by element (the column kernels).
 #pragma once
 
@@ -23,50 +24,97 @@
 
 namespace asb {
 
-// cos/sin(2 pi k / 16), k = 0..7, as plain mathematical constants.
+// cos / sin and cos / tan of 2 pi k / 32, 0 < k < 16, k != 8, as plain
+// mathematical constants
 template <typename T>
-__device__ __forceinline__ void unit16(int k, T& c, T& s) {
-    const T c1 = T(0.92387953251128675613), s1 = T(0.38268343236508977173);
-    const T h = T(0.70710678118654752440);
+__device__ __forceinline__ void unit32(int k, T& c, T& s) {
     switch (k) {
-        case 0: c = T(1); s = T(0); break;
-        case 1: c = c1; s = s1; break;
-        case 2: c = h; s = h; break;
-        case 3: c = s1; s = c1; break;
-        case 4: c = T(0); s = T(1); break;
-        case 5: c = -s1; s = c1; break;
-        case 6: c = -h; s = h; break;
-        default: c = -c1; s = s1; break;
+        case 1: c = T(0.9807852804032304491262); s = T(0.1950903220161282678483); break;
+        case 2: c = T(0.9238795325112867561282); s = T(0.3826834323650897717285); break;
+        case 3: c = T(0.8314696123025452370788); s = T(0.5555702330196022247428); break;
+        case 4: c = T(0.7071067811865475244008); s = T(0.7071067811865475244008); break;
+        case 5: c = T(0.5555702330196022247428); s = T(0.8314696123025452370788); break;
+        case 6: c = T(0.3826834323650897717285); s = T(0.9238795325112867561282); break;
+        case 7: c = T(0.1950903220161282678483); s = T(0.9807852804032304491262); break;
+        case 9: c = T(-0.1950903220161282678483); s = T(0.9807852804032304491262); break;
+        case 10: c = T(-0.3826834323650897717285); s = T(0.9238795325112867561282); break;
+        case 11: c = T(-0.5555702330196022247428); s = T(0.8314696123025452370788); break;
+        case 12: c = T(-0.7071067811865475244008); s = T(0.7071067811865475244008); break;
+        case 13: c = T(-0.8314696123025452370788); s = T(0.5555702330196022247428); break;
+        case 14: c = T(-0.9238795325112867561282); s = T(0.3826834323650897717285); break;
+        case 15: c = T(-0.9807852804032304491262); s = T(0.1950903220161282678483); break;
+        default: c = T(0); s = T(1); break;
+    }
+}
+template <typename T>
+__device__ __forceinline__ void unit32_cos_tan(int k, T& c, T& t) {
+    switch (k) {
+        case 1: c = T(0.9807852804032304491262); t = T(0.1989123673796580069116); break;
+        case 2: c = T(0.9238795325112867561282); t = T(0.4142135623730950488017); break;
+        case 3: c = T(0.8314696123025452370788); t = T(0.6681786379192989199978); break;
+        case 4: c = T(0.7071067811865475244008); t = T(1.0); break;
+        case 5: c = T(0.5555702330196022247428); t = T(1.496605762665489017601); break;
+        case 6: c = T(0.3826834323650897717285); t = T(2.414213562373095048802); break;
+        case 7: c = T(0.1950903220161282678483); t = T(5.027339492125848104515); break;
+        case 9: c = T(-0.1950903220161282678483); t = T(-5.027339492125848104515); break;
+        case 10: c = T(-0.3826834323650897717285); t = T(-2.414213562373095048802); break;
+        case 11: c = T(-0.5555702330196022247428); t = T(-1.496605762665489017601); break;
+        case 12: c = T(-0.7071067811865475244008); t = T(-1.0); break;
+        case 13: c = T(-0.8314696123025452370788); t = T(-0.6681786379192989199978); break;
+        case 14: c = T(-0.9238795325112867561282); t = T(-0.4142135623730950488017); break;
+        case 15: c = T(-0.9807852804032304491262); t = T(-0.1989123673796580069116); break;
+        default: c = T(1); t = T(0); break;
     }
 }
 
-// a * exp(DIR * 2 pi i k / R) for a compile-time R in {2,4,8,16}.
+// the same of 2 pi k / 24, 0 < k < 12, k != 6
+template <typename T>
+__device__ __forceinline__ void unit24(int k, T& c, T& s) {
+    switch (k) {
+        case 1: c = T(0.9659258262890682867497); s = T(0.2588190451025207623489); break;
+        case 2: c = T(0.8660254037844386467637); s = T(0.5); break;
+        case 3: c = T(0.7071067811865475244008); s = T(0.7071067811865475244008); break;
+        case 4: c = T(0.5); s = T(0.8660254037844386467637); break;
+        case 5: c = T(0.2588190451025207623489); s = T(0.9659258262890682867497); break;
+        case 7: c = T(-0.2588190451025207623489); s = T(0.9659258262890682867497); break;
+        case 8: c = T(-0.5); s = T(0.8660254037844386467637); break;
+        case 9: c = T(-0.7071067811865475244008); s = T(0.7071067811865475244008); break;
+        case 10: c = T(-0.8660254037844386467637); s = T(0.5); break;
+        case 11: c = T(-0.9659258262890682867497); s = T(0.2588190451025207623489); break;
+        default: c = T(0); s = T(1); break;
+    }
+}
+template <typename T>
+__device__ __forceinline__ void unit24_cos_tan(int k, T& c, T& t) {
+    switch (k) {
+        case 1: c = T(0.9659258262890682867497); t = T(0.2679491924311227064726); break;
+        case 2: c = T(0.8660254037844386467637); t = T(0.5773502691896257645091); break;
+        case 3: c = T(0.7071067811865475244008); t = T(1.0); break;
+        case 4: c = T(0.5); t = T(1.732050807568877293527); break;
+        case 5: c = T(0.2588190451025207623489); t = T(3.732050807568877293527); break;
+        case 7: c = T(-0.2588190451025207623489); t = T(-3.732050807568877293527); break;
+        case 8: c = T(-0.5); t = T(-1.732050807568877293527); break;
+        case 9: c = T(-0.7071067811865475244008); t = T(-1.0); break;
+        case 10: c = T(-0.8660254037844386467637); t = T(-0.5773502691896257645091); break;
+        case 11: c = T(-0.9659258262890682867497); t = T(-0.2679491924311227064726); break;
+        default: c = T(1); t = T(0); break;
+    }
+}
+// the circle that radix R divides: 32 points, or 24 where 3 divides R
+__host__ __device__ constexpr int unit_points(int R) { return R % 3 == 0 ? 24 : 32; }
+
+// a * exp(DIR * 2 pi i k / R) for a compile-time R that divides 32 or 24.
 template <int R, int DIR, typename T>
 __device__ __forceinline__ cplx<T> rot_const(cplx<T> a, int k) {
-    const int k16 = k * (16 / R);
-    if (k16 == 0) return a;
-    if (k16 == 4) return mul_i<DIR>(a);
+    constexpr int U = unit_points(R);
+    const int ku = k * (U / R);
+    if (ku == 0) return a;
+    if (ku == U / 4) return mul_i<DIR>(a);
     T c, s;
-    unit16<T>(k16, c, s);
+    if constexpr (U == 24) unit24<T>(ku, c, s);
+    else unit32<T>(ku, c, s);
     const T sn = DIR < 0 ? -s : s;
     return mk<T>(a.x * c - a.y * sn, a.x * sn + a.y * c);
-}
-
-// cos and tan of 2 pi k / 16, k in {1, 2, 3, 5, 6, 7}, as plain
-// mathematical constants (tan(pi/8) = sqrt(2) - 1, tan(3 pi/8) = sqrt(2) + 1)
-template <typename T>
-__device__ __forceinline__ void unit16_cos_tan(int k, T& c, T& t) {
-    const T c1 = T(0.92387953251128675613), s1 = T(0.38268343236508977173);
-    const T h = T(0.70710678118654752440);
-    const T t1 = T(0.41421356237309504880), t3 = T(2.41421356237309504880);
-    switch (k) {
-        case 1: c = c1; t = t1; break;
-        case 2: c = h; t = T(1); break;
-        case 3: c = s1; t = t3; break;
-        case 5: c = -s1; t = -t3; break;
-        case 6: c = -h; t = T(-1); break;
-        default: c = -c1; t = -t1; break;
-    }
 }
 
 // The radix-2 butterfly with the odd input rotated by exp(DIR 2 pi i k / R):
@@ -76,17 +124,19 @@ __device__ __forceinline__ void unit16_cos_tan(int k, T& c, T& t) {
 // instructions instead of a four-instruction rotation and four additions.
 template <int R, int DIR, typename T>
 __device__ __forceinline__ void bfly_rot(cplx<T> e, cplx<T> o, int k, cplx<T>& lo, cplx<T>& hi) {
-    const int k16 = k * (16 / R);
-    if (k16 == 0) {
+    constexpr int U = unit_points(R);
+    const int ku = k * (U / R);
+    if (ku == 0) {
         lo = cadd(e, o);
         hi = csub(e, o);
-    } else if (k16 == 4) {
+    } else if (ku == U / 4) {
         const cplx<T> w = mul_i<DIR>(o);
         lo = cadd(e, w);
         hi = csub(e, w);
     } else {
         T c, t;
-        unit16_cos_tan<T>(k16, c, t);
+        if constexpr (U == 24) unit24_cos_tan<T>(ku, c, t);
+        else unit32_cos_tan<T>(ku, c, t);
         if (DIR < 0) t = -t;
         const T ux = fma(-t, o.y, o.x), uy = fma(t, o.x, o.y);
         lo = mk<T>(fma(c, ux, e.x), fma(c, uy, e.y));
@@ -103,6 +153,15 @@ __device__ __forceinline__ void dft(cplx<T>* a) {
         const cplx<T> t = a[0];
         a[0] = cadd(t, a[1]);
         a[1] = csub(t, a[1]);
+    } else if constexpr (R == 3) {
+        // X0 = a0 + s, X1/2 = a0 - s/2 +- DIR i (sqrt 3 / 2) d, s/d = a1 +- a2
+        const T h = T(0.8660254037844386467637);
+        const cplx<T> sm = cadd(a[1], a[2]), d = csub(a[1], a[2]);
+        const cplx<T> m = mk<T>(fma(T(-0.5), sm.x, a[0].x), fma(T(-0.5), sm.y, a[0].y));
+        const cplx<T> r = mul_i<DIR>(d);
+        a[0] = cadd(a[0], sm);
+        a[1] = mk<T>(fma(h, r.x, m.x), fma(h, r.y, m.y));
+        a[2] = mk<T>(fma(-h, r.x, m.x), fma(-h, r.y, m.y));
     } else if constexpr (R == 4) {
         const cplx<T> s02 = cadd(a[0], a[2]), d02 = csub(a[0], a[2]);
         const cplx<T> s13 = cadd(a[1], a[3]);
@@ -119,6 +178,40 @@ __device__ __forceinline__ void dft(cplx<T>* a) {
         dft<R / 2, DIR, T>(o);
 #pragma unroll
         for (int k = 0; k < R / 2; ++k) bfly_rot<R, DIR, T>(e[k], o[k], k, a[k], a[k + R / 2]);
+    }
+}
+
+// Radix-2 butterfly with a general twiddle: lo = e + w o, hi = e - w o in six
+// fused multiply-adds (hi = 2 e - lo).
+template <typename T>
+__device__ __forceinline__ void bfly_tw(cplx<T> e, cplx<T> o, cplx<T> w, cplx<T>& lo, cplx<T>& hi) {
+    const T lx = fma(w.x, o.x, fma(-w.y, o.y, e.x));
+    const T ly = fma(w.x, o.y, fma(w.y, o.x, e.y));
+    hi = mk<T>(fma(T(2), e.x, -lx), fma(T(2), e.y, -ly));
+    lo = mk<T>(lx, ly);
+}
+
+// The DFT of R points of the inputs a[r] w^r, w[l] = w^(2^l): the twiddles go
+// into the butterflies, lo/hi = E[k] +- (w rot^k) O[k], instead of onto the
+// inputs, which takes 13 instead of 15.25 instructions per point at R = 16 and
+// no powers of w beyond w^(R/2).
+template <int R, int DIR, typename T>
+__device__ __forceinline__ void dft_tw(cplx<T>* a, const cplx<T>* w) {
+    if constexpr (R == 2) {
+        bfly_tw<T>(a[0], a[1], w[0], a[0], a[1]);
+    } else if constexpr (R > 2) {
+        cplx<T> e[R / 2], o[R / 2];
+#pragma unroll
+        for (int i = 0; i < R / 2; ++i) { e[i] = a[2 * i]; o[i] = a[2 * i + 1]; }
+        dft_tw<R / 2, DIR, T>(e, w + 1);
+        dft_tw<R / 2, DIR, T>(o, w + 1);
+#pragma unroll
+        for (int k = 0; k < R / 4; ++k) {
+            const cplx<T> t = rot_const<R, DIR, T>(w[0], k);
+            bfly_tw<T>(e[k], o[k], t, a[k], a[k + R / 2]);
+            bfly_tw<T>(e[k + R / 4], o[k + R / 4], mul_i<DIR>(t), a[k + R / 4],
+                       a[k + R / 4 + R / 2]);
+        }
     }
 }
 
@@ -146,19 +239,27 @@ __device__ __forceinline__ void dft_upper_zero(cplx<T>* a) {
 
 __host__ __device__ constexpr int ilog2c(int v) { return v <= 1 ? 0 : 1 + ilog2c(v >> 1); }
 
+// Radix of the stage that has `rem` left to transform, with at most RMAX
+// points per thread.  RMAX = 3 2^k (transforms of 3 2^n points): the first
+// stage takes the factor 3, the later ones powers of two that divide RMAX.
+__host__ __device__ constexpr int next_radix(int rem, int RMAX) {
+    const int cap = RMAX % 3 == 0 && rem % 3 != 0 ? RMAX / 3 : RMAX;
+    return rem >= cap ? cap : rem;
+}
 // Radix of stage `s` for a length-L transform with at most RMAX per stage.
 __host__ __device__ constexpr int stage_radix(int L, int RMAX, int s) {
     int rem = L;
-    for (int i = 0; i < s; ++i) rem /= (rem >= RMAX ? RMAX : rem);
-    return rem >= RMAX ? RMAX : rem;
+    for (int i = 0; i < s; ++i) rem /= next_radix(rem, RMAX);
+    return next_radix(rem, RMAX);
 }
 __host__ __device__ constexpr int num_stages(int L, int RMAX) {
     int n = 0, rem = L;
-    while (rem > 1) { rem /= (rem >= RMAX ? RMAX : rem); ++n; }
+    while (rem > 1) { rem /= next_radix(rem, RMAX); ++n; }
     return n;
 }
 
-__device__ __forceinline__ int smaddr(int i, int S, int off) { return (i + (i >> 4)) * S + off; }
+template <int PS = 4>
+__device__ __forceinline__ int smaddr(int i, int S, int off) { return (i + (i >> PS)) * S + off; }
 
 // smaddr(i0 + m * STEP) as a per-thread base plus a compile-time offset where
 // the padding term splits.  For STEP a multiple of 16, (i0 + m STEP) >> 4 =
@@ -166,11 +267,13 @@ __device__ __forceinline__ int smaddr(int i, int S, int off) { return (i + (i >>
 // RUN-aligned group that every i0 + m STEP stays in; for RUN <= 16 that group
 // lies inside one 16-element block, so the padding term does not change
 // with m.
-template <int STEP, int RUN>
+// PS: one element of padding per 2^PS.
+template <int STEP, int RUN, int PS = 4>
 __device__ __forceinline__ int smaddr_run(int i0, int m, int S, int off) {
-    if constexpr (STEP % 16 == 0) return smaddr(i0, S, off) + m * (STEP + STEP / 16) * S;
-    else if constexpr (RUN <= 16) return smaddr(i0, S, off) + m * STEP * S;
-    else return smaddr(i0 + m * STEP, S, off);
+    constexpr int PAD1 = 1 << PS;
+    if constexpr (STEP % PAD1 == 0) return smaddr<PS>(i0, S, off) + m * (STEP + STEP / PAD1) * S;
+    else if constexpr (RUN <= PAD1 && (RUN & (RUN - 1)) == 0) return smaddr<PS>(i0, S, off) + m * STEP * S;
+    else return smaddr<PS>(i0 + m * STEP, S, off);
 }
 
 // a * w (forward) or a * conj(w) (inverse), w from the exp(-2 pi i k/L) table
@@ -186,7 +289,14 @@ template <typename T, int L, int RPT, int DIR, int S, int STAGE, int SPAN, bool 
           int P0>
 __device__ __forceinline__ void fft_stages(cplx<T> (&v)[RPT], int t, cplx<T>* sm, int off,
                                            const cplx<T>* __restrict__ tw) {
-    constexpr int RMAX = RPT < 16 ? RPT : 16;
+    constexpr int RMAX = RPT < 32 ? RPT : 32;
+    // one element of padding per radix of the first stage's writes
+    constexpr int PS = RPT < 32 ? 4 : 5;
+    // twiddles in the butterflies (dft_tw) or on the inputs: FP64 with 16
+    // points per thread spills with dft_tw (the 4096-point column 77.9 -> 83
+    // us); FP32 needs fewer registers with it (4096 points: 92 -> 88, 39.6 ->
+    // 39.0 us) and 32 points per thread would need 31 powers of w
+    constexpr bool TWB = sizeof(T) == 4 || RPT >= 32;
     constexpr int NST = num_stages(L, RMAX);
     if constexpr (STAGE < NST) {
         constexpr int R = stage_radix(L, RMAX, STAGE);
@@ -203,7 +313,17 @@ __device__ __forceinline__ void fft_stages(cplx<T> (&v)[RPT], int t, cplx<T>* sm
             cplx<T> a[R];
 #pragma unroll
             for (int r = 0; r < R; ++r) a[r] = v[q + r * Q];
-            if constexpr (SPAN > 1) {
+            if constexpr (SPAN > 1 && TWB) {
+                const int jm = j % SPAN;
+                const cplx<T>* __restrict__ tb = tw - L;  // tables at offset = length
+                cplx<T> w[5];  // w^(2^l), entry jm of the length-(SPAN R / 2^l) table
+#pragma unroll
+                for (int l = 0; (1 << l) < R; ++l) {
+                    w[l] = __ldg(&tb[(SPAN * R >> l) + jm]);
+                    if (DIR > 0) w[l].y = -w[l].y;
+                }
+                dft_tw<R, DIR, T>(a, w);
+            } else if constexpr (SPAN > 1) {
                 // w^r for r = 1..R-1 from the loaded powers w, w^2, w^4, w^8
                 // (products at most three deep), applied as each is formed.
                 // w^(2^e) = exp(-2 pi i jm / (SPAN R / 2^e)) is entry jm of the
@@ -244,7 +364,7 @@ __device__ __forceinline__ void fft_stages(cplx<T> (&v)[RPT], int t, cplx<T>* sm
             // for m >= RPT / 2 exactly when r >= R / 2
             if constexpr (HZ && STAGE == 0 && R >= 2)
                 dft_upper_zero<R, DIR, T>(a);
-            else
+            else if constexpr (SPAN == 1 || !TWB)
                 dft<R, DIR, T>(a);
             if constexpr (LAST) {
 #pragma unroll
@@ -252,13 +372,13 @@ __device__ __forceinline__ void fft_stages(cplx<T> (&v)[RPT], int t, cplx<T>* sm
             } else {
                 const int base = (j / SPAN) * SPAN * R + (j % SPAN);
 #pragma unroll
-                for (int r = 0; r < R; ++r) ws[smaddr_run<SPAN, SPAN * R>(base, r, S, off)] = a[r];
+                for (int r = 0; r < R; ++r) ws[smaddr_run<SPAN, SPAN * R, PS>(base, r, S, off)] = a[r];
             }
         }
         if constexpr (!LAST) {
             __syncthreads();
 #pragma unroll
-            for (int m = 0; m < RPT; ++m) v[m] = ws[smaddr_run<TT, 1 << 30>(t, m, S, off)];
+            for (int m = 0; m < RPT; ++m) v[m] = ws[smaddr_run<TT, 1 << 30, PS>(t, m, S, off)];
             // one workspace: nobody writes it again before everyone has read
             // it.  Two (ALT > 0): the next round trip writes the other one,
             // and the one after that follows the next round trip's barrier,
@@ -269,10 +389,11 @@ __device__ __forceinline__ void fft_stages(cplx<T> (&v)[RPT], int t, cplx<T>* sm
     }
 }
 
-// Length-L transform of the strided register pattern; DIR = -1 forward
+// Length-L transform (L = 2^n, or 3 2^n with RPT = 24) of the strided
+// register pattern; DIR = -1 forward
 // (exp(-2 pi i jk/L)), +1 inverse, both unnormalised.  tw points at the
 // length-L table exp(-2 pi i k / L), k < L, inside one array that holds the
-// table of every power-of-two length M <= L at offset M (so tw - L is the
+// table of every length M = L / 2^j at offset M (so tw - L is the
 // array base and the stages read the shorter tables).  Every thread of the CTA must
 // call this (it contains __syncthreads), including threads whose transform
 // is a dummy.  HZ: the upper half of the input is zero (v[m] = 0 for
@@ -294,7 +415,7 @@ __device__ __forceinline__ void block_fft(cplx<T> (&v)[RPT], int t, cplx<T>* sm,
 // P0: the workspace its last round trip did not read
 template <int L, int RPT>
 __host__ __device__ constexpr int ping_pong_next(int p0) {
-    return (p0 + num_stages(L, RPT < 16 ? RPT : 16) - 1) & 1;
+    return (p0 + num_stages(L, RPT < 32 ? RPT : 32) - 1) & 1;
 }
 
 }  // namespace asb

@@ -11,8 +11,8 @@
 
 namespace asb {
 
-// small sizes collapse to variant 0
-__host__ __device__ constexpr int vclamp(int L, int V) { return L >= 128 ? V : 0; }
+// small transforms run the small-CTA variant
+__host__ __device__ constexpr int vclamp(int L, int V) { return L >= 128 ? V : 3; }
 
 // max dynamic shared memory + max-shared carveout, once per kernel per device
 void fft_attrs(const void* func, int bytes);
@@ -44,23 +44,19 @@ void launch_pdl(void (*k)(P...), dim3 grid, int threads, int smem, cudaStream_t 
 template <typename T, int LR, bool PAD, int V, class Load, class Store>
 void launch_row_fwd(Load ld, Store st, int nrows, cudaStream_t s, const int* gate, int B = 1) {
     constexpr int rb = row_rb_v<T>(LR, V), thr = row_threads<T>(LR, V);
-    constexpr int sm = row_fwd_smem<T, LR, PAD, V, Load>();
+    constexpr int sm = row_smem_v<T>(LR, V);
     auto k = row_fwd_kernel<T, LR, PAD, V, Load, Store>;
     fft_attrs((const void*)k, sm);
-    const int units = (nrows + rb - 1) / rb;
-    const int gx = row_fwd_staged<T, LR, PAD, V, Load::kRaw>()
-                       ? persistent_blocks((const void*)k, thr, sm, units) : units;
+    const int gx = (nrows + rb - 1) / rb;
     launch_pdl(k, dim3(gx, B), thr, sm, s, ld, st, nrows, tw<T>(LR), tw<T>(2 * LR), gate);
 }
 template <typename T, int LR, bool PAD, int V, class Load, class Store>
 void launch_row_inv(Load ld, Store st, int nrows, cudaStream_t s, const int* gate, int B = 1) {
     constexpr int rb = row_rb_v<T>(LR, V), thr = row_threads<T>(LR, V);
-    constexpr int sm = row_inv_smem<T, LR, PAD, V, Load>();
+    constexpr int sm = row_smem_v<T>(LR, V);
     auto k = row_inv_kernel<T, LR, PAD, V, Load, Store>;
     fft_attrs((const void*)k, sm);
-    const int units = (nrows + rb - 1) / rb;
-    const int gx = row_inv_staged<T, LR, PAD, V, Load::kTiled>()
-                       ? persistent_blocks((const void*)k, thr, sm, units) : units;
+    const int gx = (nrows + rb - 1) / rb;
     launch_pdl(k, dim3(gx, B), thr, sm, s, ld, st, nrows, tw<T>(LR), tw<T>(2 * LR), gate);
 }
 template <typename T, int LC, int NCM1, bool PAD, int V, class Mult>

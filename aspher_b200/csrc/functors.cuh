@@ -25,7 +25,6 @@ struct LoadRealRows {  // z[n] = (x[row*pitch + 2n], x[row*pitch + 2n + 1])
     // rescale of sc[blockIdx.y] as it is loaded
     const PkState* sc = nullptr;
     static constexpr bool kTiled = false;
-    static constexpr bool kRaw = true;  // plain rows: the row kernel may stage them
     __device__ __forceinline__ cplx<T> fix(cplx<T> v) const {
         if (sc) {
             v.x = pending_scale(sc, v.x);
@@ -61,7 +60,6 @@ struct LoadBlockRows {
     int Nl;
     long bs;
     static constexpr bool kTiled = false;
-    static constexpr bool kRaw = false;
     __device__ __forceinline__ cplx<T> operator()(int row, int n) const {
         cplx<T> z = mk<T>(T(0), T(0));
         if (row < Nl) {
@@ -94,7 +92,6 @@ struct StoreBlockRows {
 // difference in FP32.
 struct LoadDiffRows {
     static constexpr bool kTiled = false;
-    static constexpr bool kRaw = false;
     const double* x;
     const double* x0;
     int pitch;
@@ -158,7 +155,6 @@ struct LoadTiled {
     int nrows, ct;
     long bs;
     static constexpr bool kTiled = true;  // row kernels load whole tile chunks
-    static constexpr bool kRaw = false;
     __device__ __forceinline__ cplx<T> operator()(int row, int k) const {
         return base[blockIdx.y * bs + (size_t)(k / ct) * nrows * ct + (size_t)row * ct +
                     (k % ct)];

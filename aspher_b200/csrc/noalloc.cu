@@ -108,9 +108,9 @@ struct NaKernels {
     static constexpr auto fwd = row_fwd_kernel<T, LR, false, V, LoadRealRows<T>, StoreTiled<T>>;
     static constexpr auto col = col_kernel<T, LC, LR, false, V, PeriodicMult<T>>;
     static constexpr auto inv = row_inv_kernel<T, LR, false, V, LoadTiled<T>, StoreRealRows<T>>;
-    static constexpr int sm_fwd = row_fwd_smem<T, LR, false, V, LoadRealRows<T>>();
+    static constexpr int sm_fwd = row_smem_v<T>(LR, V);
     static constexpr int sm_col = col_smem_total<T, LC, LR, false, V>();
-    static constexpr int sm_inv = row_inv_smem<T, LR, false, V, LoadTiled<T>>();
+    static constexpr int sm_inv = row_smem_v<T>(LR, V);
     // their shared-memory attributes, set once per device, precision and size
     static void prepare(NaDevice& d) {
         const unsigned bit = 1u << ((sizeof(T) == 8 ? 16 : 0) + ilog2c(NS));

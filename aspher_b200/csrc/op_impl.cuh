@@ -14,19 +14,22 @@
 namespace asb {
 
 // Fastest (row, column) variant pairs measured on B200: every pair set on
-// one operator (aspher_op_set_variants) and its apply timed with CUDA
-// events, L2 flushed between applies, median of 15; sizes not listed use
-// variant 0.  Operator::autotune repeats the search in-process.
+// one operator (aspher_op_set_variants) and 6-20 of its applies timed in a
+// CUDA graph (sides of 3 2^k: the passes alone); sizes not listed use variant
+// 0.  Operator::autotune repeats the search in-process.
 struct VariantRow {
     int kind, dbl, Ns, rv, cv;
 };
 constexpr VariantRow kVariantTable[] = {
-    {0, 0, 256, 2, 3}, {0, 0, 512, 2, 1}, {0, 0, 1024, 1, 1}, {0, 0, 2048, 1, 0},
-    {0, 0, 4096, 0, 1}, {0, 0, 8192, 1, 2}, {0, 1, 256, 1, 1}, {0, 1, 512, 1, 1},
-    {0, 1, 1024, 0, 1}, {0, 1, 2048, 2, 0}, {0, 1, 4096, 0, 0}, {1, 0, 256, 3, 3},
-    {1, 0, 512, 0, 3}, {1, 0, 1024, 2, 3}, {1, 0, 2048, 1, 1}, {1, 0, 4096, 1, 0},
-    {1, 0, 8192, 0, 1}, {1, 1, 256, 3, 3}, {1, 1, 512, 1, 3}, {1, 1, 1024, 2, 2},
-    {1, 1, 2048, 2, 0}, {1, 1, 4096, 2, 0}, {1, 1, 8192, 0, 0},
+    {0, 0, 64, 3, 3}, {0, 0, 128, 3, 3}, {0, 0, 256, 3, 3}, {0, 0, 512, 2, 1},
+    {0, 0, 768, 2, 2}, {0, 0, 1024, 1, 1}, {0, 0, 1536, 0, 2}, {0, 0, 2048, 1, 2},
+    {0, 0, 3072, 0, 0}, {0, 0, 4096, 0, 2}, {0, 0, 8192, 0, 2}, {0, 1, 64, 3, 3},
+    {0, 1, 128, 3, 3}, {0, 1, 256, 3, 3}, {0, 1, 512, 3, 1}, {0, 1, 768, 2, 2},
+    {0, 1, 1024, 1, 1}, {0, 1, 1536, 0, 2}, {0, 1, 2048, 1, 1}, {0, 1, 3072, 0, 0},
+    {0, 1, 4096, 0, 2}, {1, 0, 128, 3, 3}, {1, 0, 256, 3, 3}, {1, 0, 512, 3, 3},
+    {1, 0, 1024, 3, 1}, {1, 0, 2048, 1, 2}, {1, 0, 4096, 1, 2}, {1, 0, 8192, 0, 2},
+    {1, 1, 128, 3, 3}, {1, 1, 256, 3, 3}, {1, 1, 512, 3, 3}, {1, 1, 1024, 3, 1},
+    {1, 1, 2048, 2, 1}, {1, 1, 4096, 2, 0}, {1, 1, 8192, 0, 2},
 };
 constexpr VariantRow default_variants(int kind, int dbl, int Ns) {
     for (const VariantRow& e : kVariantTable)
@@ -62,29 +65,29 @@ void launch_col_split(cplx<T>* spec, cplx<T>* acc, int nrows, int ndata, Mult m,
         default: throw Error(-1, "FFT launch variant out of range");              \
     }
 
-// ALLV = false: launch variant 0 whatever v is (one instantiation per pass;
-// the grids above kMaxVariantNs)
-template <typename T, int LR, bool PAD, bool ALLV = true, class Load, class Store>
+// ONLY >= 0: launch variant ONLY whatever v is (one instantiation per pass:
+// the grids above kMaxVariantNs and those of 3 2^k)
+template <typename T, int LR, bool PAD, int ONLY = -1, class Load, class Store>
 void row_fwd_v(int v, Load ld, Store st, int nrows, cudaStream_t s, const int* gate, int B) {
-    if constexpr (!ALLV) {
-        launch_row_fwd<T, LR, PAD, vclamp(LR, 0), Load, Store>(ld, st, nrows, s, gate, B);
+    if constexpr (ONLY >= 0) {
+        launch_row_fwd<T, LR, PAD, ONLY, Load, Store>(ld, st, nrows, s, gate, B);
     } else {
         ASB_V_SWITCH(v, LR, (launch_row_fwd<T, LR, PAD, V, Load, Store>(ld, st, nrows, s, gate, B)));
     }
 }
-template <typename T, int LR, bool PAD, bool ALLV = true, class Load, class Store>
+template <typename T, int LR, bool PAD, int ONLY = -1, class Load, class Store>
 void row_inv_v(int v, Load ld, Store st, int nrows, cudaStream_t s, const int* gate, int B) {
-    if constexpr (!ALLV) {
-        launch_row_inv<T, LR, PAD, vclamp(LR, 0), Load, Store>(ld, st, nrows, s, gate, B);
+    if constexpr (ONLY >= 0) {
+        launch_row_inv<T, LR, PAD, ONLY, Load, Store>(ld, st, nrows, s, gate, B);
     } else {
         ASB_V_SWITCH(v, LR, (launch_row_inv<T, LR, PAD, V, Load, Store>(ld, st, nrows, s, gate, B)));
     }
 }
-template <typename T, int LC, int NCM1, bool PAD, bool ALLV = true, class Mult>
+template <typename T, int LC, int NCM1, bool PAD, int ONLY = -1, class Mult>
 void col_v(int v, cplx<T>* spec, int nrows, int ndata, Mult m, cudaStream_t s, const int* gate,
            int B) {
-    if constexpr (!ALLV) {
-        launch_col<T, LC, NCM1, PAD, vclamp(LC, 0), Mult>(spec, nrows, ndata, m, s, gate, B);
+    if constexpr (ONLY >= 0) {
+        launch_col<T, LC, NCM1, PAD, ONLY, Mult>(spec, nrows, ndata, m, s, gate, B);
     } else {
         ASB_V_SWITCH(v, LC, (launch_col<T, LC, NCM1, PAD, V, Mult>(spec, nrows, ndata, m, s, gate, B)));
     }
@@ -107,10 +110,14 @@ struct FreeImpl {
     // at Ns = 8192); otherwise the column pass runs as two length-Ns halves
     // (col_split_kernel), instantiated for Ns >= kSplitMin
     static constexpr bool kFits = col_fits<T>(LC);
-    static constexpr bool kSplitOK = NS >= kSplitMin && col_fits<T>(LR);
+    static constexpr bool kSplitOK = NS >= kSplitMin && NS % 3 != 0 && col_fits<T>(LR);
     // rows and columns in one CTA each (every size but FP64 above 8192)
     static constexpr bool kSupported = row_smem_v<T>(LR, 0) <= kSmemPerSM && (kFits || kSplitOK);
-    static constexpr bool kAllV = NS <= kMaxVariantNs;
+    static constexpr bool kAllV = NS <= kMaxVariantNs && NS % 3 != 0;
+    // launch variants of the passes with one instantiation per size
+    static constexpr VariantRow kDefault = default_variants(OP_FFT, sizeof(T) == 8, NS);
+    static constexpr int kRV = vclamp(LR, kDefault.rv), kCV = vclamp(LC, kDefault.cv);
+    static constexpr int kOnlyR = kAllV ? -1 : kRV, kOnlyC = kAllV ? -1 : kCV;
     static bool split(const Operator& op) { return !kFits || (kSplitOK && op.split_cols); }
     // spectrum sized for the widest tile (16 columns); the split form keeps
     // its first half-column result in a second spectrum-shaped block after
@@ -118,15 +125,15 @@ struct FreeImpl {
     static size_t spec_elems(bool sp) { return (size_t)(LR + 16) * NS * (sp ? 2 : 1); }
     static int ct(int cv, bool sp) {
         if (sp) return col_ct_v<T>(LR, LR, vclamp(LR, 0));
-        return kAllV ? col_ct_rt<T, LC, LR>(cv) : col_ct_v<T>(LC, LR, vclamp(LC, 0));
+        return kAllV ? col_ct_rt<T, LC, LR>(cv) : col_ct_v<T>(LC, LR, kCV);
     }
 
     // row_fwd(ld) -> col(x Kh) -> row_inv(st); ld / st see the Ns x Ns
     // field(s), of which the first op.Nl rows hold data (all of them unless
     // the operator is embedded): the row passes run on those rows alone and
-    // the column pass takes the rest as zero.  RV >= 0: row launch variant
-    // RV instead of the operator's.
-    template <int RV = -1, class Load, class Store>
+    // the column pass takes the rest as zero.  RF, RI >= 0: launch variant of
+    // the forward / inverse row pass instead of the operator's.
+    template <int RF = -1, int RI = RF, class Load, class Store>
     static void apply(const Operator& op, Load ld, Store st, cplx<T>* spec, cudaStream_t s,
                       const int* gate, int B, const T* kh_over = nullptr) {
         if constexpr (!kSupported) {
@@ -140,19 +147,19 @@ struct FreeImpl {
             const int nd = op.Nl;
             const StoreTiled<T> sst{spec, NS, c, bsp};
             const LoadTiled<T> sld{spec, NS, c, bsp};
-            if constexpr (RV >= 0) launch_row_fwd<T, LR, true, RV>(ld, sst, nd, s, gate, B);
-            else row_fwd_v<T, LR, true, kAllV>(rv, ld, sst, nd, s, gate, B);
+            if constexpr (RF >= 0) launch_row_fwd<T, LR, true, RF>(ld, sst, nd, s, gate, B);
+            else row_fwd_v<T, LR, true, kOnlyR>(rv, ld, sst, nd, s, gate, B);
             if (split(op)) {
                 if constexpr (kSplitOK)
                     launch_col_split<T, LR, LR>(spec, spec + (size_t)B * bsp, NS, nd,
                                                 KhMult<T>{kh, NS + 1, LC, c}, s, gate, B);
             } else {
                 if constexpr (kFits)
-                    col_v<T, LC, LR, true, kAllV>(cv, spec, NS, nd, KhMult<T>{kh, NS + 1, LC, c},
+                    col_v<T, LC, LR, true, kOnlyC>(cv, spec, NS, nd, KhMult<T>{kh, NS + 1, LC, c},
                                                   s, gate, B);
             }
-            if constexpr (RV >= 0) launch_row_inv<T, LR, true, RV>(sld, st, nd, s, gate, B);
-            else row_inv_v<T, LR, true, kAllV>(rv, sld, st, nd, s, gate, B);
+            if constexpr (RI >= 0) launch_row_inv<T, LR, true, RI>(sld, st, nd, s, gate, B);
+            else row_inv_v<T, LR, true, kOnlyR>(rv, sld, st, nd, s, gate, B);
             count_launches(split(op) ? 4 : 3);
             ASB_CUDA(cudaGetLastError());
         }
@@ -168,9 +175,7 @@ struct FreeImpl {
     // size's default row variant (one instantiation per size)
     static void apply_block(const Operator& op, const T* x, T* y, long nl, cplx<T>* spec,
                             cudaStream_t s) {
-        constexpr int RV = kAllV ? vclamp(LR, default_variants(OP_FFT, sizeof(T) == 8, NS).rv)
-                                 : vclamp(LR, 0);
-        apply<RV>(op, LoadBlockRows<T>{x, op.Nl, nl}, StoreBlockRows<T>{y, op.Nl, nl}, spec, s,
+        apply<kRV>(op, LoadBlockRows<T>{x, op.Nl, nl}, StoreBlockRows<T>{y, op.Nl, nl}, spec, s,
                   nullptr, 1);
     }
 };
@@ -183,10 +188,16 @@ struct PeriodicImpl {
     static constexpr bool kAllV = NS <= kMaxVariantNs;
     static size_t spec_elems() { return (size_t)(LR + 16) * NS; }
     static int ct(int cv) {
-        return kAllV ? col_ct_rt<T, LC, LR>(cv) : col_ct_v<T>(LC, LR, vclamp(LC, 0));
+        return kAllV ? col_ct_rt<T, LC, LR>(cv)
+                     : col_ct_v<T>(LC, LR, vclamp(LC, default_variants(OP_PERIODIC, sizeof(T) == 8, NS).cv));
     }
 
-    template <class Load, class Mult, class Store>
+    static constexpr VariantRow kDefault = default_variants(OP_PERIODIC, sizeof(T) == 8, NS);
+    static constexpr int kRV = vclamp(LR, kDefault.rv), kCV = vclamp(LC, kDefault.cv);
+    static constexpr int kOnlyR = kAllV ? -1 : kRV, kOnlyC = kAllV ? -1 : kCV;
+
+    // RF, RI as in FreeImpl::apply
+    template <int RF = -1, int RI = RF, class Load, class Mult, class Store>
     static void apply(int rv, int cv, Load ld, Mult mult, Store st, cplx<T>* spec, cudaStream_t s,
                       const int* gate, int B) {
         if constexpr (!kSupported) {
@@ -195,9 +206,13 @@ struct PeriodicImpl {
         } else {
             const int c = ct(cv);
             const long bsp = (long)(LR / c + 1) * NS * c;
-            row_fwd_v<T, LR, false, kAllV>(rv, ld, StoreTiled<T>{spec, NS, c, bsp}, NS, s, gate, B);
-            col_v<T, LC, LR, false, kAllV>(cv, spec, NS, NS, mult, s, gate, B);
-            row_inv_v<T, LR, false, kAllV>(rv, LoadTiled<T>{spec, NS, c, bsp}, st, NS, s, gate, B);
+            const StoreTiled<T> sst{spec, NS, c, bsp};
+            const LoadTiled<T> sld{spec, NS, c, bsp};
+            if constexpr (RF >= 0) launch_row_fwd<T, LR, false, RF>(ld, sst, NS, s, gate, B);
+            else row_fwd_v<T, LR, false, kOnlyR>(rv, ld, sst, NS, s, gate, B);
+            col_v<T, LC, LR, false, kOnlyC>(cv, spec, NS, NS, mult, s, gate, B);
+            if constexpr (RI >= 0) launch_row_inv<T, LR, false, RI>(sld, st, NS, s, gate, B);
+            else row_inv_v<T, LR, false, kOnlyR>(rv, sld, st, NS, s, gate, B);
             count_launches(3);
             ASB_CUDA(cudaGetLastError());
         }
@@ -227,7 +242,6 @@ struct PeriodicImpl {
 template <typename T>
 struct LoadMaskCentered {  // contact ? g - T(gsum/ng) : 0, pairwise; g = v - T(alpha)
     static constexpr bool kTiled = false;
-    static constexpr bool kRaw = false;
     const T* ga;  // the gap is in ga or gb (PkState::par)
     const T* gb;
     const uint8_t* mask;
@@ -343,6 +357,14 @@ struct EmbeddedFourierImpl {
         case 8192: { constexpr int NS = 8192; __VA_ARGS__; } break; \
         case 16384: { constexpr int NS = 16384; __VA_ARGS__; } break; \
         default: throw Error(-1, "grid_size must be a power of two in [16, 16384]"); \
+    }
+// the same with the embedded grids' sides of 3 2^k (free-space pipeline)
+#define ASB_FREE_SWITCH(NSV, ...)                       \
+    switch (NSV) {                                       \
+        case 768: { constexpr int NS = 768; __VA_ARGS__; } break;   \
+        case 1536: { constexpr int NS = 1536; __VA_ARGS__; } break; \
+        case 3072: { constexpr int NS = 3072; __VA_ARGS__; } break; \
+        default: ASB_SIZE_SWITCH(NSV, __VA_ARGS__)       \
     }
 
 // what op_free_*.cu and op_periodic_*.cu define for their pipeline and T

@@ -37,6 +37,7 @@ namespace asb {
 // ----------------------------------------------------------------------------
 namespace {
 void* g_tw[64][2] = {};  // [device][dbl]
+void* g_tw3[64][2] = {};
 
 void build_tw(int dev) {
     std::vector<double2> hd(2 * kMaxTw);
@@ -55,6 +56,25 @@ void build_tw(int dev) {
     ASB_CUDA(cudaMalloc(&pf, hf.size() * sizeof(float2)));
     ASB_CUDA(cudaMemcpy(pd, hd.data(), hd.size() * sizeof(double2), cudaMemcpyHostToDevice));
     ASB_CUDA(cudaMemcpy(pf, hf.data(), hf.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    // lengths 3 2^j, the table of length L at offset L of an array of their own
+    std::vector<double2> hd3(2 * kMaxTw3);
+    std::vector<float2> hf3(2 * kMaxTw3);
+    for (int L = 3; L <= kMaxTw3; L <<= 1) {
+        for (int k = 0; k < L; ++k) {
+            const long double a = -2.0L * 3.14159265358979323846264338327950288L *
+                                  (long double)k / (long double)L;
+            const long double c = cosl(a), s = sinl(a);
+            hd3[L + k] = make_double2((double)c, (double)s);
+            hf3[L + k] = make_float2((float)c, (float)s);
+        }
+    }
+    void *pd3 = nullptr, *pf3 = nullptr;
+    ASB_CUDA(cudaMalloc(&pd3, hd3.size() * sizeof(double2)));
+    ASB_CUDA(cudaMalloc(&pf3, hf3.size() * sizeof(float2)));
+    ASB_CUDA(cudaMemcpy(pd3, hd3.data(), hd3.size() * sizeof(double2), cudaMemcpyHostToDevice));
+    ASB_CUDA(cudaMemcpy(pf3, hf3.data(), hf3.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    g_tw3[dev][1] = pd3;
+    g_tw3[dev][0] = pf3;
     g_tw[dev][1] = pd;
     g_tw[dev][0] = pf;
 }
@@ -68,12 +88,22 @@ const void* tw_table(bool dbl, int L) {
         std::lock_guard<std::recursive_mutex> lk(setup_mutex());
         if (!g_tw[dev][0]) build_tw(dev);
     }
+    if (L % 3 == 0) {
+        if (L < 1 || L > kMaxTw3) throw Error(-1, "twiddle length out of range");
+        if (dbl) return static_cast<const double2*>(g_tw3[dev][1]) + L;
+        return static_cast<const float2*>(g_tw3[dev][0]) + L;
+    }
     if (L < 1 || L > kMaxTw) throw Error(-1, "twiddle length out of range");
     if (dbl) return static_cast<const double2*>(g_tw[dev][1]) + L;
     return static_cast<const float2*>(g_tw[dev][0]) + L;
 }
 
 bool is_pow2(long v) { return v > 0 && (v & (v - 1)) == 0; }
+
+int embed_side(int Nl, int nc, int largest) {
+    const int n3 = nc / 4 * 3;
+    return n3 >= kMinTripleNs && Nl <= n3 && n3 <= largest ? n3 : nc;
+}
 
 std::recursive_mutex& setup_mutex() {
     static std::recursive_mutex m;
@@ -152,7 +182,6 @@ __global__ void love_table_kernel(double* __restrict__ tab, int Ns, double h, do
 // with row/column Ns zero (fft_operator.cpp:31-44), generated on the fly.
 struct LoadEmbedded {
     static constexpr bool kTiled = false;
-    static constexpr bool kRaw = false;
     const double* tab;
     int Ns, M;
     __device__ __forceinline__ double at(int iy, int ix) const {
@@ -211,7 +240,6 @@ struct StoreRealTracked {
 // transforms the odd samples and combines while storing (StoreSplitCombine).
 struct LoadEmbeddedPar {  // z[n] = (x[4n + p], x[4n + 2 + p]) of an embedded row
     static constexpr bool kTiled = false;
-    static constexpr bool kRaw = false;
     LoadEmbedded e;
     int p;
     __device__ __forceinline__ double2 operator()(int row, int n) const {
@@ -220,7 +248,6 @@ struct LoadEmbeddedPar {  // z[n] = (x[4n + p], x[4n + 2 + p]) of an embedded ro
 };
 struct LoadRealRowsPar {  // the same sampling of plain rows
     static constexpr bool kTiled = false;
-    static constexpr bool kRaw = false;
     const double* x;
     int pitch, p;
     __device__ __forceinline__ double2 operator()(int row, int n) const {
@@ -363,7 +390,7 @@ struct KhBuild {
     static constexpr bool kRowFits = row_smem_v<double>(NS, 0) <= kSmemPerSM;
     static bool split(const Operator& op) {
         if (!kRowFits) return true;
-        return NS >= kSplitMin && op.split_kh;
+        return NS >= kSplitMin && NS % 3 != 0 && op.split_kh;
     }
     static void run(Operator& op) {
         const size_t nk = (size_t)(NS + 1) * (NS + 1);
@@ -384,7 +411,7 @@ struct KhBuild {
                             1.0 / ((double)M * (double)M), mx + 2, 0.0, 0.0};
         const LoadEmbedded emb{table, NS, M};
         if (split(op)) {
-            if constexpr (NS >= kSplitMin) {
+            if constexpr (NS >= kSplitMin && NS % 3 != 0) {
                 constexpr int LH = NS / 2;  // real length Ns per parity
                 double2* E = nullptr;
                 ASB_CUDA(cudaMalloc(&E, (size_t)M * (LH + 1) * sizeof(double2)));
@@ -582,11 +609,12 @@ Operator::Operator(int kind_, int Ns_, double L_, double E_, int flags)
     if (!(E_star > 0.0) || !std::isfinite(E_star)) throw Error(-1, "E_star must be positive");
     if (flags & ~(OPF_SPLIT_COLUMNS | OPF_SPLIT_KH)) throw Error(-1, "unknown operator flags");
     if (!is_pow2(Nl) || Nl < 16) {
-        // embedded: the free-space pipeline of the next power of two
+        // embedded: the free-space pipeline of the next power of two, or of
+        // three quarters of it where the block fits that
         if (flags) throw Error(-1, "operator flags need a power-of-two grid_size in [16, 16384]");
         int nc = 16;
         while (nc < Nl) nc *= 2;
-        Ns = nc;
+        Ns = embed_side(Nl, nc, kMaxTripleNs);
         kind = OP_FFT;
     }
     std::lock_guard<std::recursive_mutex> setup(setup_mutex());
@@ -610,7 +638,7 @@ Operator::Operator(int kind_, int Ns_, double L_, double E_, int flags)
         } else {
             periodic_kernel_table(Nl, Ns, scale, table);
         }
-        ASB_SIZE_SWITCH(Ns, KhBuild<NS>::run(*this));
+        ASB_FREE_SWITCH(Ns, KhBuild<NS>::run(*this));
         const size_t nt = (size_t)(Ns + 16) * (Ns + 1);  // widest tiling
         if (supports(true)) {  // no FP64 copy where FP64 applies do not exist
             ASB_CUDA(cudaMalloc(&kh_d, nt * sizeof(double)));
@@ -654,8 +682,8 @@ Operator::~Operator() {
 int Operator::col_tile(bool dbl, int cv) const {
     int c = 1;
     if (kind == OP_FFT) {
-        if (dbl) { ASB_SIZE_SWITCH(Ns, c = FreeImpl<double, NS>::ct(cv, FreeImpl<double, NS>::split(*this))); }
-        else { ASB_SIZE_SWITCH(Ns, c = FreeImpl<float, NS>::ct(cv, FreeImpl<float, NS>::split(*this))); }
+        if (dbl) { ASB_FREE_SWITCH(Ns, c = FreeImpl<double, NS>::ct(cv, FreeImpl<double, NS>::split(*this))); }
+        else { ASB_FREE_SWITCH(Ns, c = FreeImpl<float, NS>::ct(cv, FreeImpl<float, NS>::split(*this))); }
     } else {
         if (dbl) { ASB_SIZE_SWITCH(Ns, c = PeriodicImpl<double, NS>::ct(cv)); }
         else { ASB_SIZE_SWITCH(Ns, c = PeriodicImpl<float, NS>::ct(cv)); }
@@ -756,8 +784,8 @@ double Operator::autotune(bool dbl, int reps, int& best_rv, int& best_cv) {
 size_t Operator::spectrum_bytes(bool dbl) const {
     size_t n = 0;
     if (kind == OP_FFT) {
-        if (dbl) { ASB_SIZE_SWITCH(Ns, n = FreeImpl<double, NS>::spec_elems(FreeImpl<double, NS>::split(*this)) * sizeof(double2)); }
-        else { ASB_SIZE_SWITCH(Ns, n = FreeImpl<float, NS>::spec_elems(FreeImpl<float, NS>::split(*this)) * sizeof(float2)); }
+        if (dbl) { ASB_FREE_SWITCH(Ns, n = FreeImpl<double, NS>::spec_elems(FreeImpl<double, NS>::split(*this)) * sizeof(double2)); }
+        else { ASB_FREE_SWITCH(Ns, n = FreeImpl<float, NS>::spec_elems(FreeImpl<float, NS>::split(*this)) * sizeof(float2)); }
     } else {
         if (dbl) { ASB_SIZE_SWITCH(Ns, n = PeriodicImpl<double, NS>::spec_elems() * sizeof(double2)); }
         else { ASB_SIZE_SWITCH(Ns, n = PeriodicImpl<float, NS>::spec_elems() * sizeof(float2)); }
@@ -795,8 +823,8 @@ size_t Operator::resident_bytes() const {
 bool Operator::supports(bool dbl) const {
     bool ok = true;
     if (kind == OP_FFT) {
-        if (dbl) { ASB_SIZE_SWITCH(Ns, ok = FreeImpl<double, NS>::kSupported); }
-        else { ASB_SIZE_SWITCH(Ns, ok = FreeImpl<float, NS>::kSupported); }
+        if (dbl) { ASB_FREE_SWITCH(Ns, ok = FreeImpl<double, NS>::kSupported); }
+        else { ASB_FREE_SWITCH(Ns, ok = FreeImpl<float, NS>::kSupported); }
     } else {
         if (dbl) { ASB_SIZE_SWITCH(Ns, ok = PeriodicImpl<double, NS>::kSupported); }
         else { ASB_SIZE_SWITCH(Ns, ok = PeriodicImpl<float, NS>::kSupported); }
@@ -867,7 +895,7 @@ void Operator::ensure_precond_spectrum() {
         ASB_CUDA(cudaMalloc(&tab, (size_t)Ns * Ns * sizeof(double)));
         periodic_kernel_table(Nl, Ns, 0.0, tab, 1);
         ASB_CUDA(cudaMalloc(&khp_canon, nk * sizeof(double)));
-        ASB_SIZE_SWITCH(Ns, (void)KhBuild<NS>::build(*this, tab, khp_canon));
+        ASB_FREE_SWITCH(Ns, (void)KhBuild<NS>::build(*this, tab, khp_canon));
         if (supports(true)) {
             ASB_CUDA(cudaMalloc(&khp_d, nt * sizeof(double)));
             ASB_CUDA(cudaMemset(khp_d, 0, nt * sizeof(double)));

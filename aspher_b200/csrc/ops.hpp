@@ -45,7 +45,9 @@ struct SolverCtxBase {
 
 // exp(-2 pi i k / L), k < L, for every power of two L <= kMaxTw, on the
 // current device; tw_f(L)/tw_d(L) return the length-L table.
+// Likewise for L = 3 2^j <= kMaxTw3.
 constexpr int kMaxTw = 32768;
+constexpr int kMaxTw3 = 6144;
 const void* tw_table(bool dbl, int L);
 template <typename T> inline const typename std::conditional<sizeof(T) == 4, float2, double2>::type*
 tw(int L) {
@@ -67,6 +69,16 @@ constexpr int kMaxNs = 16384;
 constexpr int kMaxVariantNs = 8192;
 
 bool is_pow2(long v);
+
+// The compute side of an embedded grid of side Nl whose next power of two (at
+// least 16) is nc: 3/4 of nc where the block fits it and it lies in
+// [kMinTripleNs, largest], else nc.  Its transforms have radix-24 and radix-8
+// stages, less efficient than the 16s and 32s of a power of two: an apply at
+// 768 / 1536 / 3072 against the next power of two took FP32 18.6 / 52.5 / 257
+// us against 20.5 / 66.8 / 312, FP64 28.1 / 108 / 510 against 36.5 / 150 /
+// 700; at 384 FP32 10.3 against 8.9, so the line lies at 768.
+constexpr int kMinTripleNs = 768, kMaxTripleNs = 3072;
+int embed_side(int Nl, int nc, int largest);
 
 // launch variants chosen for (kind, precision, Ns): the autotuned entry of
 // this process if any, else the built-in default
@@ -93,7 +105,8 @@ void scratch_trim();
 void smem_optin(const void* func, int bytes);
 
 struct Operator {
-    // the compute grid: a power of two in [16, 16384] and the pipeline
+    // the compute grid: a power of two in [16, 16384] (embedded: or 768, 1536,
+    // 3072) and the pipeline
     // (free-space padded or periodic) that every kernel of this library sees
     int kind = OP_FFT;
     int Ns = 0;
@@ -101,7 +114,7 @@ struct Operator {
     // the caller's grid side and backend.  Equal to Ns / kind unless the
     // caller's side is not a power of two in [16, 16384]: the operator then
     // runs EMBEDDED, its Nl x Nl cells the top-left block of an Ns x Ns
-    // free-space pipeline (Ns the next power of two, at least 16) whose
+    // free-space pipeline (Ns = embed_side) whose
     // kernel table holds the caller's operator at every offset |d| < Nl:
     // the Love table at the caller's cell size (backend fft: the padded
     // convolution of the block is the free-space operator of the Nl grid),
@@ -110,7 +123,7 @@ struct Operator {
     // convolution with that kernel over offsets |d| < Nl)
     int Nl = 0;
     int backend = OP_FFT;
-    bool embedded() const { return Nl != Ns || backend != kind; }
+    bool embedded() const { return Nl != Ns || backend != kind || !is_pow2(Ns); }
     // caller-facing apply: x, y hold Nl*Nl values
     void apply_caller(bool dbl, const void* x, void* y, cudaStream_t s);
     // embedded grids (even Nl) with the full-grid |k| preconditioner: the

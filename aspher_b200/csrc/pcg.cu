@@ -402,6 +402,10 @@ __host__ __device__ constexpr int disc_half(int R, int dy) {
 //   G = sum_C zf g,  G_pr = sum_C zf Real(g - gp),  gg = sum_C g^2,
 // from sums linear in zm (zm is this pass's own reduction):
 //   G = sum_C z g - zm sum_C g,  G_pr = sum_C z (g - gp) - zm sum_C (g - gp).
+// B200, per launch in the solve loop at the benchmark's contacts (1-20 % of
+// the cells), dense before / listed words after: FP32 Ns = 2048 26.5 / 16.8 us,
+// 1024 14.0 / 9.7; FP64 2048 28.4 / 19.0, 1024 14.6 / 10.6, 512 11.1 / 8.7,
+// 128 10.6 / 7.7.
 constexpr int kStMaxWords = 16;  // words per thread of the largest tile (16, 4 or 1)
 template <typename T, int R, bool LAZY, bool DOTS, bool FULL>
 __global__ void __launch_bounds__(256, 2) k_stencil(const PkParams* __restrict__ Pp, PkState* st,
@@ -449,8 +453,8 @@ __global__ void __launch_bounds__(256, 2) k_stencil(const PkParams* __restrict__
         return zT;
     };
     const long n4 = (FULL ? P.N : P.Nv) / 4;
-    const int lg = 31 - __clz(Ns), lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int tile = 256 * words;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int tile = 256 * words, lg = 31 - __clz(Ns);
     for (long base = (long)blockIdx.x * tile; base < n4; base += (long)gridDim.x * tile) {
         // the tile's words with contact, in order: thread t holds words
         // base + t * words ...
@@ -466,7 +470,7 @@ __global__ void __launch_bounds__(256, 2) k_stencil(const PkParams* __restrict__
                 st4(z, w0 + k, zero);
             }
         };
-        if (words >= 4) {  // n4 is a multiple of 4 (Ns of 16)
+        if (words >= 4) {  // such grids: n4 is a multiple of 4 (Ns of 64)
             for (int k = 0; k < words && w0 + k < n4; k += 4) {
                 const uint4 q = *reinterpret_cast<const uint4*>(mask + 4 * (w0 + k));
                 scan(k, q.x);
@@ -498,7 +502,8 @@ __global__ void __launch_bounds__(256, 2) k_stencil(const PkParams* __restrict__
         for (int e = threadIdx.x; e < total; e += 256) {
             const long i4 = base + list[e];
             const uint32_t mc = ldm4w(mask, i4);
-            const int y = (int)(i4 >> (lg - 2)), x0 = (int)(4 * i4) & (Ns - 1);
+            const int y = FULL ? (int)(i4 >> (lg - 2)) : (int)((unsigned)(4 * i4) / (unsigned)Ns);
+            const int x0 = (int)(4 * i4 - (long)y * Ns);
             T zo[4] = {T(0), T(0), T(0), T(0)};
             if constexpr (FULL) {
                 const int msk = Ns - 1;
@@ -611,7 +616,7 @@ template <typename T, bool LAZY, bool DOTS>
 void launch_stencil(int R, int Ns, int Nl, int B, cudaStream_t s, const PkParams* Pp, PkState* st,
                     const StencilW& W, const T* ga, const T* gb, const uint8_t* mask, T* z,
                     double* part, int gated) {
-    const bool full = Nl == Ns;
+    const bool full = Nl == Ns && is_pow2(Ns);
     // the largest tile that still leaves a CTA for every other SM (of the
     // rows that hold data)
     const long n4 = (long)Nl * Ns / 4;

@@ -65,7 +65,6 @@ __global__ void k_cerruti_tables(double* __restrict__ xx, double* __restrict__ x
 // the sign of an odd-in-each-axis table restored from the offsets' signs
 struct LoadEmbeddedSigned {
     static constexpr bool kTiled = false;
-    static constexpr bool kRaw = false;
     const double* tab;
     int Ns, M;
     int odd;
@@ -146,7 +145,9 @@ template <typename T>
 __host__ __device__ constexpr int tan_ct(int LC, int Ns) {
     const int tt = LC / col_rpt<T>(LC, 0);
     int ct = 16;
-    while (ct > 1 && (2 * ct * tt > 512 || ct > Ns || col_smem<T>(LC, 2 * ct) > kSmemPerSM))
+    // (3 2^k FP64: 24 points per thread take more than 128 registers)
+    const int most = LC % 3 == 0 && sizeof(T) == 8 ? 256 : 512;
+    while (ct > 1 && (2 * ct * tt > most || ct > Ns || col_smem<T>(LC, 2 * ct) > kSmemPerSM))
         ct >>= 1;
     return ct;
 }
@@ -158,14 +159,11 @@ __host__ __device__ constexpr bool col_pair_pp(int LC, int CT) {
 }
 
 // Row-pass launch variant of the tangential apply (its rows are the free-
-// space operator's zero-padded transforms, two fields as gridDim.y = 2),
-// measured on B200 with the column-pair kernel: FP32 the free-space
-// defaults (2048: 0.220 -> 0.210 ms per apply against variant 0, 256: 0.028
-// -> 0.024 ms); FP64 variant 1 up to 512, else 0 (variant 2, the free-space
-// default at 2048, took the two-field apply from 0.396 to 0.441 ms)
+// space operator's zero-padded transforms, two fields as gridDim.y = 2): the
+// free-space operator's choice at these sizes
 template <typename T>
 __host__ __device__ constexpr int tan_row_variant(int Ns) {
-    return vclamp(Ns, sizeof(T) == 4 ? (Ns <= 512 ? 2 : 1) : (Ns <= 512 ? 1 : 0));
+    return vclamp(Ns, Ns <= 256 ? 3 : (Ns <= 512 || Ns % 3 == 0 ? 2 : 1));
 }
 
 template <typename T>
@@ -257,7 +255,7 @@ struct TanOperator {
     // tangential operator of the Nl grid on the block
     int Ns = 0, Nl = 0;
     double L = 1.0, E = 1.0, nu = 0.3;
-    bool embedded() const { return Nl != Ns; }
+    bool embedded() const { return Nl != Ns || !is_pow2(Ns); }
     // caller-facing apply: q, u hold 2 Nl^2 values
     void apply_caller(bool dbl, const void* q, void* u, cudaStream_t s);
     int device = 0;
@@ -356,6 +354,8 @@ void TanOperator::build() {
 #define ASB_TAN_SIZE_SWITCH(NSV, ...)                                       \
     switch (NSV) {                                                          \
         case 16: { constexpr int NS = 16; __VA_ARGS__; } break;             \
+        case 768: { constexpr int NS = 768; __VA_ARGS__; } break;           \
+        case 1536: { constexpr int NS = 1536; __VA_ARGS__; } break;         \
         case 32: { constexpr int NS = 32; __VA_ARGS__; } break;             \
         case 64: { constexpr int NS = 64; __VA_ARGS__; } break;             \
         case 128: { constexpr int NS = 128; __VA_ARGS__; } break;           \
@@ -371,10 +371,10 @@ TanOperator::TanOperator(int Ns_, double L_, double E_, double nu_)
     : Ns(Ns_), Nl(Ns_), L(L_), E(E_), nu(nu_) {
     if (Nl < 2 || Nl > kTanMaxNs)
         throw Error(ASPHER_EINVAL, "tangential operator: grid_size must be in [2, 2048]");
-    if (!is_pow2(Nl) || Nl < 16) {  // embedded in the next power of two
+    if (!is_pow2(Nl) || Nl < 16) {  // embedded
         int nc = 16;
         while (nc < Nl) nc *= 2;
-        Ns = nc;
+        Ns = embed_side(Nl, nc, kTanMaxNs);
     }
     if (!(L > 0.0) || !std::isfinite(L)) throw Error(ASPHER_EINVAL, "domain_size must be positive");
     if (!(E > 0.0) || !std::isfinite(E)) throw Error(ASPHER_EINVAL, "E_star must be positive");

@@ -262,3 +262,47 @@ def test_embedded_apply_leaves_nothing_behind(backend, Ns):
         assert torch.equal(op.matvec_(x, torch.empty_like(x)), want)
         asb.solve_device_mixed(op, torch.as_tensor(_gap(Ns), device="cuda"), 0.01, tol=1e-6)
         assert torch.equal(op.matvec_(x, torch.empty_like(x)), want)
+
+
+@pytest.mark.parametrize("Ns", [513, 768, 1025, 1536])
+def test_compute_sides_of_three_times_a_power_of_two(Ns):
+    """Grids that fit 768, 1536 or 3072 run there instead of on the next power
+    of two (radix-24 first stages): the applies equal the restatement, to
+    1e-12 / 2e-6."""
+    import aspher_b200 as asb
+    op = asb.Operator("fft", Ns)
+    x = np.random.default_rng(Ns).standard_normal(Ns * Ns)
+    want = OSolver(Ns, backend="fft").matvec(x)
+    xd = torch.as_tensor(x, device="cuda")
+    assert _rel(op.matvec_(xd, torch.empty_like(xd)).cpu().numpy(), want) <= 1e-12
+    xf = xd.float()
+    assert _rel(op.matvec_(xf, torch.empty_like(xf)).double().cpu().numpy(), want) <= 2e-6
+
+
+@pytest.mark.parametrize("Ns", [2051, 3072])
+def test_largest_three_times_a_power_of_two(Ns):
+    """The response to a point load is the Love table around it."""
+    import aspher_b200 as asb
+    op = asb.Operator("fft", Ns)
+    tab = torch.as_tensor(op.love_table(), device="cuda").reshape(Ns, Ns)
+    for iy, ix in ((0, 0), (Ns - 1, Ns // 3)):
+        x = torch.zeros(Ns, Ns, dtype=torch.float64, device="cuda")
+        x[iy, ix] = 1.0
+        u = op.matvec_(x.reshape(-1), torch.empty(Ns * Ns, dtype=torch.float64, device="cuda"))
+        dy = (torch.arange(Ns, device="cuda") - iy).abs()
+        dx = (torch.arange(Ns, device="cuda") - ix).abs()
+        want = tab[dy][:, dx]
+        err = (u.reshape(Ns, Ns) - want).norm() / want.norm()
+        assert float(err) <= 1e-12
+
+
+@pytest.mark.parametrize("Ns", [520, 768, 1100])
+def test_tangential_three_times_a_power_of_two(Ns):
+    from oracle.tangential import CerrutiKernel, TangentialFFTOperator
+    from aspher_b200 import TangentialOperator
+    q = np.random.default_rng(Ns).standard_normal(2 * Ns * Ns)
+    want = TangentialFFTOperator(CerrutiKernel(Ns, 1.0, 1.0, 0.3)).matvec(q)
+    op = TangentialOperator(Ns)
+    assert _rel(op.matvec(q), want) <= 1e-12
+    qf = torch.as_tensor(q, dtype=torch.float32, device="cuda")
+    assert _rel(op.matvec_(qf, torch.empty_like(qf)).double().cpu().numpy(), want) <= 2e-6

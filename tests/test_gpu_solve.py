@@ -247,7 +247,8 @@ def test_eager_loop_matches_graph_loop(dtype):
 
 
 @pytest.mark.parametrize("backend,Ns", [("fft", 16), ("fft", 64), ("periodic", 128), ("fft", 48),
-                                        ("periodic", 75), ("fft", 512)])
+                                        ("periodic", 75), ("fft", 512), ("periodic", 600),
+                                        ("fft", 768)])
 @pytest.mark.parametrize("precond", ["none", "fourier"])
 def test_sparse_passes_keep_the_minimiser(backend, Ns, precond):
     """The vector passes touch a field only where the contact mask (or a
@@ -272,3 +273,11 @@ def test_sparse_passes_keep_the_minimiser(backend, Ns, precond):
         err = np.linalg.norm(r.pressure - cold.pressure) / np.linalg.norm(cold.pressure)
         assert err <= 20 * np.sqrt(tol), err  # two certified points: |dp|_S^2 <= 2 tol P g_ref
         assert abs(r.contact_area - cold.contact_area) <= 1e-3
+        # the certificate once more, from an apply of its own
+        p = np.asarray(r.pressure).ravel()
+        v = s.matvec(p) + g
+        on = p > 0
+        ref, total = g.max() - g.min(), p.sum()
+        v -= v[on].mean()
+        assert (p * (v - v.min())).sum() <= 2 * tol * total * ref
+        assert -v.min() <= 2 * tol * ref and abs(total / (load * Ns * Ns) - 1) <= 1e-10

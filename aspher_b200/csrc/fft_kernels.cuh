@@ -213,6 +213,27 @@ __host__ __device__ constexpr int col_smem_total() {
                : col_smem<T>(LC, col_ct_v<T>(LC, NCM1, V));
 }
 
+// A load or store with kBatch moves all of a thread's pairs in one call
+// (all<count, TT>(row, t, v): pairs t + m TT, m < count) after a begin() that
+// reads its scalars: the steps of the PK iteration (pk_device.cuh).
+template <class F, class = void>
+struct is_batch : std::false_type {};
+template <class F>
+struct is_batch<F, std::enable_if_t<F::kBatch>> : std::true_type {};
+
+// CTAs per SM of an inverse row pass with store F: with a step of the PK
+// iteration an FP32 pass gets 80 registers (FP64 fields: 128) instead of 64,
+// where it spilled 28-220 bytes
+template <typename T, class F>
+__host__ __device__ constexpr int row_minb_f(int LR, int v) {
+    int mb = row_minb<T>(LR, v);
+    if constexpr (is_batch<F>::value) {
+        constexpr int regs = sizeof(typename F::Real) == 8 ? 128 : 80;
+        while (mb > 1 && mb * row_threads<T>(LR, v) * regs > 65536) --mb;
+    }
+    return mb;
+}
+
 // ---- row forward ---------------------------------------------------------------
 // Load:  cplx<T> operator()(int row, int n) -> z[n] = (x[2n], x[2n+1]);
 // Store: void operator()(int row, int k, cplx<T> X), k in [0, LR]
@@ -231,7 +252,7 @@ __host__ __device__ constexpr int col_smem_total() {
 // one shared pass in seven.  Per launch on B200, before / after: FP32 Ns =
 // 2048 18.3 / 15.9 us, 1024 6.2 / 5.2, FP64 2048 41.9 / 33.6, 4096 197 / 170.
 template <typename T, int LR, bool PAD, int V, class Load, class Store>
-__global__ void __launch_bounds__(row_threads<T>(LR, V), (row_minb<T>(LR, V)))
+__global__ void __launch_bounds__(row_threads<T>(LR, V), row_minb<T>(LR, V))
 row_fwd_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
                const cplx<T>* __restrict__ tw_2lr, const int* __restrict__ gate) {
     pdl_wait();
@@ -245,10 +266,17 @@ row_fwd_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
     const int row = blockIdx.x * RB + r;
     const bool valid = row < nrows;
     cplx<T> v[RPT];
+    if constexpr (is_batch<Load>::value) {
 #pragma unroll
-    for (int m = 0; m < RPT; ++m) {
-        if (PAD && m >= RPT / 2) v[m] = mk<T>(0, 0);
-        else v[m] = valid ? ld(row, t + m * TT) : mk<T>(0, 0);
+        for (int m = 0; m < RPT; ++m) v[m] = mk<T>(0, 0);
+        ld.begin();
+        if (valid) ld.template all<(PAD && RPT > 1 ? RPT / 2 : RPT), TT>(row, t, v);
+    } else {
+#pragma unroll
+        for (int m = 0; m < RPT; ++m) {
+            if (PAD && m >= RPT / 2) v[m] = mk<T>(0, 0);
+            else v[m] = valid ? ld(row, t + m * TT) : mk<T>(0, 0);
+        }
     }
     block_fft<T, LR, RPT, -1, RB, PAD>(v, t, sm, r, tw_lr);
 #pragma unroll
@@ -306,7 +334,7 @@ row_fwd_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
 // loaded it through shared memory.  Per launch on B200, before / after: FP32
 // Ns = 2048 17.9 / 16.6 us, FP64 2048 42.6 / 35.6, 4096 197 / 187.
 template <typename T, int LR, bool PAD, int V, class Load, class Store>
-__global__ void __launch_bounds__(row_threads<T>(LR, V), row_minb<T>(LR, V))
+__global__ void __launch_bounds__(row_threads<T>(LR, V), (row_minb_f<T, Store>(LR, V)))
 row_inv_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
                const cplx<T>* __restrict__ tw_2lr, const int* __restrict__ gate) {
     pdl_wait();
@@ -319,6 +347,7 @@ row_inv_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
     const int r = threadIdx.x % RB, t = threadIdx.x / RB;
     const int row = blockIdx.x * RB + r;
     const bool valid = row < nrows;
+    if constexpr (is_batch<Store>::value) st.begin();
     cplx<T> v[RPT];
     {
         const int ct = ld.ct, lct = __ffs(ct) - 1;  // ct is a power of two
@@ -352,10 +381,14 @@ row_inv_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
     }
     __syncthreads();
     block_fft<T, LR, RPT, +1, RB>(v, t, sm, r, tw_lr);
+    if constexpr (is_batch<Store>::value) {
+        if (valid) st.template all<(PAD && RPT > 1 ? RPT / 2 : RPT), TT>(row, t, v);
+    } else {
 #pragma unroll
-    for (int m = 0; m < RPT; ++m) {
-        if (PAD && m >= RPT / 2) continue;
-        if (valid) st(row, t + m * TT, v[m]);
+        for (int m = 0; m < RPT; ++m) {
+            if (PAD && m >= RPT / 2) continue;
+            if (valid) st(row, t + m * TT, v[m]);
+        }
     }
     if constexpr (Store::kFinish) {
         __syncthreads();

@@ -5,8 +5,8 @@ namespace asb {
 
 template <>
 void free_matvec<float>(const Operator& op, const float* x, float* y, cplx<float>* spec, cudaStream_t s,
-                    const int* gate, int B, const PkState* sc) {
-    ASB_FREE_SWITCH(op.Ns, (FreeImpl<float, NS>::matvec(op, x, y, spec, s, gate, B, sc)));
+                    const int* gate, int B) {
+    ASB_FREE_SWITCH(op.Ns, (FreeImpl<float, NS>::matvec(op, x, y, spec, s, gate, B)));
 }
 
 template <>
@@ -23,9 +23,25 @@ void embedded_precond<float>(Operator& op, const float* ga, const float* gb, con
                                                             spec)));
 }
 
-void free_defect(const Operator& op, LoadDiffRows ld, StoreAddRows st, float2* spec,
-                 cudaStream_t s, const int* gate, int B) {
-    ASB_FREE_SWITCH(op.Ns, (FreeImpl<float, NS>::apply(op, ld, st, spec, s, gate, B)));
+template <>
+void free_pk_eval<float, float>(const Operator& op, const PkFields<float>& f, cplx<float>* spec, cudaStream_t s,
+        int B) {
+    ASB_FREE_SWITCH(op.Ns, (pk_eval_apply<FreeImpl<float, NS>, float, float>(op, f, spec, s, B)));
+}
+template <>
+void free_pk_line<float, float>(const Operator& op, const PkFields<float>& f, cplx<float>* spec, cudaStream_t s,
+        int B) {
+    ASB_FREE_SWITCH(op.Ns, (pk_line_apply<FreeImpl<float, NS>, float, float>(op, f, spec, s, B)));
+}
+template <>
+void free_pk_eval<double, float>(const Operator& op, const PkFields<double>& f, cplx<float>* spec, cudaStream_t s,
+        int B) {
+    ASB_FREE_SWITCH(op.Ns, (pk_eval_apply<FreeImpl<float, NS>, double, float>(op, f, spec, s, B)));
+}
+template <>
+void free_pk_line<double, float>(const Operator& op, const PkFields<double>& f, cplx<float>* spec, cudaStream_t s,
+        int B) {
+    ASB_FREE_SWITCH(op.Ns, (pk_line_apply<FreeImpl<float, NS>, double, float>(op, f, spec, s, B)));
 }
 
 }  // namespace asb

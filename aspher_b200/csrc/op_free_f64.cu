@@ -5,8 +5,8 @@ namespace asb {
 
 template <>
 void free_matvec<double>(const Operator& op, const double* x, double* y, cplx<double>* spec, cudaStream_t s,
-                    const int* gate, int B, const PkState* sc) {
-    ASB_FREE_SWITCH(op.Ns, (FreeImpl<double, NS>::matvec(op, x, y, spec, s, gate, B, sc)));
+                    const int* gate, int B) {
+    ASB_FREE_SWITCH(op.Ns, (FreeImpl<double, NS>::matvec(op, x, y, spec, s, gate, B)));
 }
 
 template <>
@@ -21,6 +21,17 @@ void embedded_precond<double>(Operator& op, const double* ga, const double* gb, 
                          double* part, cudaStream_t s, const int* gate, int B, void* spec) {
     ASB_FREE_SWITCH(op.Ns, (EmbeddedFourierImpl<double, NS>::run(op, ga, gb, mask, st, z, part, s, gate, B,
                                                             spec)));
+}
+
+template <>
+void free_pk_eval<double, double>(const Operator& op, const PkFields<double>& f, cplx<double>* spec, cudaStream_t s,
+        int B) {
+    ASB_FREE_SWITCH(op.Ns, (pk_eval_apply<FreeImpl<double, NS>, double, double>(op, f, spec, s, B)));
+}
+template <>
+void free_pk_line<double, double>(const Operator& op, const PkFields<double>& f, cplx<double>* spec, cudaStream_t s,
+        int B) {
+    ASB_FREE_SWITCH(op.Ns, (pk_line_apply<FreeImpl<double, NS>, double, double>(op, f, spec, s, B)));
 }
 
 }  // namespace asb

@@ -9,6 +9,7 @@
 #include "fft_launch.cuh"
 #include "functors.cuh"
 #include "ops.hpp"
+#include "pk_device.cuh"
 #include "reduce.cuh"
 
 namespace asb {
@@ -166,9 +167,17 @@ struct FreeImpl {
     }
 
     static void matvec(const Operator& op, const T* x, T* y, cplx<T>* spec, cudaStream_t s,
-                       const int* gate, int B, const PkState* sc) {
+                       const int* gate, int B) {
         const long bx = (long)NS * NS;
-        apply(op, LoadRealRows<T>{x, NS, bx, sc}, StoreRealRows<T>{y, NS, bx}, spec, s, gate, B);
+        apply(op, LoadRealRows<T>{x, NS, bx}, StoreRealRows<T>{y, NS, bx}, spec, s, gate, B);
+    }
+
+    // an apply with a step of the PK iteration in its store (and load)
+    template <class Load, class Store>
+    static void pk(const Operator& op, Load ld, Store st, cplx<T>* spec, cudaStream_t s,
+                   const int* gate, int B) {
+        if constexpr (is_batch<Load>::value) apply<kRV>(op, ld, st, spec, s, gate, B);
+        else apply<-1, kRV>(op, ld, st, spec, s, gate, B);
     }
 
     // an embedded operator's apply on the caller's own layout, at this
@@ -179,6 +188,29 @@ struct FreeImpl {
                   nullptr, 1);
     }
 };
+
+// The two applies of a PK iteration on the impl's operator: evaluate() in the
+// row store of the p apply (row variant of the operator for its plain load),
+// the direction update and the line-search sums in the row load and store of
+// the t apply.  F: the solver's precision, T: the transform's.
+template <class Impl, typename F, typename T>
+void pk_eval_apply(const Operator& op, const PkFields<F>& f, cplx<T>* spec, cudaStream_t s, int B) {
+    const int Ns = op.Ns;
+    const long bx = (long)Ns * Ns;
+    const StoreEval<F, T> st{f.P, f.st, f.u0, f.g0, f.p, f.ga, f.gb, f.mask, f.part, Ns, bx};
+    if constexpr (sizeof(F) != sizeof(T))
+        Impl::pk(op, LoadDiffRows{f.p, f.p0, Ns, bx, f.st}, st, spec, s, &f.st->halt, B);
+    else
+        Impl::pk(op, LoadRealRows<T>{f.p, Ns, bx, f.st}, st, spec, s, &f.st->halt, B);
+}
+template <class Impl, typename F, typename T>
+void pk_line_apply(const Operator& op, const PkFields<F>& f, cplx<T>* spec, cudaStream_t s, int B) {
+    const int Ns = op.Ns;
+    const long bx = (long)Ns * Ns;
+    Impl::pk(op, LoadDirection<F, T>{f.P, f.st, f.z, f.ga, f.gb, f.t, f.mask, Ns, bx},
+             StoreLineSums<F, T>{f.st, f.ga, f.gb, f.t, f.mask, f.part, Ns, bx}, spec, s,
+             &f.st->halt, B);
+}
 
 template <typename T, int NS>
 struct PeriodicImpl {
@@ -228,11 +260,19 @@ struct PeriodicImpl {
     }
 
     static void matvec(const Operator& op, const T* x, T* y, cplx<T>* spec, cudaStream_t s,
-                       const int* gate, int B, const PkState* sc) {
+                       const int* gate, int B) {
         const int dbl = sizeof(T) == 8;
         const long bx = (long)NS * NS;
-        apply(op.rowv[dbl], op.colv[dbl], LoadRealRows<T>{x, NS, bx, sc}, mult(op),
+        apply(op.rowv[dbl], op.colv[dbl], LoadRealRows<T>{x, NS, bx}, mult(op),
               StoreRealRows<T>{y, NS, bx}, spec, s, gate, B);
+    }
+
+    template <class Load, class Store>
+    static void pk(const Operator& op, Load ld, Store st, cplx<T>* spec, cudaStream_t s,
+                   const int* gate, int B) {
+        const int dbl = sizeof(T) == 8, rv = op.rowv[dbl], cv = op.colv[dbl];
+        if constexpr (is_batch<Load>::value) apply<kRV>(rv, cv, ld, mult(op), st, spec, s, gate, B);
+        else apply<-1, kRV>(rv, cv, ld, mult(op), st, spec, s, gate, B);
     }
 };
 
@@ -368,22 +408,29 @@ struct EmbeddedFourierImpl {
     }
 
 // what op_free_*.cu and op_periodic_*.cu define for their pipeline and T
+// (F: the solver's precision of a PK step)
+template <typename F, typename T>
+void free_pk_eval(const Operator& op, const PkFields<F>& f, cplx<T>* spec, cudaStream_t s, int B);
+template <typename F, typename T>
+void free_pk_line(const Operator& op, const PkFields<F>& f, cplx<T>* spec, cudaStream_t s, int B);
+template <typename F, typename T>
+void periodic_pk_eval(const Operator& op, const PkFields<F>& f, cplx<T>* spec, cudaStream_t s,
+                      int B);
+template <typename F, typename T>
+void periodic_pk_line(const Operator& op, const PkFields<F>& f, cplx<T>* spec, cudaStream_t s,
+                      int B);
 template <typename T>
 void free_matvec(const Operator& op, const T* x, T* y, cplx<T>* spec, cudaStream_t s,
-                 const int* gate, int B, const PkState* sc);
+                 const int* gate, int B);
 template <typename T>
 void free_apply_block(const Operator& op, const T* x, T* y, cplx<T>* spec, cudaStream_t s);
-void free_defect(const Operator& op, LoadDiffRows ld, StoreAddRows st, float2* spec,
-                 cudaStream_t s, const int* gate, int B);
 template <typename T>
 void embedded_precond(Operator& op, const T* ga, const T* gb, const uint8_t* mask, PkState* st,
                         T* z,
                       double* part, cudaStream_t s, const int* gate, int B, void* spec);
 template <typename T>
 void periodic_matvec(const Operator& op, const T* x, T* y, cplx<T>* spec, cudaStream_t s,
-                     const int* gate, int B, const PkState* sc);
-void periodic_defect(const Operator& op, LoadDiffRows ld, StoreAddRows st, float2* spec,
-                     cudaStream_t s, const int* gate, int B);
+                     const int* gate, int B);
 template <typename T>
 void periodic_precond(Operator& op, const T* ga, const T* gb, const uint8_t* mask, PkState* st,
                         T* z,

@@ -6,8 +6,8 @@ namespace asb {
 
 template <>
 void periodic_matvec<float>(const Operator& op, const float* x, float* y, cplx<float>* spec, cudaStream_t s,
-                        const int* gate, int B, const PkState* sc) {
-    ASB_SIZE_SWITCH(op.Ns, (PeriodicImpl<float, NS>::matvec(op, x, y, spec, s, gate, B, sc)));
+                        const int* gate, int B) {
+    ASB_SIZE_SWITCH(op.Ns, (PeriodicImpl<float, NS>::matvec(op, x, y, spec, s, gate, B)));
 }
 
 template <>
@@ -17,11 +17,25 @@ void periodic_precond<float>(Operator& op, const float* ga, const float* gb, con
     ASB_SIZE_SWITCH(op.Ns, (FourierImpl<float, NS>::run(op, ga, gb, mask, st, z, part, s, gate, B, spec)));
 }
 
-void periodic_defect(const Operator& op, LoadDiffRows ld, StoreAddRows st, float2* spec,
-                     cudaStream_t s, const int* gate, int B) {
-    ASB_SIZE_SWITCH(op.Ns, (PeriodicImpl<float, NS>::apply(
-                               op.rowv[0], op.colv[0], ld, PeriodicImpl<float, NS>::mult(op), st,
-                               spec, s, gate, B)));
+template <>
+void periodic_pk_eval<float, float>(const Operator& op, const PkFields<float>& f, cplx<float>* spec, cudaStream_t s,
+        int B) {
+    ASB_SIZE_SWITCH(op.Ns, (pk_eval_apply<PeriodicImpl<float, NS>, float, float>(op, f, spec, s, B)));
+}
+template <>
+void periodic_pk_line<float, float>(const Operator& op, const PkFields<float>& f, cplx<float>* spec, cudaStream_t s,
+        int B) {
+    ASB_SIZE_SWITCH(op.Ns, (pk_line_apply<PeriodicImpl<float, NS>, float, float>(op, f, spec, s, B)));
+}
+template <>
+void periodic_pk_eval<double, float>(const Operator& op, const PkFields<double>& f, cplx<float>* spec, cudaStream_t s,
+        int B) {
+    ASB_SIZE_SWITCH(op.Ns, (pk_eval_apply<PeriodicImpl<float, NS>, double, float>(op, f, spec, s, B)));
+}
+template <>
+void periodic_pk_line<double, float>(const Operator& op, const PkFields<double>& f, cplx<float>* spec, cudaStream_t s,
+        int B) {
+    ASB_SIZE_SWITCH(op.Ns, (pk_line_apply<PeriodicImpl<float, NS>, double, float>(op, f, spec, s, B)));
 }
 
 }  // namespace asb

@@ -6,8 +6,8 @@ namespace asb {
 
 template <>
 void periodic_matvec<double>(const Operator& op, const double* x, double* y, cplx<double>* spec, cudaStream_t s,
-                        const int* gate, int B, const PkState* sc) {
-    ASB_SIZE_SWITCH(op.Ns, (PeriodicImpl<double, NS>::matvec(op, x, y, spec, s, gate, B, sc)));
+                        const int* gate, int B) {
+    ASB_SIZE_SWITCH(op.Ns, (PeriodicImpl<double, NS>::matvec(op, x, y, spec, s, gate, B)));
 }
 
 template <>
@@ -15,6 +15,17 @@ void periodic_precond<double>(Operator& op, const double* ga, const double* gb, 
                         double* z,
                          double* part, cudaStream_t s, const int* gate, int B, void* spec) {
     ASB_SIZE_SWITCH(op.Ns, (FourierImpl<double, NS>::run(op, ga, gb, mask, st, z, part, s, gate, B, spec)));
+}
+
+template <>
+void periodic_pk_eval<double, double>(const Operator& op, const PkFields<double>& f, cplx<double>* spec, cudaStream_t s,
+        int B) {
+    ASB_SIZE_SWITCH(op.Ns, (pk_eval_apply<PeriodicImpl<double, NS>, double, double>(op, f, spec, s, B)));
+}
+template <>
+void periodic_pk_line<double, double>(const Operator& op, const PkFields<double>& f, cplx<double>* spec, cudaStream_t s,
+        int B) {
+    ASB_SIZE_SWITCH(op.Ns, (pk_line_apply<PeriodicImpl<double, NS>, double, double>(op, f, spec, s, B)));
 }
 
 }  // namespace asb

@@ -839,34 +839,21 @@ constexpr const char* kNoFp64Apply =
 }  // namespace
 
 void Operator::matvec(bool dbl, const void* x, void* y, cudaStream_t s, const int* gate, int B,
-                      void* spec_b, const PkState* sc) {
+                      void* spec_b) {
     if (!supports(dbl)) throw Error(-1, kNoFp64Apply);
     void* spec = spec_b ? spec_b : spectrum(dbl, s);
     if (kind == OP_FFT) {
         if (dbl)
-            free_matvec<double>(*this, (const double*)x, (double*)y, (double2*)spec, s, gate, B,
-                                sc);
+            free_matvec<double>(*this, (const double*)x, (double*)y, (double2*)spec, s, gate, B);
         else
-            free_matvec<float>(*this, (const float*)x, (float*)y, (float2*)spec, s, gate, B, sc);
+            free_matvec<float>(*this, (const float*)x, (float*)y, (float2*)spec, s, gate, B);
     } else {
         if (dbl)
             periodic_matvec<double>(*this, (const double*)x, (double*)y, (double2*)spec, s, gate,
-                                    B, sc);
+                                    B);
         else
-            periodic_matvec<float>(*this, (const float*)x, (float*)y, (float2*)spec, s, gate, B,
-                                   sc);
+            periodic_matvec<float>(*this, (const float*)x, (float*)y, (float2*)spec, s, gate, B);
     }
-}
-
-void Operator::matvec_defect(const double* x, const double* x0, double* y, const double* y0,
-                             cudaStream_t s, const int* gate, int B, void* spec_b,
-                             const PkState* sc) {
-    void* spec = spec_b ? spec_b : spectrum(false, s);
-    const long bx = (long)Ns * Ns;
-    const LoadDiffRows ld{x, x0, Ns, bx, sc};
-    const StoreAddRows st{y, y0, Ns, bx};
-    if (kind == OP_FFT) free_defect(*this, ld, st, (float2*)spec, s, gate, B);
-    else periodic_defect(*this, ld, st, (float2*)spec, s, gate, B);
 }
 
 void Operator::apply_caller(bool dbl, const void* x, void* y, cudaStream_t s) {
@@ -917,6 +904,32 @@ void Operator::ensure_precond_spectrum() {
         throw;
     }
     cudaFree(tab);
+}
+
+// the applies of a PK iteration (F: the solver's precision; FP64 fields with
+// a defect-corrected apply transform in FP32)
+namespace {
+template <typename F, typename T>
+void pk_step(Operator& op, const PkFields<F>& f, bool eval, void* spec_b, cudaStream_t s, int B) {
+    if (!op.supports(sizeof(T) == 8)) throw Error(-1, kNoFp64Apply);
+    cplx<T>* spec = static_cast<cplx<T>*>(spec_b ? spec_b : op.spectrum(sizeof(T) == 8, s));
+    if (op.kind == OP_FFT) {
+        if (eval) free_pk_eval<F, T>(op, f, spec, s, B);
+        else free_pk_line<F, T>(op, f, spec, s, B);
+    } else {
+        if (eval) periodic_pk_eval<F, T>(op, f, spec, s, B);
+        else periodic_pk_line<F, T>(op, f, spec, s, B);
+    }
+}
+}  // namespace
+void pk_apply(Operator& op, const PkFields<float>& f, bool eval, bool, void* spec, cudaStream_t s,
+              int B) {
+    pk_step<float, float>(op, f, eval, spec, s, B);
+}
+void pk_apply(Operator& op, const PkFields<double>& f, bool eval, bool defect, void* spec,
+              cudaStream_t s, int B) {
+    if (defect) pk_step<double, float>(op, f, eval, spec, s, B);
+    else pk_step<double, double>(op, f, eval, spec, s, B);
 }
 
 template <typename T>

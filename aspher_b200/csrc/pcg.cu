@@ -23,6 +23,7 @@
 #include "pk_state.hpp"
 #include "pcg.hpp"
 #include "embed.cuh"
+#include "pk_device.cuh"
 #include "reduce.cuh"
 
 #include <algorithm>
@@ -118,58 +119,11 @@ __device__ __forceinline__ const T* gap_before(const PkState* st, const T* ga, c
 #define GRID_LOOP4(N) \
     for (long i4 = blockIdx.x * (long)blockDim.x + threadIdx.x; i4 < (N) / 4; i4 += (long)gridDim.x * blockDim.x)
 
-
 // ---- evaluate() -----------------------------------------------------------------
-// The gap buffer holds v = u + (g0 - gshift) uncentred after k_eval; every
-// later consumer centres on the fly with gc(), which is bit-identical to the
-// reference's stored g = Real(v - Real(alpha)) (contact_solver.cpp:283-285),
-// so centring costs no pass of its own.
-template <typename T>
-__device__ __forceinline__ T gc(T v, T aT) { return v - aT; }
-
-__device__ __forceinline__ void set_halt(PkState* st, int h) {
-    st->halt = h;
-    st->skip_mv1 = 1;
-}
-
-// Scalar tail of the rsum / den pass (thread 0 of the last block).
-// acc = {sum_C r, sum_C g t, sum_C r t, sum_C t};
-// den = sum_C Real(r - rm) t, linear in rm: sum_C r t - rm sum_C t.
-template <typename T>
-__device__ inline void rden_tail(PkState* st, const double (&acc)[4]) {
-    st->mv++;
-    if (st->copy_best) {
-        st->copy_best = 0;
-        st->have_best = 1;
-    }
-    st->rsum = acc[0];
-    st->num = acc[1];
-    st->rmean = (double)(T)(st->nc ? acc[0] / st->nc : 0.0);
-    const double den = acc[2] - st->rmean * acc[3], num = acc[1];
-    st->den = den;
-    if (den > 0.0 && isfinite(den) && isfinite(num)) {
-        const T tau = (T)(num / den);
-        st->tau = (double)tau;
-        st->tau_ov = st->gg > 0.0 ? (double)(T)(num * num / (den * st->gg)) : (double)tau;
-    } else {
-        set_halt(st, H_IDENT);  // no usable direction: identification step
-    }
-}
-
-// The pending load rescale of an instance (PkState::scale / scale_add),
-// read once at kernel entry: the iterate is Real(x f) + a of the stored x
-// (bit-identical to the reference's p(i) *= f, where a = 0).
-template <typename T>
-struct PScale {
-    T f, a;
-    __device__ explicit PScale(const PkState* st) : f((T)st->scale), a((T)st->scale_add) {}
-    __device__ __forceinline__ T operator()(T x) const { return x * f + a; }
-};
-
-// One pass for evaluate() (contact_solver.cpp:263-303): v -> the gap buffer
-// that does not hold the last evaluation's (PkState::par), the contact mask,
-// and the sums whose last-block logic is the certificate, the convergence
-// test and the best/stall bookkeeping (contact_solver.cpp:379-412).
+// evaluate() (contact_solver.cpp:263-303) of the returned iterate: v -> the gap
+// buffer that does not hold the last evaluation's (PkState::par), the contact
+// mask, and the sums of the certificate.  The iterations' evaluate() runs in
+// the row store of the p apply (StoreEval): this pass keeps u as well.
 // The second-pass sums of the reference are linear in the centring, so they
 // come from first-pass sums:
 //   gcs = sum_C Real(v - a)            -> sum_C v - n_C a
@@ -184,8 +138,7 @@ struct PScale {
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_eval(const PkParams* __restrict__ Pp, PkState* st,
                                                       const T* u, const T* g0, const T* p, T* ga,
-                                                      T* gb, uint8_t* mask, double* part,
-                                                      int final_mode) {
+                                                      T* gb, uint8_t* mask, double* part) {
     pdl_wait();
     // instance blockIdx.y of a batched solve (0 when unbatched)
     Pp += blockIdx.y;
@@ -197,7 +150,6 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_eval(const PkPar
     p += bo_;
     mask += bo_;
     const PkParams& P = *Pp;
-    if (!final_mode && st->halt) return;
     T* g = (st->par ? ga : gb) + bo_;
     const bool stale = st->mask_stale != 0;
     const T gs = (T)P.gshift;
@@ -232,70 +184,8 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_eval(const PkPar
         if (stale || mn != mw) reinterpret_cast<uint32_t*>(mask)[i4] = mn;
     }
     const int kinds[5] = {0, 0, 1, 0, 0};
-    if (grid_reduce_last<5>(acc, kinds, part, &st->counter[0]) && threadIdx.x == 0) {
-        if (!final_mode) {
-            if (!st->u_fresh) st->mv++;
-            st->u_fresh = 0;
-            st->skip_mv1 = 0;
-            st->pk_due = 1;
-        }
-        const int nc = (int)acc[1];
-        const double alpha = nc ? acc[0] / nc : acc[2];
-        const double gmin = acc[2] - alpha;
-        const double aT = (double)(T)alpha, gmT = (double)(T)gmin;
-        const double gcs = acc[0] - (double)nc * aT;
-        st->nc = nc;
-        st->gsum = acc[0];
-        st->vmin = acc[2];
-        st->par ^= 1;
-        st->mask_stale = 0;
-        st->alpha_prev = st->alpha;
-        st->alpha = alpha;
-        st->gmin = gmin;
-        double ar = alpha, gr = gmin;
-        if (nc > 0) {  // refine_contact_mean (contact_solver.cpp:94-99)
-            const double d = gcs / nc;
-            ar += d;
-            gr -= d;
-        }
-        const double PG = P.P_total * P.g_ref;
-        const double G = acc[3] - (aT + gmT) * acc[4];
-        st->alpha_ref = ar;
-        st->gmin_ref = gr;
-        st->pv = acc[3];
-        st->gcs = gcs;
-        st->G = G;
-        st->fw = G / PG;
-        st->pen = fmax(0.0, -gr) / P.g_ref;
-        st->psum = acc[4];
-        st->load = fabs(acc[4] - P.P_total) / P.P_total;
-        st->finite = isfinite(acc[0]) && isfinite(acc[2]) && isfinite(acc[4]) && isfinite(acc[3]);
-        if (final_mode) return;
-        if (!st->finite) {
-            st->status = ST_NONFINITE;
-            set_halt(st, H_FINAL);
-            return;
-        }
-        if (st->load <= P.load_tol && st->fw <= P.tol && st->pen <= P.tol) {
-            st->status = ST_CONVERGED;
-            st->u_fresh = 1;
-            set_halt(st, H_FINAL);
-            return;
-        }
-        const double merit = fmax(st->fw, st->pen);
-        if (P.keep_best && merit < st->best_merit) {
-            st->best_merit = merit;
-            st->copy_best = 1;
-        }
-        if (merit < st->seen_merit * (1.0 - 1e-4)) {
-            st->seen_merit = merit;
-            st->stall = 0;
-        } else if (++st->stall >= P.stall_limit) {
-            set_halt(st, H_STALL);
-            return;
-        }
-        if (nc < 2) set_halt(st, H_IDENT);
-    }
+    if (grid_reduce_last<5>(acc, kinds, part, &st->counter[0]) && threadIdx.x == 0)
+        eval_tail<T>(P, st, acc, true);
 }
 
 // pk = sum p |g| / (P g_ref) (the reference's legacy error, reported and
@@ -690,92 +580,6 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_dots(const PkPar
     }
 }
 
-// Direction update t = chi_C(z_f + beta t) (and best = p when copy_best)
-// before the t apply; k_rden consumes r after it.  t is 0 off contact (k_pupd
-// clears the cells that leave it), so only groups with contact are touched.
-template <typename T>
-__global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_tupd(const PkParams* __restrict__ Pp, PkState* st, const T* z,
-                                                      const T* ga, const T* gb, T* t,
-                                                      const uint8_t* mask, const T* p, T* best) {
-    pdl_wait();
-    // instance blockIdx.y of a batched solve (0 when unbatched)
-    Pp += blockIdx.y;
-    st += blockIdx.y;
-    const long bo_ = (long)blockIdx.y * Pp->N;
-    z += bo_;
-    t += bo_;
-    mask += bo_;
-    p += bo_;
-    best += bo_;
-    const PkParams& P = *Pp;
-    if (st->halt) return;
-    const T* g = gap_now(st, ga, gb) + bo_;
-    const T zm = (T)st->zmean, beta = (T)st->beta, aT = (T)st->alpha;
-    const bool pre = P.precond != 0;
-    contact_groups(mask, P.Nv / 4, [&](long i4, uint32_t mw) {
-        T zz[4], gv[4], tt[4];
-        ldp4(t, i4, tt);
-        if (pre) ldp4(z, i4, zz);
-        else ldp4(g, i4, gv);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const T zf = pre ? (T)(zz[j] - zm) : gc(gv[j], aT);
-            tt[j] = mbyte(mw, j) ? (T)(zf + beta * tt[j]) : T(0);
-        }
-        st4(t, i4, tt);
-    });
-    if (st->copy_best) {
-        const PScale<T> ps(st);
-        GRID_LOOP4(P.Nv) {
-            T pp[4] = {T(0), T(0), T(0), T(0)};
-            if (ldm4w(mask, i4)) {
-                ldp4(p, i4, pp);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) pp[j] = ps(pp[j]);
-            }
-            st4(best, i4, pp);
-        }
-    }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_rden(const PkParams* __restrict__ Pp, PkState* st, const T* r,
-                                                      const T* ga, const T* gb, const T* t,
-                                                      const uint8_t* mask, double* part) {
-    pdl_wait();
-    // instance blockIdx.y of a batched solve (0 when unbatched)
-    Pp += blockIdx.y;
-    st += blockIdx.y;
-    part += (size_t)blockIdx.y * kPartStride;
-    const long bo_ = (long)blockIdx.y * Pp->N;
-    r += bo_;
-    t += bo_;
-    mask += bo_;
-    const PkParams& P = *Pp;
-    if (st->halt) return;
-    const T* g = gap_now(st, ga, gb) + bo_;
-    const T aT = (T)st->alpha;
-    double acc[4] = {0, 0, 0, 0};  // sum_C r, sum_C g t, sum_C r t, sum_C t
-    contact_groups(mask, P.Nv / 4, [&](long i4, uint32_t mw) {
-        T rr[4], gv[4], tt[4];
-        ldp4(r, i4, rr);
-        ldp4(g, i4, gv);
-        ldp4(t, i4, tt);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (!mbyte(mw, j)) continue;
-            const double td = (double)tt[j];
-            acc[0] += (double)rr[j];
-            acc[1] += (double)gc(gv[j], aT) * td;
-            acc[2] += (double)rr[j] * td;
-            acc[3] += td;
-        }
-    });
-    const int kinds[4] = {0, 0, 0, 0};
-    if (grid_reduce_last<4>(acc, kinds, part, &st->counter[4]) && threadIdx.x == 0)
-        rden_tail<T>(st, acc);
-}
-
 // Projected update of the pressure (contact_solver.cpp:464-501).  Off contact
 // p is 0 and changes only where the gap is negative, so a group without
 // either reads its mask word and its gap.  Keeps the mask (cells whose p is
@@ -786,7 +590,7 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_rden(const PkPar
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_pupd(const PkParams* __restrict__ Pp, PkState* st, T* p, T* t,
                                                       const T* ga, const T* gb, uint8_t* mask,
-                                                      double* part, int loop,
+                                                      T* best, double* part, int loop,
                                                       cudaGraphConditionalHandle cond, int n) {
     pdl_wait();
     // instance blockIdx.y of a batched solve (0 when unbatched)
@@ -797,6 +601,7 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_pupd(const PkPar
     p += bo_;
     t += bo_;
     mask += bo_;
+    best += bo_;
     const PkParams& P = *Pp;
     const bool end = loop && ((int)blockIdx.y == 0 || (int)blockIdx.y == n - 1);
     if (st->halt) {
@@ -808,6 +613,7 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_pupd(const PkPar
     // every block reads the pending rescale here, before it arrives at the
     // last-block counter; only the last block's tail rewrites it
     const PScale<T> ps(st);
+    const bool keep = st->copy_best != 0;  // the evaluated p is the best so far
     double acc[2] = {0, 0};  // changed (max), total
     GRID_LOOP4(P.Nv) {
         T pp[4] = {T(0), T(0), T(0), T(0)}, tt[4] = {T(0), T(0), T(0), T(0)}, gv[4];
@@ -819,10 +625,17 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_pupd(const PkPar
             gv[j] = gc(gv[j], aT);
             neg = neg || gv[j] < T(0);
         }
-        if (!mw && !neg) continue;
+        if (!mw && !neg && !keep) continue;
         if (mw) {
             ldp4(p, i4, pp);
             ldp4(t, i4, tt);
+        }
+        if (keep) {
+            T bb[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) bb[j] = mw ? ps(pp[j]) : T(0);
+            st4(best, i4, bb);
+            if (!mw && !neg) continue;
         }
         uint32_t mn = 0;
         bool left = false;
@@ -851,6 +664,10 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_pupd(const PkPar
     }
     const int kinds[2] = {2, 0};
     if (grid_reduce_last<2>(acc, kinds, part, &st->counter[6]) && threadIdx.x == 0) {
+        if (st->copy_best) {
+            st->copy_best = 0;
+            st->have_best = 1;
+        }
         st->delta = acc[0] > 0.0 ? 0.0 : 1.0;
         st->total = acc[1];
         // the load rescale (contact_solver.cpp:489-500), pending until the
@@ -863,7 +680,7 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_pupd(const PkPar
             st->scale = 1.0;
             st->scale_add = 0.0;
             st->fill = 2;
-            set_halt(st, H_FILL);
+            st->halt = H_FILL;
         } else {  // every p is 0: p = p_bar
             st->scale = 1.0;
             st->scale_add = (double)(T)P.p_bar;
@@ -871,7 +688,7 @@ __global__ void __launch_bounds__(kRedThreads, kRedMinBlocks) k_pupd(const PkPar
             st->mask_stale = 1;
         }
         st->it++;
-        if (st->it >= P.max_iter) set_halt(st, H_FINAL);  // status stays max_iterations
+        if (st->it >= P.max_iter) st->halt = H_FINAL;  // status stays max_iterations
         if (end && st->halt) cudaGraphSetConditional(cond, 0u);
     }
 }
@@ -1099,8 +916,8 @@ int red_grid(long N) {
 }
 
 // The FP64 polish stage of a mixed solve runs its loop applies
-// defect-corrected (Operator::matvec_defect: FP32 transforms of p - p0 and of
-// t around one exact FP64 apply of p0).
+// defect-corrected (pk_apply: FP32 transforms of p - p0 and of t around one
+// exact FP64 apply of p0).
 
 // Per-operator, per-precision solver context: the CG workspace of up to
 // `cap` instances (fields back to back), the device parameter and state
@@ -1154,7 +971,7 @@ struct SolverCtx : SolverCtxBase {
         ASB_CUDA(cudaEventCreateWithFlags(&ev_in, cudaEventDisableTiming));
         ASB_CUDA(cudaEventCreateWithFlags(&ev_out, cudaEventDisableTiming));
         N = (long)o.Ns * o.Ns;
-        Nv = o.embedded() ? (long)o.Nl * o.Ns : N;  // Ns is a multiple of 16
+        Nv = o.embedded() ? (long)o.Nl * o.Ns : N;  // Ns is a multiple of 8
         const size_t b = (size_t)cap * N * sizeof(T);
         T** vecs[] = {&p, &t, &u, &g, &g2, &z, &r, &best, &g0c};
         for (T** v : vecs) ASB_CUDA(cudaMalloc((void**)v, b));
@@ -1282,43 +1099,26 @@ struct SolverCtx : SolverCtxBase {
     T* at(T* v, int b) const { return v + (size_t)b * N; }
 
     // B instances: gates per instance, spectrum of the batch when B > 1
-    void apply(const T* x, T* y, const int* gate, cudaStream_t s, int B,
-               const PkState* sc = nullptr) {
-        op.matvec(sizeof(T) == 8, x, y, s, gate, B, B > 1 ? spec : nullptr, sc);
+    void apply(const T* x, T* y, const int* gate, cudaStream_t s, int B) {
+        op.matvec(sizeof(T) == 8, x, y, s, gate, B, B > 1 ? spec : nullptr);
     }
     // one CG iteration of B instances (the common path), every pass gated
     // per instance on the device:
-    //   [apply p->u] eval (evalpk) | stencil+dots  or  [precond] dots |
-    //   tupd [apply t->r] rden | pupd (load rescale pending, formed by the
-    //   next consumers of p)
-    // the loop's two applies: u = S p (gated by skip_mv1) and r = S t
-    void apply_u(cudaStream_t s, int B) {
-        if constexpr (sizeof(T) == 8) {
-            if (defect) {
-                op.matvec_defect(p, p0, u, u0, s, &st->skip_mv1, B, B > 1 ? spec : nullptr, st);
-                return;
-            }
-        }
-        // p carries its pending load rescale (formed as it is loaded)
-        apply(p, u, &st->skip_mv1, s, B, st);
-    }
-    void apply_r(cudaStream_t s, int B) {
-        if constexpr (sizeof(T) == 8) {
-            if (defect) {
-                op.matvec_defect(t, nullptr, r, nullptr, s, &st->halt, B, B > 1 ? spec : nullptr);
-                return;
-            }
-        }
-        apply(t, r, &st->halt, s, B);
+    //   [apply p->u, eval] (evalpk) | stencil+dots  or  [precond] dots |
+    //   [tupd, apply t->r, rden] | pupd (load rescale pending, formed by the
+    //   next consumers of p); steps in brackets with an apply run in its row
+    //   passes (pk_device.cuh)
+    PkFields<T> fields() const {
+        return PkFields<T>{Pd, st, g0c, p, t, z, g, g2, mask, part, defect ? (const T*)p0 : nullptr,
+                           defect ? (const T*)u0 : nullptr};
     }
     // loop: the last kernel ends the loop graph of these B instances (cond)
     void enqueue_iteration(cudaStream_t s, int B, int loop = 0,
                            cudaGraphConditionalHandle cond = 0) {
         const dim3 gr(grid, B);
         int n = 0;
-        apply_u(s, B);
-        launch_pdl(k_eval<T>, gr, kRedThreads, 0, s, Pd, st, u, g0c, p, g, g2, mask, part, 0);
-        ++n;
+        void* sp = B > 1 ? spec : nullptr;
+        pk_apply(op, fields(), true, defect, sp, s, B);
         if (with_hist) {
             launch_pdl(k_evalpk<T>, gr, kRedThreads, 0, s, Pd, st, p, g, g2, part, hist, 0);
             ++n;
@@ -1329,17 +1129,13 @@ struct SolverCtx : SolverCtxBase {
             ++n;
         } else {
             if (precond == 2)
-                fourier_precond_pk<T>(op, g, g2, mask, st, z, part, s, &st->halt, B,
-                                      B > 1 ? spec : nullptr);
+                fourier_precond_pk<T>(op, g, g2, mask, st, z, part, s, &st->halt, B, sp);
             launch_pdl(k_dots<T>, gr, kRedThreads, 0, s, Pd, st, z, g, g2, mask, part);
             ++n;
         }
-        launch_pdl(k_tupd<T>, gr, kRedThreads, 0, s, Pd, st, z, g, g2, t, mask, p, best);
-        apply_r(s, B);
-        launch_pdl(k_rden<T>, gr, kRedThreads, 0, s, Pd, st, r, g, g2, t, mask, part);
-        n += 2;
-        launch_pdl(k_pupd<T>, gr, kRedThreads, 0, s, Pd, st, p, t, g, g2, mask, part, loop, cond,
-                   B);
+        pk_apply(op, fields(), false, defect, sp, s, B);
+        launch_pdl(k_pupd<T>, gr, kRedThreads, 0, s, Pd, st, p, t, g, g2, mask, best, part, loop,
+                   cond, B);
         count_launches(n + 1);
         ASB_CUDA(cudaGetLastError());
     }
@@ -1405,7 +1201,6 @@ struct SolverCtx : SolverCtxBase {
         std::memset(gated.data(), 0, n * sizeof(PkState));
         for (auto& x : gated) {
             x.halt = H_FINAL;
-            x.skip_mv1 = 1;
         }
         ASB_CUDA(cudaMemcpyAsync(st + lo, gated.data(), n * sizeof(PkState),
                                  cudaMemcpyHostToDevice, s));
@@ -1531,6 +1326,9 @@ struct Solver {
         T *p = c.at(c.p, b), *u = c.at(c.u, b), *g = gap_field(b), *z = c.at(c.z, b),
           *r = c.at(c.r, b), *t = c.at(c.t, b);
         const T* g0 = c.at(c.g0c, b);
+        // the iteration keeps v = u + g0 only: u = S p once more (the apply
+        // the iteration counted; an exact one where it was defect-corrected)
+        c.op.matvec(sizeof(T) == 8, p, u, s, nullptr);
         double o[3];
         reduce(b, 2, p, u, g0, nullptr, 0.0, o);
         const double f_cur = o[0];
@@ -1698,7 +1496,6 @@ struct Solver {
             H.seen_merit = std::numeric_limits<double>::infinity();
             H.status = ST_MAX_ITERATIONS;
             H.halt = o.max_iter > 0 ? H_RUN : H_FINAL;
-            H.skip_mv1 = H.halt ? 1 : 0;
         }
         // defect-corrected applies (a polish stage): p0 = the starting
         // pressures, u0 = S p0 by one exact FP64 apply of all instances
@@ -1775,7 +1572,6 @@ struct Solver {
                     H.u_fresh = 0;
                     if (H.halt == H_FILL) {
                         H.halt = H_RUN;
-                        H.skip_mv1 = 0;
                     }
                     changed = true;
                     continue;
@@ -1815,7 +1611,6 @@ struct Solver {
                     continue;
                 }
                 H.halt = H_RUN;
-                H.skip_mv1 = H.u_fresh ? 1 : 0;
             }
             if (changed) write_states();
         }
@@ -1837,18 +1632,16 @@ struct Solver {
                     I.returned_best = true;
                 }
             }
-            // the certificate is evaluated from an exact apply: a
-            // defect-corrected u is recomputed
-            const bool fresh = H.u_fresh && !c.defect;
-            if (!fresh) H.mv++;
-            H.skip_mv1 = fresh ? 1 : 0;  // gates the final apply per instance
+            // the certificate is evaluated from an exact apply of the final p
+            // (counted unless the last evaluation was of the same p and exact)
+            if (!(H.u_fresh && !c.defect)) H.mv++;
             H.halt = H_FINAL;
         }
         write_states();
-        c.apply(c.p, c.u, &c.st->skip_mv1, s, B);
+        c.apply(c.p, c.u, nullptr, s, B);
         const dim3 gr(c.grid, B);
         launch_pdl(k_eval<T>, gr, kRedThreads, 0, s, c.Pd, c.st, c.u, c.g0c, c.p, c.g, c.g2, c.mask,
-                   c.part, 1);
+                   c.part);
         launch_pdl(k_evalpk<T>, gr, kRedThreads, 0, s, c.Pd, c.st, c.p, c.g, c.g2, c.part, nullptr,
                    1);
         count_launches(2);

@@ -33,7 +33,7 @@ void fourier_precond_pk(Operator& op, const T* ga, const T* gb, const uint8_t* m
 
 // polish_stage: the solve refines p_init (the FP64 stage of a mixed or
 // nested float_then_double solve); its loop applies may then be
-// defect-corrected (see Operator::matvec_defect)
+// defect-corrected (see pk_apply)
 template <typename T>
 void solve_impl(Operator& op, const aspher_solve_opts& o, const void* g0, double p_bar,
                 const void* p_init, double* pressure, double* disp, double* gap, double* hist,

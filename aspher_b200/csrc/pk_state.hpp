@@ -74,7 +74,6 @@ struct PkState {
     int halt;
     int it;
     int u_fresh;
-    int skip_mv1;  // gate of the first apply of an iteration: halt || u_fresh
     int stall, forced_id;
     int copy_best, have_best;
     int status;

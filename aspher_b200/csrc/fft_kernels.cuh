@@ -215,11 +215,14 @@ __host__ __device__ constexpr int col_smem_total() {
 
 // A load or store with kBatch moves all of a thread's pairs in one call
 // (all<count, TT>(row, t, v): pairs t + m TT, m < count) after a begin() that
-// reads its scalars: the steps of the PK iteration (pk_device.cuh).
+// reads its scalars: the steps of the PK iteration (pk_device.cuh).  Such a
+// store gets the contact mask of its pairs as well, two bits each, which the
+// kernel reads ahead of the spectrum.
 template <class F, class = void>
 struct is_batch : std::false_type {};
 template <class F>
 struct is_batch<F, std::enable_if_t<F::kBatch>> : std::true_type {};
+__device__ __forceinline__ uint32_t pair_mask(uint32_t mb, int k) { return mb >> (2 * k) & 3u; }
 
 // CTAs per SM of an inverse row pass with store F: with a step of the PK
 // iteration an FP32 pass gets 80 registers (FP64 fields: 128) instead of 64,
@@ -347,7 +350,18 @@ row_inv_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
     const int r = threadIdx.x % RB, t = threadIdx.x / RB;
     const int row = blockIdx.x * RB + r;
     const bool valid = row < nrows;
-    if constexpr (is_batch<Store>::value) st.begin();
+    constexpr int NV = PAD && RPT > 1 ? RPT / 2 : RPT;  // pairs kept
+    constexpr int NM = is_batch<Store>::value ? NV : 1;
+    uint16_t mw[NM];
+    uint32_t mb = 0;
+    if constexpr (is_batch<Store>::value) {
+        static_assert(NV <= 16, "two mask bits per pair");
+        st.begin();
+        const uint8_t* mp = st.mask + blockIdx.y * st.bs + (size_t)row * st.pitch + 2 * t;
+#pragma unroll
+        for (int k = 0; k < NV; ++k)
+            mw[k] = valid ? *reinterpret_cast<const uint16_t*>(mp + 2 * k * TT) : (uint16_t)0;
+    }
     cplx<T> v[RPT];
     {
         const int ct = ld.ct, lct = __ffs(ct) - 1;  // ct is a power of two
@@ -368,6 +382,10 @@ row_inv_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
     }
 #pragma unroll
     for (int m = 0; m < RPT; ++m) sm[smaddr_run<TT, 1 << 30>(t, m, RB, r)] = v[m];
+    if constexpr (is_batch<Store>::value) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) mb |= ((mw[k] & 1u) | (mw[k] >> 7 & 2u)) << (2 * k);
+    }
     __syncthreads();
     // inverse split step: Z[k] = A + i B w^-k, A = X[k] + conj X[-k], B = X[k] - conj X[-k]
 #pragma unroll
@@ -382,7 +400,7 @@ row_inv_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
     __syncthreads();
     block_fft<T, LR, RPT, +1, RB>(v, t, sm, r, tw_lr);
     if constexpr (is_batch<Store>::value) {
-        if (valid) st.template all<(PAD && RPT > 1 ? RPT / 2 : RPT), TT>(row, t, v);
+        if (valid) st.template all<NV, TT>(row, t, v, mb);
     } else {
 #pragma unroll
         for (int m = 0; m < RPT; ++m) {

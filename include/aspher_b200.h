@@ -75,8 +75,9 @@ typedef struct aspher_op aspher_op;
  * table and its FP64 spectrum are built on the device; synchronous.
  * grid_size in [2, 16384]; at 16384 only FP32 applies and solves exist
  * (FP64 ones return ASPHER_EINVAL).  A grid_size that is not a power of two
- * >= 16 runs embedded: its cells are the top-left block of the next
- * power-of-two grid's free-space pipeline, whose kernel table is the Love
+ * >= 16 runs embedded: its cells are the top-left block of the free-space
+ * pipeline of the next power of two (or of 768, 1536 or 3072 where the block
+ * fits one of these and is at least 513 wide), whose kernel table is the Love
  * table at cell size domain_size / grid_size (FFT) or the real-space kernel
  * of the periodic symbol on the grid_size torus (PERIODIC); every entry
  * point still takes grid_size^2 fields.  Creation flags need a power of
@@ -372,7 +373,7 @@ typedef struct aspher_tan_op aspher_tan_op;
  * Cerruti tables and their three real spectra built on the device in FP64,
  * with the reference's realness check (ASPHER_EBUILD when it fails).
  * grid_size in [2, 2048] (one that is not a power of two >= 16 runs
- * embedded in the next power of two, as for aspher_op_create; every entry
+ * embedded in a larger grid, as for aspher_op_create; every entry
  * point still takes 2 grid_size^2 fields); nu in [0, 1).  Synchronous. */
 int aspher_tan_create(int grid_size, double domain_size, double E_star, double nu,
                       aspher_tan_op** out);

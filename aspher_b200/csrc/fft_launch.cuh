@@ -6,7 +6,9 @@
 
 #include "fft_kernels.cuh"
 #include "ops.hpp"
+#include "reduce.cuh"
 
+#include <type_traits>
 #include <utility>
 
 namespace asb {
@@ -40,6 +42,14 @@ void launch_pdl(void (*k)(P...), dim3 grid, int threads, int smem, cudaStream_t 
     ASB_CUDA(cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...));
 }
 
+// values that a reducing store of a row pass writes per CTA to the instance's
+// partials (Store::kPartials), 0 for the others
+template <class S, class = void>
+struct store_partials : std::integral_constant<int, 0> {};
+template <class S>
+struct store_partials<S, std::enable_if_t<(S::kPartials > 0)>>
+    : std::integral_constant<int, S::kPartials> {};
+
 // B > 1: gridDim.y = B instances (functors / gates / spectrum per instance)
 template <typename T, int LR, bool PAD, int V, class Load, class Store>
 void launch_row_fwd(Load ld, Store st, int nrows, cudaStream_t s, const int* gate, int B = 1) {
@@ -54,6 +64,10 @@ template <typename T, int LR, bool PAD, int V, class Load, class Store>
 void launch_row_inv(Load ld, Store st, int nrows, cudaStream_t s, const int* gate, int B = 1) {
     constexpr int rb = row_rb_v<T>(LR, V), thr = row_threads<T>(LR, V);
     constexpr int sm = row_smem_v<T>(LR, V);
+    constexpr long rows = PAD ? LR : 2 * LR;  // of the whole grid
+    static_assert(Store::kFinish == (store_partials<Store>::value > 0) &&
+                      (rows + rb - 1) / rb * store_partials<Store>::value <= kPartStride,
+                  "a reducing row pass writes past its instance's partials");
     auto k = row_inv_kernel<T, LR, PAD, V, Load, Store>;
     fft_attrs((const void*)k, sm);
     const int gx = (nrows + rb - 1) / rb;

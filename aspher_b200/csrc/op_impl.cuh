@@ -323,6 +323,7 @@ struct StoreGather {  // z = contact ? G : 0; contact sum of G -> zmean
     double* part;
     long bs;  // batch stride (elements); instance blockIdx.y uses st / part of its own
     static constexpr bool kFinish = true;
+    static constexpr int kPartials = 1;
     double zs;
     __device__ __forceinline__ void operator()(int row, int n, cplx<T> v) {
         const size_t i = blockIdx.y * bs + (size_t)row * pitch + 2 * n;
@@ -332,11 +333,11 @@ struct StoreGather {  // z = contact ? G : 0; contact sum of G -> zmean
         if (m.y) zs += (double)v.y;
     }
     __device__ void finish(double*) {
-        double a[1] = {zs};
-        const int kinds[1] = {0};
+        double a[kPartials] = {zs};
+        const int kinds[kPartials] = {0};
         PkState* sb = st + blockIdx.y;
         double* pb = part + (size_t)blockIdx.y * kPartStride;
-        if (grid_reduce_last<1>(a, kinds, pb, &sb->counter[11]) && threadIdx.x == 0) {
+        if (grid_reduce_last<kPartials>(a, kinds, pb, &sb->counter[11]) && threadIdx.x == 0) {
             const int nc = sb->nc;
             sb->zmean = nc ? (double)(T)(a[0] / nc) : 0.0;
             sb->pc++;

@@ -207,6 +207,7 @@ template <typename T, typename Z>
 struct StoreEval {
     using Real = T;
     static constexpr bool kFinish = true;
+    static constexpr int kPartials = 5;
     static constexpr bool kTiled = false;
     static constexpr bool kBatch = true;
     const PkParams* P;
@@ -221,7 +222,7 @@ struct StoreEval {
     int pitch;
     long bs;
     // sum_C v, n_C, min v, pv, psum
-    double acc[5] = {0.0, 0.0, (double)INFINITY, 0.0, 0.0};
+    double acc[kPartials] = {0.0, 0.0, (double)INFINITY, 0.0, 0.0};
     T* g = nullptr;
     T gs = T(0), f = T(0), a = T(0);
     bool stale = false;
@@ -278,8 +279,8 @@ struct StoreEval {
     }
     __device__ void finish(double*) {
         PkState* sb = st + blockIdx.y;
-        const int kinds[5] = {0, 0, 1, 0, 0};
-        if (grid_reduce_last<5>(acc, kinds, part + (size_t)blockIdx.y * kPartStride,
+        const int kinds[kPartials] = {0, 0, 1, 0, 0};
+        if (grid_reduce_last<kPartials>(acc, kinds, part + (size_t)blockIdx.y * kPartStride,
                                 &sb->counter[0]) && threadIdx.x == 0)
             eval_tail<T>(P[blockIdx.y], sb, acc, false);
     }
@@ -292,6 +293,7 @@ template <typename T, typename Z>
 struct StoreLineSums {
     using Real = T;
     static constexpr bool kFinish = true;
+    static constexpr int kPartials = 4;
     static constexpr bool kTiled = false;
     static constexpr bool kBatch = true;
     PkState* st;
@@ -302,7 +304,7 @@ struct StoreLineSums {
     double* part;
     int pitch;
     long bs;
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};  // sum_C r, sum_C g t, sum_C r t, sum_C t
+    double acc[kPartials] = {0.0, 0.0, 0.0, 0.0};  // sum_C r, sum_C g t, sum_C r t, sum_C t
     const T* g = nullptr;
     T aT = T(0);
     __device__ __forceinline__ void begin() {
@@ -344,8 +346,8 @@ struct StoreLineSums {
     }
     __device__ void finish(double*) {
         PkState* sb = st + blockIdx.y;
-        const int kinds[4] = {0, 0, 0, 0};
-        if (grid_reduce_last<4>(acc, kinds, part + (size_t)blockIdx.y * kPartStride,
+        const int kinds[kPartials] = {0, 0, 0, 0};
+        if (grid_reduce_last<kPartials>(acc, kinds, part + (size_t)blockIdx.y * kPartStride,
                                 &sb->counter[4]) && threadIdx.x == 0)
             rden_tail<T>(sb, acc);
     }

@@ -14,11 +14,14 @@ constexpr int kRedThreads = 256;
 constexpr int kRedMinBlocks = 4;
 // upper bound on the grid of the vector-pass reducing kernels
 constexpr int kMaxBlocks = 1184;
-// partials per instance of a batched solve: 8 values for the largest grid of
-// any reducing kernel -- the row kernels of an 8192-row transform run up to
-// 8192 blocks (reductions fused into their stores)
-constexpr int kMaxRowBlocks = 8192;
-constexpr int kPartStride = kMaxRowBlocks * 8;
+// partials per instance of a batched solve: the largest grid of any reducing
+// kernel times its values per CTA.  That is evaluate() (five values) in the
+// inverse row pass of a 16384-sided grid, whose rows take a CTA each;
+// launch_row_inv checks every reducing row pass at compile time.
+constexpr int kMaxRowBlocks = 16384;
+constexpr int kRowValues = 5;
+constexpr int kPartStride = kMaxRowBlocks * kRowValues;
+static_assert(kMaxBlocks * 8 <= kPartStride, "the vector passes reduce up to 8 values");
 
 template <int NV>
 __device__ __forceinline__ void ident_init(double (&v)[NV], const int (&kinds)[NV]) {

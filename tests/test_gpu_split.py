@@ -203,3 +203,51 @@ def test_fp32_nested_at_16384_and_fp64_rejected():
     with pytest.raises(ValueError):
         asb.solve_nested(Ns, g, pbar, coarsest=8192, tol=1e-6, light_result=True,
                          backend="fft", precision="double")
+
+
+def _wavy_gap(Ns, shift=0.0):
+    x = torch.arange(Ns, dtype=torch.float64, device="cuda") / Ns
+    return (-0.001 * (torch.cos(2 * np.pi * (3 * x + shift))[None, :]
+                      + torch.cos(2 * np.pi * 5 * x)[:, None]
+                      + 0.3 * torch.sin(2 * np.pi * 17 * (x[None, :] + 2 * x[:, None])))).reshape(-1)
+
+
+@pytest.mark.parametrize("backend,Ns", [("fft", 13108), ("periodic", 16384)])
+def test_batched_fp32_solves_on_the_largest_grids(backend, Ns):
+    """evaluate()'s partials, five values for each of more than 13107 rows,
+    stay their instance's own: two solves batched equal the same two alone bit
+    for bit (without a preconditioner every launch of an instance has the same
+    grid in both), and the certificate of a converged solve, which comes from
+    those partials, is the one formed from its pressure here."""
+    import aspher_b200 as asb
+    op = _op(Ns, backend=backend)
+    gs = [_wavy_gap(Ns, s).float() for s in (0.0, 0.2)]
+    kw = dict(tol=1e-9, max_iter=5, precond="none", dtype=torch.float32, keep_best=True)
+    both = asb.solve_device_batch(op, gs, [0.005, 0.003], **kw)
+    for g, load, b in zip(gs, (0.005, 0.003), both):
+        a = asb.solve_device(op, g, load, light=True, **kw)
+        assert a.iterations == b.iterations == 5
+        assert torch.equal(a.pressure_device, b.pressure_device)
+        assert (a.fw_error, a.penetration_error, a.contact_area) == \
+            (b.fw_error, b.penetration_error, b.contact_area)
+        del a
+    del both, b
+    load = 5e-5
+    r = asb.solve_device(op, gs[0], load, tol=0.03, max_iter=60, precond="fourier",
+                         dtype=torch.float32, light=True)
+    assert r.status == "converged"
+    p = r.pressure_device.float()
+    v = torch.empty_like(p)
+    op.matvec_(p, v)
+    v += gs[0]
+    on = p > 0
+    assert r.contact_area == float(on.sum()) / Ns ** 2
+    g = v.double() - v[on].double().mean()
+    ref = float(gs[0].double().max() - gs[0].double().min())
+    P = load * Ns * Ns
+    # FP32 fields: 1e-7 of the gap's range per term
+    fw = float((p.double() * (g - g.min())).sum()) / (P * ref)
+    assert abs(fw - r.fw_error) <= 1e-3 * fw + 1e-6, (fw, r.fw_error)
+    assert abs(-float(g.min()) / ref - r.penetration_error) <= 1e-5
+    del op, gs, r, p, v, g, on
+    torch.cuda.empty_cache()

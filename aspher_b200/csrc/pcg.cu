@@ -1616,6 +1616,7 @@ struct Solver {
         }
 
         // ---- final, freshly evaluated diagnostics (contact_solver.cpp:518-586)
+        const std::vector<PkState> loop = h;
         for (int b = 0; b < B; ++b) {
             PkState& H = h[b];
             InstHost& I = ih[b];
@@ -1647,6 +1648,22 @@ struct Solver {
         count_launches(2);
         ASB_CUDA(cudaGetLastError());
         read_states();
+        // A solve whose loop converged on an exact apply keeps the certificate
+        // that ended it: the same p and u, whose sums k_eval adds in another
+        // order.  At a tolerance that the loop met by less than that rounding
+        // (1e-16 of sum p v, whatever G is) its own would not hold.
+        for (int b = 0; b < B; ++b) {
+            if (ih[b].status != ST_CONVERGED || c.defect) continue;
+            const PkState& L = loop[b];
+            PkState& H = h[b];
+            H.alpha_ref = L.alpha_ref;
+            H.gmin_ref = L.gmin_ref;
+            H.G = L.G;
+            H.fw = L.fw;
+            H.pen = L.pen;
+            H.psum = L.psum;
+            H.load = L.load;
+        }
         // objective sum p (0.5 u + g0s) of every instance in one batched pass
         k_reduce<T><<<dim3(c.grid, B), kRedThreads, 0, s>>>(c.Pd, c.st, 5, c.p, c.u, c.g0c, nullptr,
                                                           0.0, c.part);

@@ -281,3 +281,23 @@ def test_sparse_passes_keep_the_minimiser(backend, Ns, precond):
         v -= v[on].mean()
         assert (p * (v - v.min())).sum() <= 2 * tol * total * ref
         assert -v.min() <= 2 * tol * ref and abs(total / (load * Ns * Ns) - 1) <= 1e-10
+
+
+@pytest.mark.parametrize("backend,Ns,dtype,ks", [("fft", 128, torch.float64, range(12, 60, 4)),
+                                                 ("periodic", 96, torch.float64, range(12, 60, 4)),
+                                                 ("fft", 256, torch.float32, range(10, 40, 3))])
+def test_the_certificate_that_ends_the_loop_is_the_one_returned(backend, Ns, dtype, ks):
+    """A tolerance one step below an iterate's own certificate: the loop and
+    the final evaluation sum in different orders, so either may round to the
+    other side of it.  What the loop accepted is not refused afterwards."""
+    import aspher_b200 as asb
+    op = asb.Operator(backend, Ns)
+    g = torch.from_numpy(asb.self_affine_gap(Ns, hurst=0.8, rms=0.002, k_lo=1.5, k_hi=Ns / 8,
+                                             seed=4)).cuda().to(dtype)
+    kw = dict(precond="fourier", dtype=dtype, light=True)
+    for k in ks:
+        r = asb.solve_device(op, g, 0.01, tol=1e-14, max_iter=k, **kw)
+        tol = float(np.nextafter(max(r.fw_error, r.penetration_error), 0.0))
+        r = asb.solve_device(op, g, 0.01, tol=tol, max_iter=4000, **kw)
+        assert r.status == "converged", (k, tol, r.status, r.status_reason, r.fw_error)
+        assert r.fw_error <= tol and r.penetration_error <= tol

@@ -181,40 +181,6 @@ __device__ __forceinline__ void dft(cplx<T>* a) {
     }
 }
 
-// Radix-2 butterfly with a general twiddle: lo = e + w o, hi = e - w o in six
-// fused multiply-adds (hi = 2 e - lo).
-template <typename T>
-__device__ __forceinline__ void bfly_tw(cplx<T> e, cplx<T> o, cplx<T> w, cplx<T>& lo, cplx<T>& hi) {
-    const T lx = fma(w.x, o.x, fma(-w.y, o.y, e.x));
-    const T ly = fma(w.x, o.y, fma(w.y, o.x, e.y));
-    hi = mk<T>(fma(T(2), e.x, -lx), fma(T(2), e.y, -ly));
-    lo = mk<T>(lx, ly);
-}
-
-// The DFT of R points of the inputs a[r] w^r, w[l] = w^(2^l): the twiddles go
-// into the butterflies, lo/hi = E[k] +- (w rot^k) O[k], instead of onto the
-// inputs, which takes 13 instead of 15.25 instructions per point at R = 16 and
-// no powers of w beyond w^(R/2).
-template <int R, int DIR, typename T>
-__device__ __forceinline__ void dft_tw(cplx<T>* a, const cplx<T>* w) {
-    if constexpr (R == 2) {
-        bfly_tw<T>(a[0], a[1], w[0], a[0], a[1]);
-    } else if constexpr (R > 2) {
-        cplx<T> e[R / 2], o[R / 2];
-#pragma unroll
-        for (int i = 0; i < R / 2; ++i) { e[i] = a[2 * i]; o[i] = a[2 * i + 1]; }
-        dft_tw<R / 2, DIR, T>(e, w + 1);
-        dft_tw<R / 2, DIR, T>(o, w + 1);
-#pragma unroll
-        for (int k = 0; k < R / 4; ++k) {
-            const cplx<T> t = rot_const<R, DIR, T>(w[0], k);
-            bfly_tw<T>(e[k], o[k], t, a[k], a[k + R / 2]);
-            bfly_tw<T>(e[k + R / 4], o[k + R / 4], mul_i<DIR>(t), a[k + R / 4],
-                       a[k + R / 4 + R / 2]);
-        }
-    }
-}
-
 // The DFT of R points whose upper half a[R/2 .. R-1] is zero (the first
 // stage of a zero-padded transform): with w = exp(DIR 2 pi i / R),
 //   X[2k] = DFT_{R/2}(a)[k],   X[2k+1] = DFT_{R/2}(a[n] w^n)[k],  n < R/2,
@@ -292,11 +258,6 @@ __device__ __forceinline__ void fft_stages(cplx<T> (&v)[RPT], int t, cplx<T>* sm
     constexpr int RMAX = RPT < 32 ? RPT : 32;
     // one element of padding per radix of the first stage's writes
     constexpr int PS = RPT < 32 ? 4 : 5;
-    // twiddles in the butterflies (dft_tw) or on the inputs: FP64 with 16
-    // points per thread spills with dft_tw (the 4096-point column 77.9 -> 83
-    // us); FP32 needs fewer registers with it (4096 points: 92 -> 88, 39.6 ->
-    // 39.0 us) and 32 points per thread would need 31 powers of w
-    constexpr bool TWB = sizeof(T) == 4 || RPT >= 32;
     constexpr int NST = num_stages(L, RMAX);
     if constexpr (STAGE < NST) {
         constexpr int R = stage_radix(L, RMAX, STAGE);
@@ -313,50 +274,39 @@ __device__ __forceinline__ void fft_stages(cplx<T> (&v)[RPT], int t, cplx<T>* sm
             cplx<T> a[R];
 #pragma unroll
             for (int r = 0; r < R; ++r) a[r] = v[q + r * Q];
-            if constexpr (SPAN > 1 && TWB) {
-                const int jm = j % SPAN;
-                const cplx<T>* __restrict__ tb = tw - L;  // tables at offset = length
-                cplx<T> w[5];  // w^(2^l), entry jm of the length-(SPAN R / 2^l) table
-#pragma unroll
-                for (int l = 0; (1 << l) < R; ++l) {
-                    w[l] = __ldg(&tb[(SPAN * R >> l) + jm]);
-                    if (DIR > 0) w[l].y = -w[l].y;
-                }
-                dft_tw<R, DIR, T>(a, w);
-            } else if constexpr (SPAN > 1) {
-                // w^r for r = 1..R-1 from the loaded powers w, w^2, w^4, w^8
+            if constexpr (SPAN > 1) {
+                // w^r for r = 1..R-1 from the loaded powers w, w^2, w^4, .. w^(R/2)
                 // (products at most three deep), applied as each is formed.
                 // w^(2^e) = exp(-2 pi i jm / (SPAN R / 2^e)) is entry jm of the
                 // length-(SPAN R / 2^e) table, so consecutive threads (jm)
                 // read consecutive entries instead of a stride of L/(SPAN R).
+                // On the inputs, not folded into the butterflies (lo = e + w o,
+                // hi = 2 e - lo): that saves 2 instructions in 15 per point,
+                // but hi carries lo's rounding as well and a point passes
+                // log2 R rounded twiddles.  Against 64 bits an FP32 apply of a
+                // positive field was 18-35 % further off than pocketfft's FP32
+                // so, 2-16 % is; solves in FP32 stagnated a fifth higher.
+                // Free-space apply, folded / on the inputs: FP32 2048 70.9 /
+                // 71.7 us, 4096 324 / 340, FP64 4096 722 / 698.
                 const int jm = j % SPAN;
                 const cplx<T>* __restrict__ tb = tw - L;  // tables at offset = length
-                const cplx<T> w1 = __ldg(&tb[SPAN * R + jm]);
-                a[1] = tw_apply<DIR>(a[1], w1);
-                if constexpr (R >= 4) {
-                    const cplx<T> w2 = __ldg(&tb[SPAN * R / 2 + jm]);
-                    a[2] = tw_apply<DIR>(a[2], w2);
-                    const cplx<T> w3 = cmul(w2, w1);
-                    a[3] = tw_apply<DIR>(a[3], w3);
-                    if constexpr (R >= 8) {
-                        const cplx<T> w4 = __ldg(&tb[SPAN * R / 4 + jm]);
-                        a[4] = tw_apply<DIR>(a[4], w4);
-                        a[5] = tw_apply<DIR>(a[5], cmul(w4, w1));
-                        a[6] = tw_apply<DIR>(a[6], cmul(w4, w2));
-                        a[7] = tw_apply<DIR>(a[7], cmul(w4, w3));
-                        if constexpr (R >= 16) {
-                            const cplx<T> w8 = __ldg(&tb[SPAN * R / 8 + jm]);
-                            a[8] = tw_apply<DIR>(a[8], w8);
-                            a[9] = tw_apply<DIR>(a[9], cmul(w8, w1));
-                            a[10] = tw_apply<DIR>(a[10], cmul(w8, w2));
-                            a[11] = tw_apply<DIR>(a[11], cmul(w8, w3));
-                            const cplx<T> w12 = cmul(w8, w4);
-                            a[12] = tw_apply<DIR>(a[12], w12);
-                            a[13] = tw_apply<DIR>(a[13], cmul(w12, w1));
-                            a[14] = tw_apply<DIR>(a[14], cmul(w12, w2));
-                            a[15] = tw_apply<DIR>(a[15], cmul(w12, w3));
-                        }
-                    }
+                auto power = [&](int e) { return __ldg(&tb[SPAN * R / e + jm]); };
+                constexpr int LOW = R < 8 ? R : 8;  // w^1 .. w^(LOW-1) stay in registers
+                cplx<T> w[LOW], w8 = mk<T>(T(0), T(0)), w16 = w8;
+#pragma unroll
+                for (int r = 1; r < LOW; ++r) {
+                    w[r] = (r & (r - 1)) == 0 ? power(r) : cmul(w[r > 4 ? 4 : 2], w[r > 4 ? r - 4 : 1]);
+                    a[r] = tw_apply<DIR>(a[r], w[r]);
+                }
+#pragma unroll
+                for (int h = 8; h < R; h += 8) {
+                    cplx<T> wh;
+                    if (h == 8) wh = w8 = power(8);
+                    else if (h == 16) wh = w16 = power(16);
+                    else wh = cmul(w16, w8);
+                    a[h] = tw_apply<DIR>(a[h], wh);
+#pragma unroll
+                    for (int r = 1; r < LOW; ++r) a[h + r] = tw_apply<DIR>(a[h + r], cmul(wh, w[r]));
                 }
             }
             // the zero upper half of the input (HZ) is the upper half of
@@ -364,7 +314,7 @@ __device__ __forceinline__ void fft_stages(cplx<T> (&v)[RPT], int t, cplx<T>* sm
             // for m >= RPT / 2 exactly when r >= R / 2
             if constexpr (HZ && STAGE == 0 && R >= 2)
                 dft_upper_zero<R, DIR, T>(a);
-            else if constexpr (SPAN == 1 || !TWB)
+            else
                 dft<R, DIR, T>(a);
             if constexpr (LAST) {
 #pragma unroll

@@ -170,3 +170,31 @@ def test_preconditioners_match_oracle(kind, radius, Ns):
         assert np.all(got[c == 0] == 0.0)
         assert rel(got, ref) < tol
         assert abs(got[c == 1].astype(np.float64).sum()) <= 1e-5 * np.abs(got).sum()
+
+
+@pytest.mark.parametrize("Ns,reps", [(64, 100), (128, 60), (1024, 12)])
+def test_fp32_apply_rounds_like_the_fp32_fft(Ns, reps):
+    """An FP32 apply of a positive field is no further from 64 bits than
+    pocketfft's FP32 transforms with the same FP32 spectrum, but for a sixth:
+    stages that round each output once.  (A butterfly whose second output is
+    formed from the rounded first carries 1.5 times the variance, 1.22 times
+    the error; such transforms were 1.19-1.26 times pocketfft's here.)"""
+    import scipy.fft as sf
+    from aspher_b200 import Operator
+    op, ref = Operator("fft", Ns), OFFT(Ns, 1.0, 1.0)
+    ref.build_single_caches()
+    M = 2 * Ns
+    Kh = (ref.Kh * (float(M) * M)).astype(np.float32)
+    rng = np.random.default_rng(Ns)
+    ours, theirs = [], []
+    for _ in range(reps):
+        x = rng.random((Ns, Ns)).astype(np.float32)
+        want = ref.matvec(x.astype(np.float64).ravel()).reshape(Ns, Ns)
+        y = sf.irfft2(sf.rfft2(x, s=(M, M), workers=-1) * Kh, s=(M, M), workers=-1)[:Ns, :Ns]
+        assert y.dtype == np.float32
+        theirs.append(np.linalg.norm(y - want) / np.linalg.norm(want))
+        xd = torch.from_numpy(x).cuda().reshape(-1)
+        u = op.matvec_(xd, torch.empty_like(xd)).cpu().numpy().reshape(Ns, Ns)
+        ours.append(np.linalg.norm(u - want) / np.linalg.norm(want))
+    rms = lambda e: float(np.sqrt(np.mean(np.square(e))))  # noqa: E731
+    assert rms(ours) <= 7.0 / 6.0 * rms(theirs), (rms(ours), rms(theirs))

@@ -16,6 +16,30 @@ namespace asb {
 // small transforms run the small-CTA variant
 __host__ __device__ constexpr int vclamp(int L, int V) { return L >= 128 ? V : 3; }
 
+// Fastest (row, column) variant pairs measured on B200: every pair set on
+// one operator (aspher_op_set_variants) and 6-20 of its applies timed in a
+// CUDA graph (sides of 3 2^k: the passes alone); sizes not listed use variant
+// 0.  Operator::autotune repeats the search in-process.
+struct VariantRow {
+    int kind, dbl, Ns, rv, cv;
+};
+constexpr VariantRow kVariantTable[] = {
+    {0, 0, 64, 3, 3}, {0, 0, 128, 3, 3}, {0, 0, 256, 3, 3}, {0, 0, 512, 2, 1},
+    {0, 0, 768, 2, 2}, {0, 0, 1024, 1, 1}, {0, 0, 1536, 0, 2}, {0, 0, 2048, 1, 2},
+    {0, 0, 3072, 0, 0}, {0, 0, 4096, 0, 2}, {0, 0, 8192, 0, 2}, {0, 1, 64, 3, 3},
+    {0, 1, 128, 3, 3}, {0, 1, 256, 3, 3}, {0, 1, 512, 3, 1}, {0, 1, 768, 2, 2},
+    {0, 1, 1024, 1, 1}, {0, 1, 1536, 0, 2}, {0, 1, 2048, 1, 1}, {0, 1, 3072, 0, 0},
+    {0, 1, 4096, 0, 2}, {1, 0, 128, 3, 3}, {1, 0, 256, 3, 3}, {1, 0, 512, 3, 3},
+    {1, 0, 1024, 3, 1}, {1, 0, 2048, 1, 2}, {1, 0, 4096, 1, 2}, {1, 0, 8192, 0, 2},
+    {1, 1, 128, 3, 3}, {1, 1, 256, 3, 3}, {1, 1, 512, 3, 3}, {1, 1, 1024, 3, 1},
+    {1, 1, 2048, 2, 1}, {1, 1, 4096, 2, 0}, {1, 1, 8192, 0, 2},
+};
+constexpr VariantRow default_variants(int kind, int dbl, int Ns) {
+    for (const VariantRow& e : kVariantTable)
+        if (e.kind == kind && e.dbl == dbl && e.Ns == Ns) return e;
+    return VariantRow{kind, dbl, Ns, 0, 0};
+}
+
 // max dynamic shared memory + max-shared carveout, once per kernel per device
 void fft_attrs(const void* func, int bytes);
 // CTAs of a persistent pass kernel: at most occupancy x SMs, at most `units`

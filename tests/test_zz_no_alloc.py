@@ -95,3 +95,30 @@ def test_noalloc_rejects_bad_buffers_and_dtype():
     assert b"dtype" in _lib.lib().aspher_last_error()
     assert _noalloc(Ns, 0.0, 1.0, x, y, dtype=_lib.F64) == E
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("Ns", [512, 1024])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_noalloc_has_launch_shapes_of_its_own_size(Ns, dtype):
+    """The launch shape follows the size and the precision as the operator's
+    does: best of five batches, a call takes at most 1.9 times the operator's
+    (1.2-1.6 here, ordinary launches and the symbol formed per element; one
+    shape for every size took 2.3-2.8)."""
+    from aspher_b200 import Operator
+    op = Operator("periodic", Ns)
+    x = torch.randn(Ns * Ns, dtype=dtype, device="cuda")
+    y = torch.empty_like(x)
+
+    def ms(call):
+        best = float("inf")
+        for _ in range(6):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record()
+            for _ in range(100):
+                call()
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        return best
+    ours, ref = ms(lambda: _noalloc(Ns, 1.0, 1.0, x, y)), ms(lambda: op.matvec_(x, y))
+    assert ours <= 1.9 * ref, (ours, ref)

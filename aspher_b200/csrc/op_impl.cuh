@@ -22,15 +22,19 @@ void launch_col_split(cplx<T>* spec, cplx<T>* acc, int nrows, int ndata, Mult m,
     constexpr int V = vclamp(LH, 0);
     constexpr int ct = col_ct_v<T>(LH, NCM1, V), thr = col_threads<T>(LH, NCM1, V);
     constexpr int sm = col_smem<T>(LH, ct);
-    auto k0 = col_split_kernel<T, LH, NCM1, V, 0, Mult>;
-    auto k1 = col_split_kernel<T, LH, NCM1, V, 1, Mult>;
-    fft_attrs((const void*)k0, sm);
-    fft_attrs((const void*)k1, sm);
     const dim3 grid(NCM1 / ct + 1, B);
-    launch_pdl(k0, grid, thr, sm, s, spec, acc, nrows, ndata, m, tw<T>(LH),
-               tw<T>(2 * LH), gate);
-    launch_pdl(k1, grid, thr, sm, s, spec, acc, nrows, ndata, m, tw<T>(LH),
-               tw<T>(2 * LH), gate);
+    auto go = [&](auto all) {
+        auto k0 = col_split_kernel<T, LH, NCM1, V, 0, decltype(all)::value, Mult>;
+        auto k1 = col_split_kernel<T, LH, NCM1, V, 1, decltype(all)::value, Mult>;
+        fft_attrs((const void*)k0, sm);
+        fft_attrs((const void*)k1, sm);
+        launch_pdl(k0, grid, thr, sm, s, spec, acc, nrows, ndata, m, tw<T>(LH), tw<T>(2 * LH),
+                   gate);
+        launch_pdl(k1, grid, thr, sm, s, spec, acc, nrows, ndata, m, tw<T>(LH), tw<T>(2 * LH),
+                   gate);
+    };
+    if (ndata >= LH) go(std::true_type{});
+    else go(std::false_type{});
 }
 
 #define ASB_V_SWITCH(VV, L, ...)                                                   \

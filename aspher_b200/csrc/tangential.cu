@@ -192,8 +192,10 @@ struct TanMix {
 // as 2 CT transforms: field c / CT, column c % CT); per column the pruned
 // forward transform (upper half zero), the 2x2 mix with the other field's
 // column through shared memory, the inverse transform keeping rows < Ns.
-// ndata as in col_kernel.
-template <typename T, int LC, int CT>
+// ndata as in col_kernel; ALL: every row holds data.  A compare per row costs
+// the FP64 kernel its registers (spills): Ns = 1024 57.4 us without, 73.9
+// with, 2048 222 and 280.
+template <typename T, int LC, int CT, bool ALL>
 __global__ void __launch_bounds__(2 * CT * (LC / col_rpt<T>(LC, 0)))
 col_pair_kernel(cplx<T>* __restrict__ spec, long bsp, int nrows, int ndata, TanMix<T> mix,
                 const cplx<T>* __restrict__ tw_lc) {
@@ -218,8 +220,8 @@ col_pair_kernel(cplx<T>* __restrict__ spec, long bsp, int nrows, int ndata, TanM
     cplx<T> v[RPT];
 #pragma unroll
     for (int m = 0; m < RPT; ++m)
-        v[m] = m >= RPT / 2 || t + m * TT >= ndata ? mk<T>(0, 0)
-                                                   : base[(size_t)(t + m * TT) * CT + cc];
+        v[m] = m >= RPT / 2 || (!ALL && t + m * TT >= ndata)
+                   ? mk<T>(0, 0) : base[(size_t)(t + m * TT) * CT + cc];
     block_fft<T, LC, RPT, -1, S, true, ALT>(v, t, sm, c, tw_lc);
     // every thread publishes its column's spectrum, then reads the other
     // field's column at the same kx (the forward transform's last stage ran
@@ -241,7 +243,7 @@ col_pair_kernel(cplx<T>* __restrict__ spec, long bsp, int nrows, int ndata, TanM
     block_fft<T, LC, RPT, +1, S, false, ALT, ALT ? (PX ^ 1) : 0>(v, t, sm, c, tw_lc);
 #pragma unroll
     for (int m = 0; m < RPT / 2; ++m)
-        if (t + m * TT < ndata) base[(size_t)(t + m * TT) * CT + cc] = v[m];
+        if (ALL || t + m * TT < ndata) base[(size_t)(t + m * TT) * CT + cc] = v[m];
 }
 
 }  // namespace
@@ -432,7 +434,7 @@ void TanOperator::apply(Load ld, Store st, int nd, cudaStream_t s) {
         constexpr int thr = 2 * CT * (LC / col_rpt<T>(LC, 0));
         constexpr int sm = col_pair_pp<T>(LC, CT) ? 2 * align16(col_smem<T>(LC, 2 * CT))
                                                   : col_smem<T>(LC, 2 * CT);
-        auto k = col_pair_kernel<T, LC, CT>;
+        auto k = nd >= NS ? col_pair_kernel<T, LC, CT, true> : col_pair_kernel<T, LC, CT, false>;
         fft_attrs((const void*)k, sm);
         const TanMix<T> mix{static_cast<const T*>(kt[dbl][0]), static_cast<const T*>(kt[dbl][1]),
                             static_cast<const T*>(kt[dbl][2]), NS + 1, CT, LC};

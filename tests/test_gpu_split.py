@@ -251,3 +251,42 @@ def test_batched_fp32_solves_on_the_largest_grids(backend, Ns):
     assert abs(-float(g.min()) / ref - r.penetration_error) <= 1e-5
     del op, gs, r, p, v, g, on
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("Ns,dtype,tol", [(4500, torch.float64, 1e-13), (8200, torch.float32, 2e-6)])
+def test_split_columns_of_an_embedded_grid(Ns, dtype, tol):
+    """The split column pass where only the first rows of the compute grid hold
+    data: the response to a load in the last cell is the Love table around it."""
+    op = _op(Ns)
+    T = torch.from_numpy(op.love_table()).cuda().reshape(Ns, Ns)
+    x = torch.zeros(Ns * Ns, dtype=dtype, device="cuda")
+    x[-1] = 1.0
+    u = op.matvec_(x, torch.empty_like(x)).double().reshape(Ns, Ns)
+    want = torch.flip(T, (0, 1))
+    assert float((u - want).norm() / want.norm()) <= tol
+    del op, T, x, u, want
+    torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("Ns,dtype", [(1024, torch.float64), (2048, torch.float64)])
+def test_full_grids_pay_nothing_for_the_embedded_form(Ns, dtype):
+    """The column-pair kernel of a full grid has no compare per row: an apply
+    takes less than that of the embedded grid one smaller, which has them
+    (0.86-0.87 of its time; 1.00-1.02 where the two shared the code)."""
+    from aspher_b200 import TangentialOperator
+
+    def ms(n):
+        op = TangentialOperator(n)
+        q = torch.randn(2 * n * n, dtype=dtype, device="cuda")
+        u = torch.empty_like(q)
+        best = float("inf")
+        for _ in range(6):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record()
+            for _ in range(30):
+                op.matvec_(q, u)
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        return best
+    assert ms(Ns) <= 0.97 * ms(Ns - 1), "full grid slower than an embedded one"

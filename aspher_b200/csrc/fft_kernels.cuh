@@ -55,11 +55,13 @@ struct TiledSpec {
 // (points per thread, threads per CTA, CTAs per SM), measured on B200 over
 // all pairs (tests of the choice: Operator::autotune):
 // Row kernels.  FP32: V0 16/512/2, V1 16/256/4, V2 8/256/4; FP64: V0
-// 16/512/1, V1 16/256/2, V2 8/256/3; V3 the small CTAs of small grids (64
+// 16/512/1, V1 16/256/2, V2 8/256/3.  V3: the small CTAs of small grids (64
 // threads, 8 points, 4 up to 128 points per row), which put a grid of 64 to
-// 512 rows on all the SMs.  Sides of 3 2^k: V2 24/128/4 (FP64 2), the others
-// 24/256/2 (1) (FP64 Ns = 128, the forward pass: 5.4 us with
-// 16-point threads in 512-thread CTAs, 1.7 us).
+// 512 rows on all the SMs (FP64 Ns = 128, the forward pass: 5.4 us with
+// 16-point threads in 512-thread CTAs, 1.7 us); from 1024 points on 8/512/2,
+// two rows of 2048 FP64 points per CTA in runs twice as long (periodic 4096
+// apply 292.5 us with V2, 281.0).  Sides of 3 2^k: V2 24/128/4 (FP64 2), the
+// others 24/256/2 (1).
 template <typename T>
 __host__ __device__ constexpr int row_rpt(int LR, int v) {
     if (LR % 3 == 0) return 24;
@@ -70,12 +72,14 @@ __host__ __device__ constexpr int row_rpt(int LR, int v) {
 template <typename T>
 __host__ __device__ constexpr int row_target_threads(int LR, int v) {
     if (LR % 3 == 0) return v == 2 ? 128 : 256;
-    return v == 0 ? 512 : (v == 3 ? 64 : 256);
+    return v == 0 ? 512 : (v == 3 ? (LR >= 1024 ? 512 : 64) : 256);
 }
 template <typename T>
 __host__ __device__ constexpr int row_minb_req(int LR, int v) {
     if (LR % 3 == 0) return (sizeof(T) == 4 ? 2 : 1) * (v == 2 ? 2 : 1);
-    return sizeof(T) == 4 ? (v == 0 ? 2 : (v == 3 ? 1 : 4)) : (v == 1 ? 2 : (v == 2 ? 3 : 1));
+    const bool wide = v == 3 && LR >= 1024;
+    return sizeof(T) == 4 ? (v == 0 || wide ? 2 : (v == 3 ? 1 : 4))
+                          : (v == 1 || wide ? 2 : (v == 2 ? 3 : 1));
 }
 template <typename T>
 __host__ __device__ constexpr int row_rb_v(int LR, int v) {

@@ -61,3 +61,30 @@ def test_autotune_keeps_the_apply(backend):
     assert op.variants(torch.float32)[:2] == (rv, cv)
     y = _apply(op, x)
     assert np.linalg.norm(y - y0) <= 2e-6 * np.linalg.norm(y0)
+
+
+def test_long_rows_of_the_wide_variant():
+    """Row variant 3 from 1024 points per row on: 512-thread CTAs, two FP64 rows
+    of 2048 points each.  Same apply, and at periodic 4096 the default for its
+    time (0.96 of variant 2's)."""
+    import aspher_b200 as asb
+    op = asb.Operator("periodic", 4096)
+    x = torch.randn(4096 * 4096, dtype=torch.float64, device="cuda")
+    rv, cv, _ = op.variants(torch.float64)
+
+    def ms(row):
+        op.set_variants(row, cv, torch.float64)
+        y = torch.empty_like(x)
+        best = float("inf")
+        for _ in range(6):
+            e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            e0.record()
+            for _ in range(20):
+                op.matvec_(x, y)
+            e1.record()
+            torch.cuda.synchronize()
+            best = min(best, e0.elapsed_time(e1))
+        return best, y
+    (t, y), (t2, y2) = ms(rv), ms(2)
+    assert float((y - y2).norm()) <= 1e-13 * float(y2.norm())
+    assert t <= 0.98 * t2, (t, t2)

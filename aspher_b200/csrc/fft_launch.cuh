@@ -13,8 +13,11 @@
 
 namespace asb {
 
-// small transforms run the small-CTA variant
-__host__ __device__ constexpr int vclamp(int L, int V) { return L >= 128 ? V : 3; }
+// small transforms run the small-CTA variant; those of 3 2^k points have two
+// shapes, variant 2 and the other three
+__host__ __device__ constexpr int vclamp(int L, int V) {
+    return L % 3 == 0 ? (V == 2 ? 2 : 0) : (L >= 128 ? V : 3);
+}
 
 // Fastest (row, column) variant pairs measured on B200: every pair set on
 // one operator (aspher_op_set_variants) and 6-20 of its applies timed in a

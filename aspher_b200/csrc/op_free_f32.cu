@@ -23,25 +23,4 @@ void embedded_precond<float>(Operator& op, const float* ga, const float* gb, con
                                                             spec)));
 }
 
-template <>
-void free_pk_eval<float, float>(const Operator& op, const PkFields<float>& f, cplx<float>* spec, cudaStream_t s,
-        int B) {
-    ASB_FREE_SWITCH(op.Ns, (pk_eval_apply<FreeImpl<float, NS>, float, float>(op, f, spec, s, B)));
-}
-template <>
-void free_pk_line<float, float>(const Operator& op, const PkFields<float>& f, cplx<float>* spec, cudaStream_t s,
-        int B) {
-    ASB_FREE_SWITCH(op.Ns, (pk_line_apply<FreeImpl<float, NS>, float, float>(op, f, spec, s, B)));
-}
-template <>
-void free_pk_eval<double, float>(const Operator& op, const PkFields<double>& f, cplx<float>* spec, cudaStream_t s,
-        int B) {
-    ASB_FREE_SWITCH(op.Ns, (pk_eval_apply<FreeImpl<float, NS>, double, float>(op, f, spec, s, B)));
-}
-template <>
-void free_pk_line<double, float>(const Operator& op, const PkFields<double>& f, cplx<float>* spec, cudaStream_t s,
-        int B) {
-    ASB_FREE_SWITCH(op.Ns, (pk_line_apply<FreeImpl<float, NS>, double, float>(op, f, spec, s, B)));
-}
-
 }  // namespace asb

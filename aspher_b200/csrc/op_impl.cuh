@@ -2,7 +2,7 @@
 // free-space and the periodic apply and of the full-grid |k| preconditioner,
 // as templates over the compute grid.  Their kernels are compiled by
 // op_free_*.cu and op_periodic_*.cu (one translation unit per pipeline and
-// precision); operators.cu uses the layout constants alone.
+// precision, the PK steps apart); operators.cu uses the layout constants alone.
 #pragma once
 
 #include "fft_kernels.cuh"
@@ -47,7 +47,7 @@ void launch_col_split(cplx<T>* spec, cplx<T>* acc, int nrows, int ndata, Mult m,
     }
 
 // ONLY >= 0: launch variant ONLY whatever v is (one instantiation per pass:
-// the grids above kMaxVariantNs and those of 3 2^k)
+// the grids above kMaxVariantNs)
 template <typename T, int LR, bool PAD, int ONLY = -1, class Load, class Store>
 void row_fwd_v(int v, Load ld, Store st, int nrows, cudaStream_t s, const int* gate, int B) {
     if constexpr (ONLY >= 0) {
@@ -94,8 +94,8 @@ struct FreeImpl {
     static constexpr bool kSplitOK = NS >= kSplitMin && NS % 3 != 0 && col_fits<T>(LR);
     // rows and columns in one CTA each (every size but FP64 above 8192)
     static constexpr bool kSupported = row_smem_v<T>(LR, 0) <= kSmemPerSM && (kFits || kSplitOK);
-    static constexpr bool kAllV = NS <= kMaxVariantNs && NS % 3 != 0;
-    // launch variants of the passes with one instantiation per size
+    static constexpr bool kAllV = NS <= kMaxVariantNs;
+    // the one launch variant of the grids above kMaxVariantNs
     static constexpr VariantRow kDefault = default_variants(OP_FFT, sizeof(T) == 8, NS);
     static constexpr int kRV = vclamp(LR, kDefault.rv), kCV = vclamp(LC, kDefault.cv);
     static constexpr int kOnlyR = kAllV ? -1 : kRV, kOnlyC = kAllV ? -1 : kCV;
@@ -112,9 +112,8 @@ struct FreeImpl {
     // row_fwd(ld) -> col(x Kh) -> row_inv(st); ld / st see the Ns x Ns
     // field(s), of which the first op.Nl rows hold data (all of them unless
     // the operator is embedded): the row passes run on those rows alone and
-    // the column pass takes the rest as zero.  RF, RI >= 0: launch variant of
-    // the forward / inverse row pass instead of the operator's.
-    template <int RF = -1, int RI = RF, class Load, class Store>
+    // the column pass takes the rest as zero.
+    template <class Load, class Store>
     static void apply(const Operator& op, Load ld, Store st, cplx<T>* spec, cudaStream_t s,
                       const int* gate, int B, const T* kh_over = nullptr) {
         if constexpr (!kSupported) {
@@ -126,10 +125,7 @@ struct FreeImpl {
             const T* kh = kh_over ? kh_over : (dbl ? (const T*)op.kh_d : (const T*)op.kh_f);
             const long bsp = (long)(LR / c + 1) * NS * c;
             const int nd = op.Nl;
-            const StoreTiled<T> sst{spec, NS, c, bsp};
-            const LoadTiled<T> sld{spec, NS, c, bsp};
-            if constexpr (RF >= 0) launch_row_fwd<T, LR, true, RF>(ld, sst, nd, s, gate, B);
-            else row_fwd_v<T, LR, true, kOnlyR>(rv, ld, sst, nd, s, gate, B);
+            row_fwd_v<T, LR, true, kOnlyR>(rv, ld, StoreTiled<T>{spec, NS, c, bsp}, nd, s, gate, B);
             if (split(op)) {
                 if constexpr (kSplitOK)
                     launch_col_split<T, LR, LR>(spec, spec + (size_t)B * bsp, NS, nd,
@@ -139,8 +135,7 @@ struct FreeImpl {
                     col_v<T, LC, LR, true, kOnlyC>(cv, spec, NS, nd, KhMult<T>{kh, NS + 1, LC, c},
                                                   s, gate, B);
             }
-            if constexpr (RI >= 0) launch_row_inv<T, LR, true, RI>(sld, st, nd, s, gate, B);
-            else row_inv_v<T, LR, true, kOnlyR>(rv, sld, st, nd, s, gate, B);
+            row_inv_v<T, LR, true, kOnlyR>(rv, LoadTiled<T>{spec, NS, c, bsp}, st, nd, s, gate, B);
             count_launches(split(op) ? 4 : 3);
             ASB_CUDA(cudaGetLastError());
         }
@@ -156,23 +151,20 @@ struct FreeImpl {
     template <class Load, class Store>
     static void pk(const Operator& op, Load ld, Store st, cplx<T>* spec, cudaStream_t s,
                    const int* gate, int B) {
-        if constexpr (is_batch<Load>::value) apply<kRV>(op, ld, st, spec, s, gate, B);
-        else apply<-1, kRV>(op, ld, st, spec, s, gate, B);
+        apply(op, ld, st, spec, s, gate, B);
     }
 
-    // an embedded operator's apply on the caller's own layout, at this
-    // size's default row variant (one instantiation per size)
+    // an embedded operator's apply on the caller's own layout
     static void apply_block(const Operator& op, const T* x, T* y, long nl, cplx<T>* spec,
                             cudaStream_t s) {
-        apply<kRV>(op, LoadBlockRows<T>{x, op.Nl, nl}, StoreBlockRows<T>{y, op.Nl, nl}, spec, s,
-                  nullptr, 1);
+        apply(op, LoadBlockRows<T>{x, op.Nl, nl}, StoreBlockRows<T>{y, op.Nl, nl}, spec, s,
+              nullptr, 1);
     }
 };
 
 // The two applies of a PK iteration on the impl's operator: evaluate() in the
-// row store of the p apply (row variant of the operator for its plain load),
-// the direction update and the line-search sums in the row load and store of
-// the t apply.  F: the solver's precision, T: the transform's.
+// row store of the p apply, the direction update and the line-search sums in
+// the row load and store of the t apply.  F: the solver's precision, T: the transform's.
 template <class Impl, typename F, typename T>
 void pk_eval_apply(const Operator& op, const PkFields<F>& f, cplx<T>* spec, cudaStream_t s, int B) {
     const int Ns = op.Ns;
@@ -208,8 +200,7 @@ struct PeriodicImpl {
     static constexpr int kRV = vclamp(LR, kDefault.rv), kCV = vclamp(LC, kDefault.cv);
     static constexpr int kOnlyR = kAllV ? -1 : kRV, kOnlyC = kAllV ? -1 : kCV;
 
-    // RF, RI as in FreeImpl::apply
-    template <int RF = -1, int RI = RF, class Load, class Mult, class Store>
+    template <class Load, class Mult, class Store>
     static void apply(int rv, int cv, Load ld, Mult mult, Store st, cplx<T>* spec, cudaStream_t s,
                       const int* gate, int B) {
         if constexpr (!kSupported) {
@@ -218,13 +209,9 @@ struct PeriodicImpl {
         } else {
             const int c = ct(cv);
             const long bsp = (long)(LR / c + 1) * NS * c;
-            const StoreTiled<T> sst{spec, NS, c, bsp};
-            const LoadTiled<T> sld{spec, NS, c, bsp};
-            if constexpr (RF >= 0) launch_row_fwd<T, LR, false, RF>(ld, sst, NS, s, gate, B);
-            else row_fwd_v<T, LR, false, kOnlyR>(rv, ld, sst, NS, s, gate, B);
+            row_fwd_v<T, LR, false, kOnlyR>(rv, ld, StoreTiled<T>{spec, NS, c, bsp}, NS, s, gate, B);
             col_v<T, LC, LR, false, kOnlyC>(cv, spec, NS, NS, mult, s, gate, B);
-            if constexpr (RI >= 0) launch_row_inv<T, LR, false, RI>(sld, st, NS, s, gate, B);
-            else row_inv_v<T, LR, false, kOnlyR>(rv, sld, st, NS, s, gate, B);
+            row_inv_v<T, LR, false, kOnlyR>(rv, LoadTiled<T>{spec, NS, c, bsp}, st, NS, s, gate, B);
             count_launches(3);
             ASB_CUDA(cudaGetLastError());
         }
@@ -250,9 +237,8 @@ struct PeriodicImpl {
     template <class Load, class Store>
     static void pk(const Operator& op, Load ld, Store st, cplx<T>* spec, cudaStream_t s,
                    const int* gate, int B) {
-        const int dbl = sizeof(T) == 8, rv = op.rowv[dbl], cv = op.colv[dbl];
-        if constexpr (is_batch<Load>::value) apply<kRV>(rv, cv, ld, mult(op), st, spec, s, gate, B);
-        else apply<-1, kRV>(rv, cv, ld, mult(op), st, spec, s, gate, B);
+        const int dbl = sizeof(T) == 8;
+        apply(op.rowv[dbl], op.colv[dbl], ld, mult(op), st, spec, s, gate, B);
     }
 };
 

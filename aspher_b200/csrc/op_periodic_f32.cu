@@ -17,25 +17,4 @@ void periodic_precond<float>(Operator& op, const float* ga, const float* gb, con
     ASB_SIZE_SWITCH(op.Ns, (FourierImpl<float, NS>::run(op, ga, gb, mask, st, z, part, s, gate, B, spec)));
 }
 
-template <>
-void periodic_pk_eval<float, float>(const Operator& op, const PkFields<float>& f, cplx<float>* spec, cudaStream_t s,
-        int B) {
-    ASB_SIZE_SWITCH(op.Ns, (pk_eval_apply<PeriodicImpl<float, NS>, float, float>(op, f, spec, s, B)));
-}
-template <>
-void periodic_pk_line<float, float>(const Operator& op, const PkFields<float>& f, cplx<float>* spec, cudaStream_t s,
-        int B) {
-    ASB_SIZE_SWITCH(op.Ns, (pk_line_apply<PeriodicImpl<float, NS>, float, float>(op, f, spec, s, B)));
-}
-template <>
-void periodic_pk_eval<double, float>(const Operator& op, const PkFields<double>& f, cplx<float>* spec, cudaStream_t s,
-        int B) {
-    ASB_SIZE_SWITCH(op.Ns, (pk_eval_apply<PeriodicImpl<float, NS>, double, float>(op, f, spec, s, B)));
-}
-template <>
-void periodic_pk_line<double, float>(const Operator& op, const PkFields<double>& f, cplx<float>* spec, cudaStream_t s,
-        int B) {
-    ASB_SIZE_SWITCH(op.Ns, (pk_line_apply<PeriodicImpl<float, NS>, double, float>(op, f, spec, s, B)));
-}
-
 }  // namespace asb

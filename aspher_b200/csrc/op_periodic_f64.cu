@@ -17,15 +17,4 @@ void periodic_precond<double>(Operator& op, const double* ga, const double* gb, 
     ASB_SIZE_SWITCH(op.Ns, (FourierImpl<double, NS>::run(op, ga, gb, mask, st, z, part, s, gate, B, spec)));
 }
 
-template <>
-void periodic_pk_eval<double, double>(const Operator& op, const PkFields<double>& f, cplx<double>* spec, cudaStream_t s,
-        int B) {
-    ASB_SIZE_SWITCH(op.Ns, (pk_eval_apply<PeriodicImpl<double, NS>, double, double>(op, f, spec, s, B)));
-}
-template <>
-void periodic_pk_line<double, double>(const Operator& op, const PkFields<double>& f, cplx<double>* spec, cudaStream_t s,
-        int B) {
-    ASB_SIZE_SWITCH(op.Ns, (pk_line_apply<PeriodicImpl<double, NS>, double, double>(op, f, spec, s, B)));
-}
-
 }  // namespace asb

@@ -1,0 +1,17 @@
+// The PK steps of the periodic pipeline in FP32 (see op_impl.cuh).
+#include "op_impl.cuh"
+
+namespace asb {
+
+template <>
+void periodic_pk_eval<float, float>(const Operator& op, const PkFields<float>& f, cplx<float>* spec, cudaStream_t s,
+        int B) {
+    ASB_SIZE_SWITCH(op.Ns, (pk_eval_apply<PeriodicImpl<float, NS>, float, float>(op, f, spec, s, B)));
+}
+template <>
+void periodic_pk_line<float, float>(const Operator& op, const PkFields<float>& f, cplx<float>* spec, cudaStream_t s,
+        int B) {
+    ASB_SIZE_SWITCH(op.Ns, (pk_line_apply<PeriodicImpl<float, NS>, float, float>(op, f, spec, s, B)));
+}
+
+}  // namespace asb

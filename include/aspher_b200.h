@@ -120,8 +120,10 @@ int aspher_op_get_info(const aspher_op* op, aspher_op_info* info);
 
 /* Launch variants of the three FFT passes (row variant: registers per thread
  * and rows per CTA of the two row passes; column variant: registers per
- * thread, columns per CTA and CTAs per SM of the column pass).  Variants
- * 0..3; the half-spectrum layout follows the column variant's tile width.
+ * thread, columns per CTA and CTAs per SM of the column pass), in applies and
+ * in the iterations of a solve.  Variants 0..3 (compute sides below 128 have
+ * one shape, 768, 1536 and 3072 two, 16384 one); the half-spectrum layout
+ * follows the column variant's tile width.
  * No reference counterpart (the reference's FFT engine has no launch shape). */
 int aspher_op_set_variants(aspher_op* op, int dtype, int row_variant, int col_variant);
 int aspher_op_get_variants(const aspher_op* op, int dtype, int* row_variant, int* col_variant,

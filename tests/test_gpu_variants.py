@@ -88,3 +88,47 @@ def test_long_rows_of_the_wide_variant():
     (t, y), (t2, y2) = ms(rv), ms(2)
     assert float((y - y2).norm()) <= 1e-13 * float(y2.norm())
     assert t <= 0.98 * t2, (t, t2)
+
+
+@pytest.mark.parametrize("backend", ["fft", "periodic"])
+def test_variants_reach_the_embedded_apply(backend):
+    """A grid of 300 on the 512-sided pipeline: row variants with other points
+    per thread round differently, within the tolerance of the default's apply."""
+    import aspher_b200 as asb
+    op = asb.Operator(backend, 300)
+    cv = op.variants(torch.float64)[1]
+    x = torch.randn(300 * 300, dtype=torch.float64, device="cuda")
+    ys = []
+    for rv in range(4):
+        op.set_variants(rv, cv, torch.float64)
+        ys.append(op.matvec_(x, torch.empty_like(x)))
+        assert float((ys[-1] - ys[0]).norm()) <= 1e-13 * float(ys[0].norm())
+    assert not torch.equal(ys[0], ys[2])  # 16 and 8 points per thread
+
+
+@pytest.mark.parametrize("backend,Ns,dtype,tol", [
+    ("fft", 768, torch.float64, 1e-8), ("periodic", 600, torch.float64, 1e-8),
+    ("fft", 256, torch.float64, 1e-8), ("periodic", 512, torch.float64, 1e-8),
+    ("fft", 256, torch.float32, 1e-4), ("periodic", 512, torch.float32, 1e-4)])
+def test_variants_reach_the_passes_of_a_solve(backend, Ns, dtype, tol):
+    """The row passes that carry evaluate(), the direction update and the line
+    sums take the row variant: their CTAs reduce in other groups, so ten
+    iterations end in other bits of the same pressure (in FP32 the sums are
+    rounded to the field's 24 bits and only other points per thread show: sides
+    of 3 2^k have 24 in both shapes).  Every pair of variants gives that
+    pressure."""
+    import aspher_b200 as asb
+    op = asb.Operator(backend, Ns)
+    g = torch.from_numpy(asb.self_affine_gap(Ns, hurst=0.8, rms=0.002, k_lo=1.5, k_hi=Ns / 8,
+                                             seed=6)).cuda().to(dtype)
+
+    def pressure(rv, cv):
+        op.set_variants(rv, cv, dtype)
+        r = asb.solve_device(op, g, 0.02, tol=1e-12, max_iter=10, precond="fourier", dtype=dtype,
+                             light=True)
+        return r.pressure_device
+    p0 = pressure(0, 1)
+    assert not torch.equal(pressure(2, 1), p0)
+    for rv in range(4):
+        for cv in range(4):
+            assert float((pressure(rv, cv) - p0).norm()) <= tol * float(p0.norm()), (rv, cv)

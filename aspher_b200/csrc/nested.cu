@@ -237,8 +237,11 @@ std::shared_ptr<Operator> cached_operator(int kind, int Ns, double L, double E) 
 }
 
 void clear_operator_cache() {
-    std::lock_guard<std::mutex> lk(g_cache_mu);
-    g_op_cache.clear();
+    {
+        std::lock_guard<std::mutex> lk(g_cache_mu);
+        g_op_cache.clear();
+    }
+    scratch_trim();
 }
 
 // nested_solve.cpp:27-39

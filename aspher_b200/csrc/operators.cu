@@ -119,7 +119,7 @@ long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
 namespace {
 std::mutex g_pool_mu;
 cudaMemPool_t g_pool[64] = {};  // per device
-std::atomic<int> g_live_ops{0};
+std::atomic<int> g_scratch_users{0};
 }  // namespace
 
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
@@ -152,9 +152,15 @@ cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
 }
 
 void scratch_trim() {
+    std::lock_guard<std::recursive_mutex> setup(setup_mutex());
     std::lock_guard<std::mutex> lk(g_pool_mu);
     for (cudaMemPool_t pool : g_pool)
         if (pool) cudaMemPoolTrimTo(pool, 0);
+}
+
+ScratchUse::ScratchUse() { g_scratch_users.fetch_add(1); }
+ScratchUse::~ScratchUse() {
+    if (g_scratch_users.fetch_sub(1) == 1) scratch_trim();
 }
 
 void smem_optin(const void* func, int bytes) {
@@ -658,12 +664,10 @@ Operator::Operator(int kind_, int Ns_, double L_, double E_, int flags)
         set_variants(dbl != 0, rv, cv);
     }
     ASB_CUDA(cudaDeviceSynchronize());
-    g_live_ops.fetch_add(1);
 }
 
 Operator::~Operator() {
     std::lock_guard<std::recursive_mutex> setup(setup_mutex());
-    if (g_live_ops.fetch_sub(1) == 1) scratch_trim();
     ctx_f.reset();
     ctx_d.reset();
     cudaFree(khp_canon);

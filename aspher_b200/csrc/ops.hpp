@@ -95,16 +95,26 @@ std::recursive_mutex& setup_mutex();
 // every freed byte back to the driver at the next synchronisation, and these
 // drivers synchronise: a nested call to 2048 x 2048 in FP64, 37 ms of kernels,
 // took 44-160 ms and once 1.2 s, mapping its 150 MB anew.  This pool keeps up
-// to kScratchKeep bytes between calls; scratch_trim() gives them back (the
-// last operator's end does).  Safe from any thread and stream.
+// to kScratchKeep bytes between calls; scratch_trim() gives them back: at the
+// end of the last operator of any kind (ScratchUse) and with the operator
+// cache.  Safe from any thread and stream.
 constexpr size_t kScratchKeep = size_t(1) << 30;
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
 void scratch_trim();
+// Held by every operator, as its first member: it goes last, after the frees of
+// the operator's own memory (which wait for scratch freed in stream order).
+struct ScratchUse {
+    ScratchUse();
+    ~ScratchUse();
+    ScratchUse(const ScratchUse&) = delete;
+    ScratchUse& operator=(const ScratchUse&) = delete;
+};
 
 // Opt into >48 KB dynamic shared memory once per kernel per device.
 void smem_optin(const void* func, int bytes);
 
 struct Operator {
+    ScratchUse scratch_use;
     // the compute grid: a power of two in [16, 16384] (embedded: or 768, 1536,
     // 3072) and the pipeline
     // (free-space padded or periodic) that every kernel of this library sees

@@ -249,7 +249,8 @@ col_pair_kernel(cplx<T>* __restrict__ spec, long bsp, int nrows, int ndata, TanM
 }  // namespace
 
 struct TanOperator {
-    // Ns: the compute grid (a power of two in [16, 2048]); Nl: the caller's
+    ScratchUse scratch_use;
+    // Ns: the compute grid (a power of two in [16, 2048], or 768 or 1536); Nl: the caller's
     // side.  Nl < Ns (a side that is not a power of two >= 16) runs
     // embedded: the caller's cells are the top-left block of the compute
     // grid, the Cerruti tables at the caller's cell size L / Nl, so the

@@ -501,7 +501,10 @@ int aspher_solve_nested(int backend, int grid_size, double domain_size, double E
 int aspher_stencil_for_level(int engine, int precond, double prev_occupancy,
                              double occupancy_max);
 
-/* Drops the cached per-level operators of aspher_solve_nested. */
+/* Drops the cached operators of aspher_solve_nested and aspher_solve_many, and
+ * gives the driver back the scratch (at most 1 GiB per device) that the library
+ * keeps between calls.  The end of the last operator, tangential ones among
+ * them, gives that scratch back as well. */
 int aspher_operator_cache_clear(void);
 
 #ifdef __cplusplus

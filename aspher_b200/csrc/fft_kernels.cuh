@@ -36,7 +36,8 @@ namespace asb {
 
 constexpr int kVariants = 4;
 // Batched launches (gridDim.y = instances) read instance b's gate at
-// gate[b * kGateStride]: the gates live in consecutive PkState records.
+// gate[b * kGateStride]: the gates live in consecutive PkState records, which
+// the kernel in front and a reducing store write (hence no __restrict__).
 constexpr int kGateStride = (int)(sizeof(PkState) / sizeof(int));
 static_assert(sizeof(PkState) % sizeof(int) == 0, "PkState must be a whole number of ints");
 constexpr int kSmemPerSM = 227 * 1024;
@@ -261,7 +262,7 @@ __host__ __device__ constexpr int row_minb_f(int LR, int v) {
 template <typename T, int LR, bool PAD, int V, class Load, class Store>
 __global__ void __launch_bounds__(row_threads<T>(LR, V), row_minb<T>(LR, V))
 row_fwd_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
-               const cplx<T>* __restrict__ tw_2lr, const int* __restrict__ gate) {
+               const cplx<T>* __restrict__ tw_2lr, const int* gate) {
     pdl_wait();
     if (gate && gate[blockIdx.y * kGateStride]) return;
     constexpr int RPT = row_rpt<T>(LR, V);
@@ -343,7 +344,7 @@ row_fwd_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
 template <typename T, int LR, bool PAD, int V, class Load, class Store>
 __global__ void __launch_bounds__(row_threads<T>(LR, V), (row_minb_f<T, Store>(LR, V)))
 row_inv_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
-               const cplx<T>* __restrict__ tw_2lr, const int* __restrict__ gate) {
+               const cplx<T>* __restrict__ tw_2lr, const int* gate) {
     pdl_wait();
     if (gate && gate[blockIdx.y * kGateStride]) return;
     constexpr int RPT = row_rpt<T>(LR, V);
@@ -427,7 +428,7 @@ row_inv_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
 template <typename T, int LC, int NCM1, bool PAD, int V, class Mult>
 __global__ void __launch_bounds__(col_threads<T>(LC, NCM1, V), col_minb<T>(LC, NCM1, V))
 col_kernel(cplx<T>* __restrict__ spec, int nrows, int ndata, Mult mul,
-           const cplx<T>* __restrict__ tw_lc, const int* __restrict__ gate) {
+           const cplx<T>* __restrict__ tw_lc, const int* gate) {
     pdl_wait();
     if (gate && gate[blockIdx.y * kGateStride]) return;
     constexpr int RPT = col_rpt<T>(LC, V);
@@ -525,7 +526,7 @@ __global__ void __launch_bounds__(col_threads<T>(LH, NCM1, V), col_minb<T>(LH, N
 col_split_kernel(cplx<T>* __restrict__ spec, cplx<T>* __restrict__ acc, int nrows, int ndata,
                  Mult mul,
                  const cplx<T>* __restrict__ tw_lh, const cplx<T>* __restrict__ tw_m,
-                 const int* __restrict__ gate) {
+                 const int* gate) {
     pdl_wait();
     if (gate && gate[blockIdx.y * kGateStride]) return;
     constexpr int RPT = col_rpt<T>(LH, V);

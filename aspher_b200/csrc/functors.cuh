@@ -9,11 +9,13 @@ namespace asb {
 // Every functor offsets by blockIdx.y * bs (elements): instance blockIdx.y
 // of a batched launch (bs = 0 or gridDim.y = 1 for a single field).
 // The PK loop's pressure with the pending load rescale of instance
-// blockIdx.y (PkState::scale / scale_add): Real(x f) + a.
+// blockIdx.y (PkState::scale / scale_add): Real(x f) + a.  Plain loads: the
+// kernel in front writes the state, and a read-only load need not stay behind
+// pdl_wait().
 template <typename T>
 __device__ __forceinline__ T pending_scale(const PkState* sc, T x) {
     const PkState* sb = sc + blockIdx.y;
-    return x * (T)__ldg(&sb->scale) + (T)__ldg(&sb->scale_add);
+    return x * (T)sb->scale + (T)sb->scale_add;
 }
 
 template <typename T>

@@ -44,19 +44,7 @@
 namespace asb {
 
 // ---- vector helpers ------------------------------------------------------------
-template <typename T>
-__device__ __forceinline__ void ld4(const T* __restrict__ p, long i4, T (&a)[4]) {
-    if constexpr (sizeof(T) == 4) {
-        const float4 v = __ldg(reinterpret_cast<const float4*>(p) + i4);
-        a[0] = v.x; a[1] = v.y; a[2] = v.z; a[3] = v.w;
-    } else {
-        const double2 v0 = __ldg(reinterpret_cast<const double2*>(p) + 2 * i4);
-        const double2 v1 = __ldg(reinterpret_cast<const double2*>(p) + 2 * i4 + 1);
-        a[0] = v0.x; a[1] = v0.y; a[2] = v1.x; a[3] = v1.y;
-    }
-}
-// load through L2 without the read-only path (for arrays written earlier in
-// the same kernel sequence by other kernels it does not matter; kept plain)
+// plain loads: the fields are written by the kernels in front
 template <typename T>
 __device__ __forceinline__ void ldp4(const T* p, long i4, T (&a)[4]) {
     if constexpr (sizeof(T) == 4) {

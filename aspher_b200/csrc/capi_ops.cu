@@ -98,7 +98,7 @@ int aspher_op_get_info(const aspher_op* op, aspher_op_info* info) {
     info->backend = o.backend;
     info->grid_size = o.Nl;
     // the transform side of the compute pipeline (embedded grids: that of
-    // the power-of-two grid the caller's block sits in)
+    // the grid the caller's block sits in)
     info->padded_side = o.kind == asb::OP_FFT ? 2 * o.Ns : o.Ns;
     info->n = (int64_t)o.Nl * o.Nl;
     if (o.kind == asb::OP_FFT)

@@ -1,5 +1,5 @@
 // Embedded grids: the caller's Nl x Nl field as the top-left block of the
-// power-of-two Ns x Ns compute field (row pitch Nl outside, Ns inside).
+// Ns x Ns compute field (row pitch Nl outside, Ns inside).
 // Scalar element accesses only: an odd Nl leaves caller rows at every
 // alignment.
 #pragma once

@@ -42,16 +42,6 @@ constexpr int kGateStride = (int)(sizeof(PkState) / sizeof(int));
 static_assert(sizeof(PkState) % sizeof(int) == 0, "PkState must be a whole number of ints");
 constexpr int kSmemPerSM = 227 * 1024;
 
-template <typename T>
-struct TiledSpec {
-    cplx<T>* base;
-    int nrows;
-    int ct;
-    __device__ __forceinline__ size_t idx(int row, int k) const {
-        return (size_t)(k / ct) * nrows * ct + (size_t)row * ct + (k % ct);
-    }
-};
-
 // ---- variant tables -----------------------------------------------------------------
 // (points per thread, threads per CTA, CTAs per SM), measured on B200 over
 // all pairs (tests of the choice: Operator::autotune):
@@ -244,10 +234,10 @@ __host__ __device__ constexpr int row_minb_f(int LR, int v) {
 
 // ---- row forward ---------------------------------------------------------------
 // Load:  cplx<T> operator()(int row, int n) -> z[n] = (x[2n], x[2n+1]);
-// Store: void operator()(int row, int k, cplx<T> X), k in [0, LR]
-//        static constexpr bool kTiled: true for the tiled half-spectrum store
-//        (then the kernel writes the tiles through base / nrows / ct / bs
-//        itself); static constexpr bool kFinish: when true, every thread
+// Store: void operator()(int row, int k, cplx<T> X), k in [0, LR]; with
+//        static constexpr bool kTiled (the tiled half spectrum) the kernel
+//        writes the tiles through base / nrows / ct / bs itself;
+//        static constexpr bool kFinish: when true, every thread
 //        calls finish(double* scratch) once, after a __syncthreads() at the end
 // Dynamic shared memory: row_smem_v<T>(LR, V).
 //

@@ -26,7 +26,6 @@ struct LoadRealRows {  // z[n] = (x[row*pitch + 2n], x[row*pitch + 2n + 1])
     // optional: x is the PK loop's pressure, scaled by the pending load
     // rescale of sc[blockIdx.y] as it is loaded
     const PkState* sc = nullptr;
-    static constexpr bool kTiled = false;
     __device__ __forceinline__ cplx<T> fix(cplx<T> v) const {
         if (sc) {
             v.x = pending_scale(sc, v.x);
@@ -46,7 +45,6 @@ struct StoreRealRows {
     int pitch;
     long bs;
     static constexpr bool kFinish = false;
-    static constexpr bool kTiled = false;
     __device__ __forceinline__ void operator()(int row, int n, cplx<T> z) const {
         *reinterpret_cast<cplx<T>*>(y + blockIdx.y * bs + (size_t)row * pitch + 2 * n) = z;
     }
@@ -61,7 +59,6 @@ struct LoadBlockRows {
     const T* x;
     int Nl;
     long bs;
-    static constexpr bool kTiled = false;
     __device__ __forceinline__ cplx<T> operator()(int row, int n) const {
         cplx<T> z = mk<T>(T(0), T(0));
         if (row < Nl) {
@@ -79,7 +76,6 @@ struct StoreBlockRows {
     int Nl;
     long bs;
     static constexpr bool kFinish = false;
-    static constexpr bool kTiled = false;
     __device__ __forceinline__ void operator()(int row, int n, cplx<T> z) const {
         if (row >= Nl) return;
         T* r = y + blockIdx.y * bs + (size_t)row * Nl;
@@ -92,7 +88,6 @@ struct StoreBlockRows {
 // FP64 rows in, FP32 pairs out: x - x0, rounded once.  A defect-corrected FP64
 // apply (pk_apply) transforms this difference in FP32.
 struct LoadDiffRows {
-    static constexpr bool kTiled = false;
     const double* x;
     const double* x0;
     int pitch;
@@ -114,16 +109,14 @@ struct LoadDiffRows {
     }
 };
 
+// the tiled half spectrum of row_fwd_kernel's stores and row_inv_kernel's loads
 template <typename T>
 struct StoreTiled {
     cplx<T>* base;
     int nrows, ct;
     long bs;
     static constexpr bool kFinish = false;
-    static constexpr bool kTiled = true;  // row kernels store whole tile chunks
-    __device__ __forceinline__ void operator()(int row, int k, cplx<T> X) const {
-        base[blockIdx.y * bs + (size_t)(k / ct) * nrows * ct + (size_t)row * ct + (k % ct)] = X;
-    }
+    static constexpr bool kTiled = true;
     __device__ void finish(double*) const {}
 };
 
@@ -132,11 +125,6 @@ struct LoadTiled {
     const cplx<T>* base;
     int nrows, ct;
     long bs;
-    static constexpr bool kTiled = true;  // row kernels load whole tile chunks
-    __device__ __forceinline__ cplx<T> operator()(int row, int k) const {
-        return base[blockIdx.y * bs + (size_t)(k / ct) * nrows * ct + (size_t)row * ct +
-                    (k % ct)];
-    }
 };
 
 // Free-space multiplier: real Kh, even-folded in ky, tiled like the spectrum

@@ -247,7 +247,6 @@ struct PeriodicImpl {
 // ----------------------------------------------------------------------------
 template <typename T>
 struct LoadMaskCentered {  // contact ? g - T(gsum/ng) : 0, pairwise; g = v - T(alpha)
-    static constexpr bool kTiled = false;
     const T* ga;  // the gap is in ga or gb (PkState::par)
     const T* gb;
     const uint8_t* mask;
@@ -281,7 +280,6 @@ struct FourierMult {  // |k| / Ns^2 as the reference's float table, cast to T
 
 template <typename T>
 struct StoreGather {  // z = contact ? G : 0; contact sum of G -> zmean
-    static constexpr bool kTiled = false;
     T* z;
     const uint8_t* mask;
     int pitch;

@@ -187,7 +187,6 @@ __global__ void love_table_kernel(double* __restrict__ tab, int Ns, double h, do
 // Embedded table K(iy, ix) = T(|d(iy)|, |d(ix)|), d(i) = i (i < Ns) or i - M,
 // with row/column Ns zero (fft_operator.cpp:31-44), generated on the fly.
 struct LoadEmbedded {
-    static constexpr bool kTiled = false;
     const double* tab;
     int Ns, M;
     __device__ __forceinline__ double at(int iy, int ix) const {
@@ -245,7 +244,6 @@ struct StoreRealTracked {
 // pass stores E (row_fwd of the even samples, StoreCplxRows), the second
 // transforms the odd samples and combines while storing (StoreSplitCombine).
 struct LoadEmbeddedPar {  // z[n] = (x[4n + p], x[4n + 2 + p]) of an embedded row
-    static constexpr bool kTiled = false;
     LoadEmbedded e;
     int p;
     __device__ __forceinline__ double2 operator()(int row, int n) const {
@@ -253,7 +251,6 @@ struct LoadEmbeddedPar {  // z[n] = (x[4n + p], x[4n + 2 + p]) of an embedded ro
     }
 };
 struct LoadRealRowsPar {  // the same sampling of plain rows
-    static constexpr bool kTiled = false;
     const double* x;
     int pitch, p;
     __device__ __forceinline__ double2 operator()(int row, int n) const {

@@ -6,9 +6,12 @@
 // double}; every reduction is accumulated in FP64 as in the reference.
 //
 // One CG iteration is the kernel sequence
-//   [apply p->u] eval [evalpk] stencil+dots tupd [apply t->r] rden pupd
-// where each pass is one sweep and each reduction's scalar logic runs in the
-// last block of its pass (see pk_state.hpp).  Outside the contact set p, t
+//   row_fwd col row_inv+evaluate()        u = S p   (u itself is not stored)
+//   [evalpk] stencil+dots                 or [preconditioner] dots
+//   row_fwd+direction col row_inv+line sums   r = S t (nor is r)
+//   pupd                                  update, pending rescale, the loop's end
+// where each reduction's scalar logic runs in the last block of its pass (see
+// pk_state.hpp, pk_device.cuh).  Outside the contact set p, t
 // and the direction's dots are exactly zero, and a solve spends its
 // iterations at contact fractions of 1-30 %, so the passes read the mask (a
 // byte per cell) first and touch the fields of a group of four cells only
@@ -27,9 +30,6 @@
 #include "reduce.cuh"
 
 #include <algorithm>
-#include <map>
-#include <tuple>
-#include <utility>
 #include <chrono>
 #include <cmath>
 #include <cstdlib>
@@ -39,6 +39,8 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <tuple>
+#include <utility>
 #include <vector>
 
 namespace asb {
@@ -918,6 +920,7 @@ struct SolverCtx : SolverCtxBase {
     int cap = 1;
     long N = 0;
     long Nv = 0;  // the prefix of a field that the vector passes visit (PkParams::Nv)
+    // u and r: the identification step and the final certificate alone
     T *p = nullptr, *t = nullptr, *u = nullptr, *g = nullptr, *g2 = nullptr, *z = nullptr,
       *r = nullptr, *best = nullptr;
     T* g0c = nullptr;  // the solves' gaps, copied in so the loop graph is reusable

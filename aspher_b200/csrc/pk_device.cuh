@@ -141,7 +141,6 @@ __host__ __device__ constexpr int pairs_in_flight(int nv, int most) {
 template <typename T, typename Z>
 struct LoadDirection {
     using Real = T;
-    static constexpr bool kTiled = false;
     static constexpr bool kBatch = true;
     const PkParams* P;
     const PkState* st;
@@ -198,7 +197,6 @@ struct LoadDirection {
             }
         }
     }
-    __device__ __forceinline__ cplx<Z> operator()(int, int) const { return mk<Z>(Z(0), Z(0)); }
 };
 
 // evaluate() in the inverse row store of the p apply (the sums of k_eval; u
@@ -208,7 +206,6 @@ struct StoreEval {
     using Real = T;
     static constexpr bool kFinish = true;
     static constexpr int kPartials = 5;
-    static constexpr bool kTiled = false;
     static constexpr bool kBatch = true;
     const PkParams* P;
     PkState* st;
@@ -284,7 +281,6 @@ struct StoreEval {
                                 &sb->counter[0]) && threadIdx.x == 0)
             eval_tail<T>(P[blockIdx.y], sb, acc, false);
     }
-    __device__ __forceinline__ void operator()(int, int, cplx<Z>) const {}
 };
 
 // The line-search sums in the inverse row store of the t apply (r itself is
@@ -294,7 +290,6 @@ struct StoreLineSums {
     using Real = T;
     static constexpr bool kFinish = true;
     static constexpr int kPartials = 4;
-    static constexpr bool kTiled = false;
     static constexpr bool kBatch = true;
     PkState* st;
     const T* ga;
@@ -351,7 +346,6 @@ struct StoreLineSums {
                                 &sb->counter[4]) && threadIdx.x == 0)
             rden_tail<T>(sb, acc);
     }
-    __device__ __forceinline__ void operator()(int, int, cplx<Z>) const {}
 };
 
 // The fields of a PK iteration of gridDim.y instances, as the row passes see

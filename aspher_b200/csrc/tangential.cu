@@ -64,7 +64,6 @@ __global__ void k_cerruti_tables(double* __restrict__ xx, double* __restrict__ x
 // grid (offset d >= 0 at d, d < 0 at M + d, row / column Ns zero); odd:
 // the sign of an odd-in-each-axis table restored from the offsets' signs
 struct LoadEmbeddedSigned {
-    static constexpr bool kTiled = false;
     const double* tab;
     int Ns, M;
     int odd;

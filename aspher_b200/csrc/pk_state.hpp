@@ -73,6 +73,8 @@ struct PkState {
     // control
     int halt;
     int it;
+    // the reference holds u = S p of the current p: its next evaluation makes no
+    // apply, so mv (the reference's count) does not count ours
     int u_fresh;
     int stall, forced_id;
     int copy_best, have_best;

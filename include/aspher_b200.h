@@ -205,6 +205,11 @@ typedef struct {
     double effective_tol;
     double p_ref;
     double g_ref;
+    /* the applies that the reference's algorithm makes and counts.  Where it reuses u = S p (after an accepted
+     * identification step, in the certificate of an exact solve that
+     * converged) this library, whose iteration does not store u, forms it
+     * again: those applies, and the one at the head of an identification
+     * step, are not counted. */
     int64_t matvec_count;
     int64_t precond_count;
     int identification_steps;

@@ -301,3 +301,19 @@ def test_the_certificate_that_ends_the_loop_is_the_one_returned(backend, Ns, dty
         r = asb.solve_device(op, g, 0.01, tol=tol, max_iter=4000, **kw)
         assert r.status == "converged", (k, tol, r.status, r.status_reason, r.fw_error)
         assert r.fw_error <= tol and r.penetration_error <= tol
+
+
+@pytest.mark.parametrize("backend,Ns,kw", [("fft", 64, dict(stall_limit=1)),
+                                           ("periodic", 32, dict(stall_limit=1)),
+                                           ("fft", 64, {}), ("periodic", 64, dict(max_iter=9))])
+def test_matvec_count_is_the_references(backend, Ns, kw):
+    """matvec_count counts the applies of the reference's algorithm: equal to
+    its count with and without identification steps, converged or not."""
+    import aspher_b200 as asb
+    g = _rough(Ns)
+    kw = dict(dict(tol=1e-10, max_iter=3000), **kw)
+    o = OSolver(Ns, backend=backend).solve(g, 0.02, **kw)
+    r = asb.solve_device(asb.Operator(backend, Ns), torch.from_numpy(np.asarray(g)).cuda(), 0.02,
+                         dtype=torch.float64, **kw)
+    assert (r.iterations, r.identification_steps) == (o.iterations, o.identification_steps)
+    assert r.matvec_count == o.matvec_count

@@ -19,6 +19,10 @@ __host__ __device__ constexpr int vclamp(int L, int V) {
     return L % 3 == 0 ? (V == 2 ? 2 : 0) : (L >= 128 ? V : 3);
 }
 
+// the set-up's row passes: variant 0 but for rows of 16 points, which it would
+// run in CTAs of 16 threads, half a warp of the reduction in their stores
+__host__ __device__ constexpr int build_variant(int L) { return L < 32 ? 3 : 0; }
+
 // Fastest (row, column) variant pairs measured on B200: every pair set on
 // one operator (aspher_op_set_variants) and 6-20 of its applies timed in a
 // CUDA graph (sides of 3 2^k: the passes alone); sizes not listed use variant
@@ -82,6 +86,7 @@ template <typename T, int LR, bool PAD, int V, class Load, class Store>
 void launch_row_fwd(Load ld, Store st, int nrows, cudaStream_t s, const int* gate, int B = 1) {
     constexpr int rb = row_rb_v<T>(LR, V), thr = row_threads<T>(LR, V);
     constexpr int sm = row_smem_v<T>(LR, V);
+    static_assert(!Store::kFinish || thr % 32 == 0, "a reduction needs whole warps");
     auto k = row_fwd_kernel<T, LR, PAD, V, Load, Store>;
     fft_attrs((const void*)k, sm);
     const int gx = (nrows + rb - 1) / rb;
@@ -95,6 +100,7 @@ void launch_row_inv(Load ld, Store st, int nrows, cudaStream_t s, const int* gat
     static_assert(Store::kFinish == (store_partials<Store>::value > 0) &&
                       (rows + rb - 1) / rb * store_partials<Store>::value <= kPartStride,
                   "a reducing row pass writes past its instance's partials");
+    static_assert(!Store::kFinish || thr % 32 == 0, "a reduction needs whole warps");
     auto k = row_inv_kernel<T, LR, PAD, V, Load, Store>;
     fft_attrs((const void*)k, sm);
     const int gx = (nrows + rb - 1) / rb;

@@ -440,11 +440,11 @@ struct KhBuild {
         } else {
             if constexpr (kRowFits) {
                 // pass A over the M rows of the embedded table (real by evenness in ix)
-                launch_row_fwd<double, LR, false, 0>(emb, sa, M, nullptr, nullptr);
+                launch_row_fwd<double, LR, false, build_variant(LR)>(emb, sa, M, nullptr, nullptr);
                 ASB_CUDA(cudaGetLastError());
                 // pass B over the Ns+1 rows of the transposed buffer (each M long)
-                launch_row_fwd<double, LR, false, 0>(LoadRealRows<double>{yt, M, 0}, sb, NS + 1,
-                                                     nullptr, nullptr);
+                launch_row_fwd<double, LR, false, build_variant(LR)>(LoadRealRows<double>{yt, M, 0},
+                                                                     sb, NS + 1, nullptr, nullptr);
                 ASB_CUDA(cudaGetLastError());
             }
         }

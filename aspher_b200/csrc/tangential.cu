@@ -302,12 +302,12 @@ void TanOperator::build() {
         // pass A: rows of the embedded table -> transposed (real part of an
         // even row, imaginary part of an odd one)
         StorePartTracked sa{yt, M, nullptr, 0, odd, 1.0, mb, 0.0, 0.0};
-        launch_row_fwd<double, LR, false, 0>(emb, sa, M, nullptr, nullptr);
+        launch_row_fwd<double, LR, false, build_variant(LR)>(emb, sa, M, nullptr, nullptr);
         // pass B: rows of the transposed buffer; for the odd table the two
         // imaginary factors give K = -Im(X_B)
         StorePartTracked sb{nullptr, M, odd ? cxy : cxx, (int)nk, odd, odd ? -norm : norm,
                             mb + 2, 0.0, 0.0};
-        launch_row_fwd<double, LR, false, 0>(LoadRealRows<double>{yt, M, 0}, sb, NS + 1, nullptr,
+        launch_row_fwd<double, LR, false, build_variant(LR)>(LoadRealRows<double>{yt, M, 0}, sb, NS + 1, nullptr,
                                              nullptr);
         ASB_CUDA(cudaGetLastError());
     }

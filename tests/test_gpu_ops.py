@@ -198,3 +198,23 @@ def test_fp32_apply_rounds_like_the_fp32_fft(Ns, reps):
         ours.append(np.linalg.norm(u - want) / np.linalg.norm(want))
     rms = lambda e: float(np.sqrt(np.mean(np.square(e))))  # noqa: E731
     assert rms(ours) <= 7.0 / 6.0 * rms(theirs), (rms(ours), rms(theirs))
+
+
+@pytest.mark.parametrize("backend,Ns", [("fft", 16), ("fft", 9), ("periodic", 16), ("periodic", 11)])
+def test_smallest_grids_build_and_apply(backend, Ns):
+    """Rows of 16 and 8 points: the reductions of their passes (the realness
+    check of the kernel spectrum, the contact sum of the preconditioner's
+    gather) run on whole warps."""
+    op = _op(backend, Ns)
+    O = OFFT if backend == "fft" else OPer
+    o = O(Ns, 1.0, 1.0)
+    if backend == "fft":
+        assert op.info().max_im_ratio < 1e-12
+    x = np.random.default_rng(Ns).standard_normal(Ns * Ns)
+    assert rel(_mv(op, x, torch.float64), o.matvec(x)) < 1e-12
+    if Ns % 2 == 0:
+        m = (np.arange(Ns * Ns) % 3 != 0)
+        g = torch.from_numpy(x).cuda()
+        z = op.precond_("fourier-fft", g, torch.from_numpy(m.astype(np.uint8)).cuda(),
+                        torch.empty_like(g)).cpu().numpy()
+        assert abs(z[m].sum()) <= 1e-12 * np.abs(z).sum() and np.all(z[~m] == 0)

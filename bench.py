@@ -609,11 +609,44 @@ def run_ours(args):
         }
         it64 = [r.iterations for r in last64]
         line["cpu_baseline"] = cpu_baseline()
+        line, detail = compact(line)
+        print("bench detail: " + json.dumps(detail), file=sys.stderr, flush=True)
         print(json.dumps(line), flush=True)
     for b in list(ops):
         del ops[b]
     if world > 1:
         dist.destroy_process_group()
+
+
+# legs whose full record (per-problem, per-direction and per-step lists: some
+# 15 KB) goes to stderr, and what of each stays on the result line
+SUMMARY = {
+    "single_mixed": ("value", "unit"),
+    "uneven_batch": ("value", "unit", "problems", "converged"),
+    "adjoint": (),
+    "large_single": ("seconds", "status"),
+    "precision_study": (),
+    "fp64_gpu": ("value", "unit", "ratio_mixed_over_fp64"),
+    "accuracy_gate": ("pass",),
+    "solve_roofline": ("achieved", "peak", "unit", "frac"),
+    "tangential_apply": (),
+    "step_ms": (),
+    "cpu_baseline": ("value", "unit", "cores", "kind", "sample"),
+}
+
+
+def compact(line):
+    """(the result line, the detail): one JSON line short enough to be read back
+    whole, with every key of the contract, and the legs' full records."""
+    short, detail = dict(line), {}
+    for key, keep in SUMMARY.items():
+        if key not in short or not isinstance(short[key], dict):
+            continue
+        detail[key] = short.pop(key)
+        kept = {k: detail[key][k] for k in keep if k in detail[key]}
+        if kept:
+            short[key] = kept
+    return short, detail
 
 
 def large_single(dev, Ns=8192, pbar=0.005, active=True):

@@ -286,24 +286,27 @@ __device__ __forceinline__ void fft_stages(cplx<T> (&v)[RPT], int t, cplx<T>* sm
                 // log2 R rounded twiddles.  Against 64 bits an FP32 apply of a
                 // positive field was 18-35 % further off than pocketfft's FP32
                 // so, 2-16 % is; solves in FP32 stagnated a fifth higher.
-                // Free-space apply, folded / on the inputs: FP32 2048 70.9 /
-                // 71.7 us, 4096 324 / 340, FP64 4096 722 / 698.
+                // Free-space apply, folded / on the inputs: FP32 2048 71.9 /
+                // 72.5 us, 4096 326 / 340, FP64 4096 724 / 708.
                 const int jm = j % SPAN;
                 const cplx<T>* __restrict__ tb = tw - L;  // tables at offset = length
                 auto power = [&](int e) { return __ldg(&tb[SPAN * R / e + jm]); };
-                constexpr int LOW = R < 8 ? R : 8;  // w^1 .. w^(LOW-1) stay in registers
-                cplx<T> w[LOW], w8 = mk<T>(T(0), T(0)), w16 = w8;
+                // w .. w^(LOW-1) stay in registers: three at radix 16 (seven
+                // spill in the FP64 column kernels), seven at 32 (4 % of the
+                // FP32 apply at 4096, 1.5 % of the FP64 one)
+                constexpr int LOW = R > 16 ? 8 : (R < 4 ? R : 4);
+                cplx<T> w[LOW], wa = mk<T>(T(0), T(0)), wb = wa;
 #pragma unroll
                 for (int r = 1; r < LOW; ++r) {
                     w[r] = (r & (r - 1)) == 0 ? power(r) : cmul(w[r > 4 ? 4 : 2], w[r > 4 ? r - 4 : 1]);
                     a[r] = tw_apply<DIR>(a[r], w[r]);
                 }
 #pragma unroll
-                for (int h = 8; h < R; h += 8) {
+                for (int h = LOW; h < R; h += LOW) {
                     cplx<T> wh;
-                    if (h == 8) wh = w8 = power(8);
-                    else if (h == 16) wh = w16 = power(16);
-                    else wh = cmul(w16, w8);
+                    if (h == LOW) wh = wa = power(h);
+                    else if (h == 2 * LOW) wh = wb = power(h);
+                    else wh = cmul(wb, wa);
                     a[h] = tw_apply<DIR>(a[h], wh);
 #pragma unroll
                     for (int r = 1; r < LOW; ++r) a[h + r] = tw_apply<DIR>(a[h + r], cmul(wh, w[r]));

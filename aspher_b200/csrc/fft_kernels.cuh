@@ -51,7 +51,7 @@ constexpr int kSmemPerSM = 227 * 1024;
 // 512 rows on all the SMs (FP64 Ns = 128, the forward pass: 5.4 us with
 // 16-point threads in 512-thread CTAs, 1.7 us); from 1024 points on 8/512/2,
 // two rows of 2048 FP64 points per CTA in runs twice as long (periodic 4096
-// apply 292.5 us with V2, 281.0).  Sides of 3 2^k: V2 24/128/4 (FP64 2), the
+// apply 268 us with V2, 263).  Sides of 3 2^k: V2 24/128/4 (FP64 2), the
 // others 24/256/2 (1).
 template <typename T>
 __host__ __device__ constexpr int row_rpt(int LR, int v) {

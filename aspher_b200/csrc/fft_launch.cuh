@@ -37,7 +37,7 @@ constexpr VariantRow kVariantTable[] = {
     {0, 1, 128, 3, 3}, {0, 1, 256, 3, 3}, {0, 1, 512, 3, 1}, {0, 1, 768, 2, 2},
     {0, 1, 1024, 1, 1}, {0, 1, 1536, 0, 2}, {0, 1, 2048, 1, 1}, {0, 1, 3072, 0, 0},
     {0, 1, 4096, 0, 2}, {1, 0, 128, 3, 3}, {1, 0, 256, 3, 3}, {1, 0, 512, 3, 3},
-    {1, 0, 1024, 3, 1}, {1, 0, 2048, 1, 2}, {1, 0, 4096, 1, 2}, {1, 0, 8192, 0, 2},
+    {1, 0, 1024, 3, 1}, {1, 0, 2048, 2, 2}, {1, 0, 4096, 1, 2}, {1, 0, 8192, 0, 2},
     {1, 1, 128, 3, 3}, {1, 1, 256, 3, 3}, {1, 1, 512, 3, 3}, {1, 1, 1024, 3, 1},
     {1, 1, 2048, 2, 1}, {1, 1, 4096, 3, 0}, {1, 1, 8192, 0, 2},
 };

@@ -102,8 +102,8 @@ __host__ __device__ constexpr int row_minb(int LR, int v) {
 // Column kernel.  FP32: V0 16/<=512/1, V1 16/<=256/3, V2 32/<=256/2 (512/1
 // from 8192 points on); FP64: V0 16/<=512/1, V1 16/<=256/2, V2 32/<=256/1; V3
 // small CTAs (4 points and 64 threads up to 256 points, then 8 and 128).
-// 32 points per thread: 4096 points FP32 39.0 -> 33.5 us, 8192 points 203 ->
-// 166 us, FP64 8192 points 387 -> 344 us (one round trip less).
+// 32 points per thread (one round trip less) against V0: 4096 points FP32
+// 43.3 -> 37.9 us, 8192 points 208 -> 186, FP64 8192 points 385 -> 340.
 template <typename T>
 __host__ __device__ constexpr int col_rpt(int LC, int v) {
     if (LC % 3 == 0) return 24;
@@ -245,10 +245,11 @@ __host__ __device__ constexpr int row_minb_f(int LR, int v) {
 // and the ct columns of a tile's row then make one contiguous run, so the
 // spectrum goes from the registers straight to its tile (RB ct elements per
 // run) and only Z[-k], another thread's, comes through shared memory.  The
-// pass is bound by the shared-memory / L1 data pipe (57-65 % busy; issue
-// 45 %): reading Z[k] from shared memory as well and storing by chunk cost
-// one shared pass in seven.  Per launch on B200, before / after: FP32 Ns =
-// 2048 18.3 / 15.9 us, 1024 6.2 / 5.2, FP64 2048 41.9 / 33.6, 4096 197 / 170.
+// pass is bound by L1 (its throughput 75 % in FP32, the shared-memory data
+// pipe 60 %, issue 48 %): reading Z[k] from shared memory as well and storing
+// by chunk cost one shared pass in seven.  Per launch in back-to-back applies,
+// before / after: FP32 Ns = 2048 22.2 / 20.6 us, 4096 148.6 / 80.5, FP64 2048
+// 43.0 / 43.9, 4096 196 / 185.
 template <typename T, int LR, bool PAD, int V, class Load, class Store>
 __global__ void __launch_bounds__(row_threads<T>(LR, V), row_minb<T>(LR, V))
 row_fwd_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
@@ -329,8 +330,9 @@ row_fwd_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
 //
 // One group of RB rows per CTA in the thread order of row_fwd_kernel: X[k]
 // comes from its tile into the thread's registers, X[-k] from the thread that
-// loaded it through shared memory.  Per launch on B200, before / after: FP32
-// Ns = 2048 17.9 / 16.6 us, FP64 2048 42.6 / 35.6, 4096 197 / 187.
+// loaded it through shared memory.  Per launch in back-to-back applies, before
+// / after: FP32 Ns = 2048 18.9 / 17.2 us, 4096 118 / 77, FP64 2048 41.8 / 40.5,
+// 4096 202 / 188.
 template <typename T, int LR, bool PAD, int V, class Load, class Store>
 __global__ void __launch_bounds__(row_threads<T>(LR, V), (row_minb_f<T, Store>(LR, V)))
 row_inv_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
@@ -413,7 +415,8 @@ row_inv_kernel(Load ld, Store st, int nrows, const cplx<T>* __restrict__ tw_lr,
 // Mult: cplx<T> operator()(cplx<T> X, int kx, int ky).  nrows: rows of the
 // layout; ndata: the rows that hold data (fewer only in the zero-padded
 // transform of an embedded operator: the rest read as zero and are not
-// written).  One unit = one tile of CT columns; instance blockIdx.y owns NCM1/CT + 1 contiguous tiles.
+// written).  One unit = one tile of CT columns; instance blockIdx.y owns
+// NCM1/CT + 1 contiguous tiles.
 // Dynamic shared memory: col_smem_total<T, LC, NCM1, PAD, V>().
 template <typename T, int LC, int NCM1, bool PAD, int V, class Mult>
 __global__ void __launch_bounds__(col_threads<T>(LC, NCM1, V), col_minb<T>(LC, NCM1, V))

@@ -74,9 +74,10 @@ bool is_pow2(long v);
 // least 16) is nc: 3/4 of nc where the block fits it and it lies in
 // [kMinTripleNs, largest], else nc.  Its transforms have radix-24 and radix-8
 // stages, less efficient than the 16s and 32s of a power of two: an apply at
-// 768 / 1536 / 3072 against the next power of two took FP32 18.6 / 52.5 / 257
-// us against 20.5 / 66.8 / 312, FP64 28.1 / 108 / 510 against 36.5 / 150 /
-// 700; at 384 FP32 10.3 against 8.9, so the line lies at 768.
+// 768 / 1536 / 3072 against the next power of two takes FP32 17.1 / 51.3 / 244
+// us against 21.7 / 71.7 / 340, FP64 26.8 / 101 / 480 against 37.2 / 151 / 705;
+// at 384 FP32 13.1 against 8.8 and FP64 16.3 against 11.6 (an FP64 iteration
+// 73 us against 63), so the line lies at 768.
 constexpr int kMinTripleNs = 768, kMaxTripleNs = 3072;
 int embed_side(int Nl, int nc, int largest);
 

@@ -285,7 +285,10 @@ __host__ __device__ constexpr int disc_half(int R, int dy) {
 // B200, per launch in the solve loop at the benchmark's contacts (1-20 % of
 // the cells), dense before / listed words after: FP32 Ns = 2048 26.5 / 16.8 us,
 // 1024 14.0 / 9.7; FP64 2048 28.4 / 19.0, 1024 14.6 / 10.6, 512 11.1 / 8.7,
-// 128 10.6 / 7.7.
+// 128 10.6 / 7.7.  Where most of the grid is in contact the list saves nothing
+// and a gathered tap costs more than one from a register window: FP32 2048 at
+// 8 / 82 / 100 % 14.4 / 30.8 / 32.2 us (dense 26.6 / 27.2 / 27.0), FP64 16.0 /
+// 37.8 / 39.0 (28.6 / 30.0 / 30.3); 512 FP64 stays ahead (9.7, dense 12.2).
 constexpr int kStMaxWords = 16;  // words per thread of the largest tile (16, 4 or 1)
 template <typename T, int R, bool LAZY, bool DOTS, bool FULL>
 __global__ void __launch_bounds__(256, 2) k_stencil(const PkParams* __restrict__ Pp, PkState* st,
